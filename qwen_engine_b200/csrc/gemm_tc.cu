@@ -1167,12 +1167,17 @@ int gemm_tc_launch(const GemmArgs& g, int sm_count, cudaStream_t stream) {
     while (S > 2 && tc_smem_bytes(T, S, g.K) > 227 * 1024) --S;
     if (tc_smem_bytes(T, S, g.K) > 227 * 1024) return W4A16_ERR_TOO_LARGE;
     a.T = T;
-    a.stages = S;
     // two issuing warps for token tiles of at most 128 (measured: gate_up at 16 tokens 18.3 -> 14.3 us, down at 128
     // tokens 39.0 -> 30.5 us; at 256 tokens the tensor pipe, not the issue, paces the loop and one warp is as fast);
     // each has its own accumulator, so the column count doubles
     a.issuers = T <= 128 ? 2 : 1;
     while (a.issuers > 1 && a.issuers * T > 512) --a.issuers;
+    // Two issuing warps walk the k-blocks independently, so "this slot's previous use is over" follows from a warp's own
+    // order only if a slot always belongs to the same warp: an even number of stages.  With an odd number a parity
+    // wait can take the phase before last for the last one (129-255 tokens on 9472 or more rows ran 5 stages and
+    // ended in a launch failure).
+    if (a.issuers == 2) S &= ~1;
+    a.stages = S;
     int cols = 32;
     while (cols < a.issuers * T) cols *= 2;
     a.tmem_cols = cols;

@@ -1,4 +1,5 @@
-"""Builds libw4a16_b200.so in-tree with nvcc for sm_100a (cross-compiles without a GPU).
+"""Builds libw4a16_b200.so in-tree with nvcc for sm_100a (cross-compiles without a GPU), and beside it the Python
+entry points of the launch functions (_launch.so, host C++ on torch's headers).
 
     python -m qwen_engine_b200.build [--force] [--verbose]
 """
@@ -13,6 +14,8 @@ from pathlib import Path
 PKG = Path(__file__).resolve().parent
 CSRC = PKG / "csrc"
 LIB = PKG / "libw4a16_b200.so"
+LAUNCH = PKG / "_launch.so"
+LAUNCH_SOURCE = CSRC / "py_launch.cpp"
 SOURCES = ["c_abi.cu", "q8_1_quantize.cu", "gemv_decode.cu", "gemm_prefill.cu", "gemm_tc.cu", "decode_sweep.cu", "sweep_persistent.cu",
            "gemv_static_scratch.cu", "sampling.cu", "embed_lookup.cu", "qwenbin.cu"]
 NVCC_FLAGS = [
@@ -37,17 +40,52 @@ def _inputs():
     return files
 
 
-def up_to_date() -> bool:
-    if not LIB.exists():
+def _newer(target: Path, inputs) -> bool:
+    if not target.exists():
         return False
-    t = LIB.stat().st_mtime
-    return all(f.stat().st_mtime <= t for f in _inputs())
+    t = target.stat().st_mtime
+    return all(f.stat().st_mtime <= t for f in inputs)
+
+
+def up_to_date() -> bool:
+    return _newer(LIB, _inputs()) and _launch_up_to_date()
+
+
+def _launch_up_to_date() -> bool:
+    return _newer(LAUNCH, [LAUNCH_SOURCE, PKG.parent / "include" / "w4a16_b200.h"])
+
+
+def build_launch(force: bool = False) -> Path:
+    """The CPython module; it finds libw4a16_b200.so beside itself at run time."""
+    if not force and _launch_up_to_date():
+        return LAUNCH
+    import sysconfig
+
+    import torch
+    from torch.utils import cpp_extension
+
+    torch_lib = Path(torch.__file__).resolve().parent / "lib"
+    includes = [*cpp_extension.include_paths(device_type="cuda"), sysconfig.get_paths()["include"]]
+    cmd = [shutil.which("g++") or "g++", "-O2", "-std=c++20", "-shared", "-fPIC", "-fvisibility=hidden",
+           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch.compiled_with_cxx11_abi())}", *[f"-isystem{p}" for p in includes],
+           str(LAUNCH_SOURCE), "-o", str(LAUNCH), f"-L{PKG}", "-l:libw4a16_b200.so", f"-L{torch_lib}", "-ltorch_python",
+           "-ltorch", "-ltorch_cpu", "-lc10", "-lc10_cuda", "-Wl,-rpath,$ORIGIN"]
+    res = subprocess.run(cmd, capture_output=True, text=True)
+    if res.returncode != 0:
+        sys.stderr.write(res.stdout + res.stderr)
+        raise RuntimeError("g++ failed building _launch.so")
+    return LAUNCH
 
 
 def build(force: bool = False, verbose: bool = False) -> Path:
-    """One nvcc -c per source file, in parallel, then one link step."""
-    if not force and up_to_date():
-        return LIB
+    """One nvcc -c per source file, in parallel, then one link step; then the Python module."""
+    if force or not _newer(LIB, _inputs()):
+        _build_lib(verbose)
+    build_launch(force)
+    return LIB
+
+
+def _build_lib(verbose: bool) -> None:
     from concurrent.futures import ThreadPoolExecutor
     objdir = PKG / "build"
     objdir.mkdir(exist_ok=True)
@@ -75,7 +113,6 @@ def build(force: bool = False, verbose: bool = False) -> Path:
     if link.returncode != 0:
         sys.stderr.write(link.stdout + link.stderr)
         raise RuntimeError("linking libw4a16_b200.so failed")
-    return LIB
 
 
 if __name__ == "__main__":

@@ -47,6 +47,33 @@ def _stream(stream) -> int:
     return stream.cuda_stream if hasattr(stream, "cuda_stream") else int(stream)
 
 
+# The launch functions themselves are builtins (csrc/py_launch.cpp): at 1-4 us a kernel, argument handling in Python would
+# take longer than the work.  Each is `name(<arguments of the C function, in its order>, stream=None, ...)`.
+_NATIVE = (
+    "launch_quantize_fp16_to_q8_1", "launch_rmsnorm_q8_1", "quantize_attn_heads_f32_to_q8_1",
+    "gemv_attn_heads_f32_w4a16", "launch_gemv_w4a16", "gemv_w4a16_static_scratch", "launch_gemv_w4a8",
+    "launch_embed_lookup_w4a16", "launch_sample_and_advance", "launch_gemv_w4a8_sample_candidates",
+    "launch_gemv_w4a8_sample_one_launch", "launch_sample_finish", "launch_gemv_w4a8_sample_and_advance",
+    "launch_gemv_qkv_w4a8", "launch_gemv_dual_gate_up_swiglu_w4a16", "launch_gemv_dual_gate_up_swiglu_w4a8",
+    "launch_gemv_rmsnorm_w4a16", "launch_gemv_qkv_rmsnorm_w4a16", "launch_gemv_dual_gate_up_swiglu_rmsnorm_w4a16",
+    "launch_gemv_dual_gate_up_swiglu_rmsnorm_w4a16_q8_1", "launch_gemm_prefill_w4a16",
+    "launch_gemm_prefill_qkv_w4a16", "launch_gemm_prefill_dual_gate_up_swiglu_w4a16", "gemv_group_dots",
+)
+try:
+    from . import _launch
+except ImportError as _e:      # not built (yet): the functions exist and say so, so that the build script can import this
+    _launch_error = str(_e)
+
+    class _launch:  # noqa: N801
+        @staticmethod
+        def missing(*_args, **_kwargs):
+            raise ImportError(f"qwen_engine_b200/_launch.so cannot be loaded ({_launch_error}): build it with "
+                              "`python -m qwen_engine_b200.build` (there is no non-CUDA fallback)")
+
+globals().update({_n: getattr(_launch, _n, None) or _launch.missing for _n in _NATIVE})
+_sweep_run_device = getattr(_launch, "sweep_run_device", None) or _launch.missing
+
+
 @dataclass
 class QKVProjectionView:
     """reference include/kernels.cuh:23-27"""
@@ -94,57 +121,6 @@ def set_pdl(enabled: bool) -> None:
     set_option(OPT_PDL, int(bool(enabled)))
 
 
-def launch_quantize_fp16_to_q8_1(input_x, out_q8, out_scale, out_sum8, num_elements, stream=None):
-    check("w4a16_quantize_fp16_to_q8_1", load().w4a16_quantize_fp16_to_q8_1(
-        _ptr(input_x), _ptr(out_q8), _ptr(out_scale), _ptr(out_sum8), num_elements, _stream(stream)))
-
-
-def launch_rmsnorm_q8_1(input, gamma, output_fp16_opt, out_q8, out_scale, out_sum8, stream=None,
-                        hidden_size=HIDDEN_SIZE):
-    check("w4a16_rmsnorm_q8_1", load().w4a16_rmsnorm_q8_1(
-        _ptr(input), _ptr(gamma), _ptr(output_fp16_opt), _ptr(out_q8), _ptr(out_scale), _ptr(out_sum8),
-        _stream(stream), hidden_size))
-
-
-def quantize_attn_heads_f32_to_q8_1(attn_acc, attn_out_fp16_opt, out_q8, out_scale, out_sum8, num_heads, head_dim=128,
-                                    stream=None):
-    """Q8_1 of attention heads from their fp32 accumulators, with the rule of the reference's flash-decode
-    combine step (src/kernels/attention_gqa.cu:258-310): per head, q = rn(acc / d)."""
-    check("w4a16_quantize_attn_heads_f32_to_q8_1", load().w4a16_quantize_attn_heads_f32_to_q8_1(
-        _ptr(attn_acc), _ptr(attn_out_fp16_opt), _ptr(out_q8), _ptr(out_scale), _ptr(out_sum8), num_heads, head_dim,
-        _stream(stream)))
-
-
-def gemv_attn_heads_f32_w4a16(qweight, scales, attn_acc, residual, output_y, out_features, in_features, stream=None):
-    """O projection straight from the fp32 attention accumulators (quantised per head in the GEMV's prologue)."""
-    check("w4a16_gemv_attn_heads_f32_w4a16", load().w4a16_gemv_attn_heads_f32_w4a16(
-        _ptr(qweight), _ptr(scales), _ptr(attn_acc), _ptr(residual), _ptr(output_y), out_features, in_features,
-        _stream(stream)))
-
-
-def launch_gemv_w4a16(qweight, scales, input_x, residual, output_y, out_features, in_features, stream=None):
-    check("w4a16_gemv_w4a16", load().w4a16_gemv_w4a16(
-        _ptr(qweight), _ptr(scales), _ptr(input_x), _ptr(residual), _ptr(output_y), out_features, in_features,
-        _stream(stream)))
-
-
-def gemv_w4a16_static_scratch(qweight, scales, input_x, residual, output_y, out_features, in_features,
-                              stream=None):
-    """launch_gemv_w4a16 for callers that can neither pass nor allocate scratch: the Q8_1 form of
-    the activation goes into a fixed array inside the library (in_features <= 32768; calls that
-    overlap on the GPU race on that array)."""
-    check("w4a16_gemv_w4a16_static_scratch", load().w4a16_gemv_w4a16_static_scratch(
-        _ptr(qweight), _ptr(scales), _ptr(input_x), _ptr(residual), _ptr(output_y), out_features, in_features,
-        _stream(stream)))
-
-
-def launch_gemv_w4a8(qweight, scales, input_q8, input_scale, input_sum8, residual, output_y, out_features,
-                     in_features, stream=None):
-    check("w4a16_gemv_w4a8", load().w4a16_gemv_w4a8(
-        _ptr(qweight), _ptr(scales), _ptr(input_q8), _ptr(input_scale), _ptr(input_sum8), _ptr(residual),
-        _ptr(output_y), out_features, in_features, _stream(stream)))
-
-
 def gemv_w4a8_peers(qweight, scales, input_q8, input_scale, input_sum8, output_y, peer_ptrs, out_features,
                     in_features, stream=None):
     """launch_gemv_w4a8 that also stores its output slice at the device addresses `peer_ptrs` (the slice's
@@ -174,36 +150,11 @@ def read_sample_control(control) -> dict:
     return {"token_id": token_id, "seq_pos": seq_pos, "temperature": temperature, "rng_seed": rng_seed}
 
 
-def launch_embed_lookup_w4a16(embed_qweight, embed_scales, d_token_ids, out_hidden, d_control, num_tokens, stream=None,
-                              hidden_size=HIDDEN_SIZE, vocab_size=VOCAB_SIZE):
-    """Mirror of launch_embed_lookup_w4a16 (reference include/kernels.cuh); vocab_size bounds the token ids."""
-    check("w4a16_embed_lookup_w4a16", load().w4a16_embed_lookup_w4a16(
-        _ptr(embed_qweight), _ptr(embed_scales), _ptr(d_token_ids), _ptr(out_hidden), _ptr(d_control), num_tokens,
-        _stream(stream), hidden_size, vocab_size))
-
-
-def launch_sample_and_advance(logits, sample_scratch_val, sample_scratch_idx, d_control, d_token_out, stream=None,
-                              vocab_size=VOCAB_SIZE):
-    """Mirror of launch_sample_and_advance (reference include/kernels.cuh:210-219)."""
-    check("w4a16_sample_and_advance", load().w4a16_sample_and_advance(
-        _ptr(logits), _ptr(sample_scratch_val), _ptr(sample_scratch_idx), _ptr(d_control), _ptr(d_token_out),
-        _stream(stream), vocab_size))
-
-
 def sample_slots(out_features: int) -> int:
     n = load().w4a16_sample_slots(out_features)
     if n < 0:
         check("w4a16_sample_slots", n)
     return n
-
-
-def launch_gemv_w4a8_sample_candidates(qweight, scales, input_q8, input_scale, input_sum8, output_logits, candidate_val,
-                                       candidate_idx, d_control, index_offset, out_features, in_features, stream=None):
-    """lm_head GEMV that leaves one (score, index) candidate per CTA; output_logits may be None."""
-    check("w4a16_gemv_w4a8_sample_candidates", load().w4a16_gemv_w4a8_sample_candidates(
-        _ptr(qweight), _ptr(scales), _ptr(input_q8), _ptr(input_scale), _ptr(input_sum8), _ptr(output_logits),
-        _ptr(candidate_val), _ptr(candidate_idx), _ptr(d_control), index_offset, out_features, in_features,
-        _stream(stream)))
 
 
 def gemv_w4a8_sample_candidates_peers(qweight, scales, input_q8, input_scale, input_sum8, candidate_val, candidate_idx,
@@ -262,126 +213,12 @@ def sample_finish_after_signals(candidate_val_ptr, candidate_idx_ptr, count, hal
         _ptr(d_control), _ptr(d_token_out), _stream(stream)))
 
 
-def launch_gemv_w4a8_sample_one_launch(qweight, scales, input_q8, input_scale, input_sum8, output_logits, sample_scratch_val,
-                                       sample_scratch_idx, d_counter, d_control, d_token_out, out_features, in_features,
-                                       stream=None):
-    """lm_head + token selection + control-block advance in one launch (d_counter: zero-initialised int32 [1])."""
-    check("w4a16_gemv_w4a8_sample_one_launch", load().w4a16_gemv_w4a8_sample_one_launch(
-        _ptr(qweight), _ptr(scales), _ptr(input_q8), _ptr(input_scale), _ptr(input_sum8), _ptr(output_logits),
-        _ptr(sample_scratch_val), _ptr(sample_scratch_idx), _ptr(d_counter), _ptr(d_control), _ptr(d_token_out),
-        out_features, in_features, _stream(stream)))
-
-
-def launch_sample_finish(candidate_val, candidate_idx, count, d_control, d_token_out, stream=None):
-    check("w4a16_sample_finish", load().w4a16_sample_finish(
-        _ptr(candidate_val), _ptr(candidate_idx), count, _ptr(d_control), _ptr(d_token_out), _stream(stream)))
-
-
-def launch_gemv_w4a8_sample_and_advance(qweight, scales, input_q8, input_scale, input_sum8, output_logits,
-                                        sample_scratch_val, sample_scratch_idx, d_control, d_token_out, out_features,
-                                        in_features, stream=None):
-    """launch_gemv_w4a8 (lm_head) + launch_sample_and_advance in one pass over the weights."""
-    check("w4a16_gemv_w4a8_sample_and_advance", load().w4a16_gemv_w4a8_sample_and_advance(
-        _ptr(qweight), _ptr(scales), _ptr(input_q8), _ptr(input_scale), _ptr(input_sum8), _ptr(output_logits),
-        _ptr(sample_scratch_val), _ptr(sample_scratch_idx), _ptr(d_control), _ptr(d_token_out), out_features,
-        in_features, _stream(stream)))
-
-
-def launch_gemv_qkv_w4a8(view: QKVProjectionView, input_q8, input_scale, input_sum8, stream=None,
-                         in_features=HIDDEN_SIZE, num_q_heads=NUM_Q_HEADS, num_kv_heads=NUM_KV_HEADS,
-                         head_dim=HEAD_DIM):
-    pod = view.pod()
-    check("w4a16_gemv_qkv_w4a8", load().w4a16_gemv_qkv_w4a8(
-        ctypes.byref(pod), _ptr(input_q8), _ptr(input_scale), _ptr(input_sum8), _stream(stream), in_features,
-        num_q_heads, num_kv_heads, head_dim))
-
-
-def launch_gemv_dual_gate_up_swiglu_w4a16(gate_up_qweight, gate_up_scales, input_x, output_mlp, hidden_size,
-                                          intermediate_size, stream=None):
-    check("w4a16_gemv_dual_gate_up_swiglu_w4a16", load().w4a16_gemv_dual_gate_up_swiglu_w4a16(
-        _ptr(gate_up_qweight), _ptr(gate_up_scales), _ptr(input_x), _ptr(output_mlp), hidden_size,
-        intermediate_size, _stream(stream)))
-
-
-def launch_gemv_dual_gate_up_swiglu_w4a8(gate_up_qweight, gate_up_scales, input_q8, input_scale, input_sum8,
-                                         output_mlp, hidden_size, intermediate_size, stream=None):
-    check("w4a16_gemv_dual_gate_up_swiglu_w4a8", load().w4a16_gemv_dual_gate_up_swiglu_w4a8(
-        _ptr(gate_up_qweight), _ptr(gate_up_scales), _ptr(input_q8), _ptr(input_scale), _ptr(input_sum8),
-        _ptr(output_mlp), hidden_size, intermediate_size, _stream(stream)))
-
-
-def launch_gemv_rmsnorm_w4a16(qweight, scales, input_x, gamma, residual, output_y, out_features, in_features,
-                              stream=None):
-    """launch_rmsnorm_q8_1 + launch_gemv_w4a8 in one launch (gamma None: quantise only)."""
-    check("w4a16_gemv_rmsnorm_w4a16", load().w4a16_gemv_rmsnorm_w4a16(
-        _ptr(qweight), _ptr(scales), _ptr(input_x), _ptr(gamma), _ptr(residual), _ptr(output_y), out_features,
-        in_features, _stream(stream)))
-
-
-def launch_gemv_qkv_rmsnorm_w4a16(view: QKVProjectionView, input_x, gamma, stream=None, in_features=HIDDEN_SIZE,
-                                  num_q_heads=NUM_Q_HEADS, num_kv_heads=NUM_KV_HEADS, head_dim=HEAD_DIM):
-    """launch_rmsnorm_q8_1 + launch_gemv_qkv_w4a8 in one launch."""
-    pod = view.pod()
-    check("w4a16_gemv_qkv_rmsnorm_w4a16", load().w4a16_gemv_qkv_rmsnorm_w4a16(
-        ctypes.byref(pod), _ptr(input_x), _ptr(gamma), _stream(stream), in_features, num_q_heads, num_kv_heads,
-        head_dim))
-
-
-def launch_gemv_dual_gate_up_swiglu_rmsnorm_w4a16(gate_up_qweight, gate_up_scales, input_x, gamma, output_mlp,
-                                                  hidden_size, intermediate_size, stream=None):
-    """launch_rmsnorm_q8_1 + launch_gemv_dual_gate_up_swiglu_w4a8 in one launch."""
-    check("w4a16_gemv_dual_gate_up_swiglu_rmsnorm_w4a16", load().w4a16_gemv_dual_gate_up_swiglu_rmsnorm_w4a16(
-        _ptr(gate_up_qweight), _ptr(gate_up_scales), _ptr(input_x), _ptr(gamma), _ptr(output_mlp), hidden_size,
-        intermediate_size, _stream(stream)))
-
-
-def launch_gemv_dual_gate_up_swiglu_rmsnorm_w4a16_q8_1(gate_up_qweight, gate_up_scales, input_x, gamma, output_mlp,
-                                                       output_q8, output_scale, output_sum8, hidden_size,
-                                                       intermediate_size, stream=None):
-    """The launch above, which also leaves the Q8_1 form of output_mlp (the down projection's input)."""
-    check("w4a16_gemv_dual_gate_up_swiglu_rmsnorm_w4a16_q8_1",
-          load().w4a16_gemv_dual_gate_up_swiglu_rmsnorm_w4a16_q8_1(
-              _ptr(gate_up_qweight), _ptr(gate_up_scales), _ptr(input_x), _ptr(gamma), _ptr(output_mlp),
-              _ptr(output_q8), _ptr(output_scale), _ptr(output_sum8), hidden_size, intermediate_size,
-              _stream(stream)))
-
-
 def gemm_prefill_w4a16_block(qweight, scales, input_x, residual_ptr, output_ptr, ldc, peer_ptrs, M, N, K, stream=None):
     """launch_gemm_prefill_w4a16 into a column block of an [M][ldc] matrix (addresses as integers), also stored
     at `peer_ptrs` (the block's place in peer GPUs' matrices)."""
     arr = (ctypes.c_void_p * max(1, len(peer_ptrs)))(*peer_ptrs)
     check("w4a16_gemm_prefill_w4a16_block", load().w4a16_gemm_prefill_w4a16_block(
         _ptr(qweight), _ptr(scales), _ptr(input_x), residual_ptr, output_ptr, ldc, arr, len(peer_ptrs), M, N, K,
-        _stream(stream)))
-
-
-def launch_gemm_prefill_w4a16(qweight, scales, input_x, residual, output_y, M, N, K, stream=None, sm_count=0):
-    check("w4a16_gemm_prefill_w4a16", load().w4a16_gemm_prefill_w4a16(
-        _ptr(qweight), _ptr(scales), _ptr(input_x), _ptr(residual), _ptr(output_y), M, N, K, _stream(stream),
-        sm_count))
-
-
-def launch_gemm_prefill_qkv_w4a16(view: QKVProjectionView, input_x, M, stream=None, in_features=HIDDEN_SIZE,
-                                  num_q_heads=NUM_Q_HEADS, num_kv_heads=NUM_KV_HEADS, head_dim=HEAD_DIM,
-                                  sm_count=0):
-    pod = view.pod()
-    check("w4a16_gemm_prefill_qkv_w4a16", load().w4a16_gemm_prefill_qkv_w4a16(
-        ctypes.byref(pod), _ptr(input_x), M, _stream(stream), in_features, num_q_heads, num_kv_heads, head_dim,
-        sm_count))
-
-
-def launch_gemm_prefill_dual_gate_up_swiglu_w4a16(gate_up_qweight, gate_up_scales, input_x, output_mlp, M,
-                                                  stream=None, hidden_size=HIDDEN_SIZE,
-                                                  intermediate_size=INTERMEDIATE_SIZE):
-    check("w4a16_gemm_prefill_dual_gate_up_swiglu_w4a16", load().w4a16_gemm_prefill_dual_gate_up_swiglu_w4a16(
-        _ptr(gate_up_qweight), _ptr(gate_up_scales), _ptr(input_x), _ptr(output_mlp), M, _stream(stream),
-        hidden_size, intermediate_size))
-
-
-def gemv_group_dots(qweight, input_q8, input_sum8, out_dots, out_features, in_features, stream=None):
-    """Diagnostic: int32 per-group partial sums of the decode GEMV (no reference launcher)."""
-    check("w4a16_gemv_group_dots", load().w4a16_gemv_group_dots(
-        _ptr(qweight), _ptr(input_q8), _ptr(input_sum8), _ptr(out_dots), out_features, in_features,
         _stream(stream)))
 
 
@@ -423,11 +260,11 @@ class DecodeSweep:
         handle = ctypes.c_void_p()
         check("w4a16_sweep_create", lib.w4a16_sweep_create(ctypes.byref(desc), _stream(stream), ctypes.byref(handle)))
         self._h = handle
+        self._handle = handle.value
         self.launches = lib.w4a16_sweep_launches(handle)
 
     def run_device(self, h_in: torch.Tensor, h_out: torch.Tensor, stream=None):
-        check("w4a16_sweep_run_device", load().w4a16_sweep_run_device(self._h, _ptr(h_in), _ptr(h_out),
-                                                                      _stream(stream)))
+        _sweep_run_device(self._handle, h_in, h_out, stream)
 
     def run_host(self, h_in: torch.Tensor, h_out: torch.Tensor, stream=None):
         """h_in / h_out: pinned host fp16 tensors; asynchronous on the stream."""
@@ -448,6 +285,7 @@ class DecodeSweep:
         if self._h is not None:
             load().w4a16_sweep_destroy(self._h)
             self._h = None
+            self._handle = 0
 
     def __del__(self):
         try:

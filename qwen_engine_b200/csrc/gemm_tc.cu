@@ -961,6 +961,8 @@ __global__ void __launch_bounds__(kPairThreads, 1) gemm_w4a16_tc_pair_kernel(con
     if (warp == kDqWarps) tmem_dealloc_pair(tmem_base, static_cast<uint32_t>(a.tmem_cols));
 }
 
+#include "gemm_tc_stream.cuh"
+
 // ---- host side ----------------------------------------------------------------------------
 
 using EncodeTiledFn = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
@@ -987,20 +989,21 @@ struct MapKey {
     const void* base;
     uint64_t inner, outer, row_bytes;
     uint32_t box_inner, box_outer;
-    int dt;
+    int dt, swizzle;
     bool operator==(const MapKey& o) const {
         return base == o.base && inner == o.inner && outer == o.outer && row_bytes == o.row_bytes &&
-               box_inner == o.box_inner && box_outer == o.box_outer && dt == o.dt;
+               box_inner == o.box_inner && box_outer == o.box_outer && dt == o.dt && swizzle == o.swizzle;
     }
 };
 constexpr size_t kMapCacheEntries = 256;
 
 bool encode_2d(CUtensorMap* map, CUtensorMapDataType dt, const void* base, uint64_t inner, uint64_t outer,
-               uint64_t row_bytes, uint32_t box_inner, uint32_t box_outer) {
+               uint64_t row_bytes, uint32_t box_inner, uint32_t box_outer,
+               CUtensorMapSwizzle swizzle = CU_TENSOR_MAP_SWIZZLE_128B) {
     static std::mutex mu;
     static std::vector<std::pair<MapKey, CUtensorMap>> cache;
     static size_t next = 0;
-    const MapKey key{base, inner, outer, row_bytes, box_inner, box_outer, static_cast<int>(dt)};
+    const MapKey key{base, inner, outer, row_bytes, box_inner, box_outer, static_cast<int>(dt), static_cast<int>(swizzle)};
     {
         std::lock_guard<std::mutex> lock(mu);
         for (const auto& kv : cache)
@@ -1013,7 +1016,7 @@ bool encode_2d(CUtensorMap* map, CUtensorMapDataType dt, const void* base, uint6
     const cuuint32_t box[2] = {box_inner, box_outer};
     const cuuint32_t estr[2] = {1, 1};
     if (fn(map, dt, 2, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-           CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
+           swizzle, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
         return false;
     std::lock_guard<std::mutex> lock(mu);
     if (cache.size() < kMapCacheEntries) cache.emplace_back(key, *map);
@@ -1107,6 +1110,9 @@ int gemm_tc_set_attributes() {
     auto raise_pair = [&e](auto* kernel) {
         if (e == cudaSuccess) e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
     };
+    raise_pair(gemm_w4a16_tc_stream_kernel<kPlain>);
+    raise_pair(gemm_w4a16_tc_stream_kernel<kQkv>);
+    raise_pair(gemm_w4a16_tc_stream_kernel<kSwiglu>);
     raise_pair(gemm_w4a16_tc_pair_kernel<kPlain, 256>);
     raise_pair(gemm_w4a16_tc_pair_kernel<kQkv, 256>);
     raise_pair(gemm_w4a16_tc_pair_kernel<kSwiglu, 256>);
@@ -1131,7 +1137,112 @@ bool gemm_tc_supported(const GemmArgs& g) {
     return tc_smem_bytes(16, 2, g.K) <= 227 * 1024;
 }
 
+namespace {
+constexpr int kStreamDoesNotFit = -1000;     // a K range whose group scales and rings are beyond a CTA's shared memory
+template <int MODE>
+int stream_active_clusters(int ksplit, size_t smem) {
+    static std::mutex mu;
+    static std::vector<std::pair<uint64_t, int>> cache;
+    int dev = 0;
+    cudaGetDevice(&dev);
+    const uint64_t key = (static_cast<uint64_t>(dev) << 48) ^ (static_cast<uint64_t>(ksplit) << 32) ^ static_cast<uint64_t>(smem);
+    std::lock_guard<std::mutex> lock(mu);
+    for (const auto& kv : cache)
+        if (kv.first == key) return kv.second;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(1, 1, static_cast<unsigned>(ksplit));
+    cfg.blockDim = dim3(kStThreads);
+    cfg.dynamicSmemBytes = smem;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = 1; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = static_cast<unsigned>(ksplit);
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    int n = 0;
+    if (cudaOccupancyMaxActiveClusters(&n, gemm_w4a16_tc_stream_kernel<MODE>, &cfg) != cudaSuccess) { cudaGetLastError(); n = 0; }
+    cache.emplace_back(key, n);
+    return n;
+}
+template <int MODE>
+int launch_stream(StreamArgs& a, const __half* x, int tiles, int sm_count, cudaStream_t stream) {
+    // Token tiles and K slices, two steps each at least, within one CTA per SM where that is possible.  Estimated cycles of a
+    // CTA, from measurements on B200: 400 a step of dequantisation or 4 T of MMA, whichever is longer; the exchange of
+    // partials at 18 bytes a cycle with its latency; 25 a token for the epilogue.
+    const int steps = a.K / kGroup;
+    StreamArgs best = a;
+    size_t smem = 0, best_smem = 0;
+    double best_cost = 0;
+    const int ts_min = (a.M + 127) / 128, ts_max = (a.M + 15) / 16;
+    for (int ts = ts_min; ts <= ts_max; ++ts) {
+        const int T = ((a.M + ts - 1) / ts + 15) & ~15;
+        if (ts > ts_min && ((a.M + T - 1) / T != ts || tiles * ts > sm_count)) continue;
+        for (int split = std::max(1, std::min({kStMaxSplit, sm_count / (tiles * ts), steps / 2})); split >= 1; --split) {
+            a.T = T;
+            a.ksplit = split;
+            const int per = (steps + split - 1) / split;
+            const double cost = per * std::max(400.0, 4.0 * T) + (split > 1 ? 1500.0 + T * 512.0 * (split - 1) / split / 18.0 + 25.0 * T / split : 25.0 * T);
+            if (best_smem != 0 && cost >= best_cost) continue;
+            if (!plan_stream(per, &a, &smem)) continue;
+            if (split > 1 && stream_active_clusters<MODE>(split, smem) < tiles * ts) continue;
+            best = a;
+            best_smem = smem;
+            best_cost = cost;
+        }
+    }
+    if (best_smem == 0) return kStreamDoesNotFit;
+    a = best;
+    smem = best_smem;
+    if (!encode_2d(&a.tmap_x, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, x, static_cast<uint64_t>(a.K), static_cast<uint64_t>(a.M),
+                   static_cast<uint64_t>(a.K) * 2, kBK, static_cast<uint32_t>(a.T)))
+        return W4A16_ERR_INVALID_ARG;
+    return static_cast<int>(launch_kernel_cluster(gemm_w4a16_tc_stream_kernel<MODE>, dim3(tiles, (a.M + a.T - 1) / a.T, a.ksplit), dim3(kStThreads), smem,
+                                                  stream, pdl_enabled(), dim3(1, 1, static_cast<unsigned>(a.ksplit)), a));
+}
+// The streaming form; *taken says whether it applies (up to 256 tokens, K range within a CTA's staging).
+int gemm_tc_stream_launch(const GemmArgs& g, int sm_count, cudaStream_t stream, bool* taken) {
+    *taken = false;
+    if (g.M > 256) return 0;
+    StreamArgs a;
+    a.num_peers = g.mode == kPlain ? g.num_peers : 0;
+    for (int p = 0; p < 7; ++p) a.peer_out[p] = p < a.num_peers ? g.peer_out[p] : nullptr;
+    const int nt = g.mode == kQkv ? 3 : 1;
+    int total_tiles = 0;
+    for (int t = 0; t < 3; ++t) {
+        a.scales[t] = g.scales[t];
+        a.out[t] = g.out[t];
+        a.rows[t] = t < nt ? g.rows[t] : 0;
+        a.tiles[t] = (a.rows[t] + kTileRows - 1) / kTileRows;
+        total_tiles += a.tiles[t];
+        a.out_ld[t] = g.mode == kSwiglu ? g.rows[0] / 2 : a.rows[t];
+        if (g.mode == kPlain && t == 0 && g.ldc > 0) a.out_ld[0] = g.ldc;
+    }
+    a.residual = g.residual;
+    a.M = g.M;
+    a.K = g.K;
+    for (int t = 0; t < nt; ++t) {
+        if (!encode_2d(&a.tmap_w[t], CU_TENSOR_MAP_DATA_TYPE_UINT8, g.qweight[t], static_cast<uint64_t>(g.K / 2),
+                       static_cast<uint64_t>(g.rows[t]), static_cast<uint64_t>(g.K / 2), 64, kTileRows, CU_TENSOR_MAP_SWIZZLE_64B))
+            return W4A16_ERR_INVALID_ARG;
+    }
+    for (int t = nt; t < 3; ++t) a.tmap_w[t] = a.tmap_w[0];
+    int e;
+    switch (g.mode) {
+        case kPlain: e = launch_stream<kPlain>(a, g.x, total_tiles, sm_count, stream); break;
+        case kQkv: e = launch_stream<kQkv>(a, g.x, total_tiles, sm_count, stream); break;
+        default: e = launch_stream<kSwiglu>(a, g.x, total_tiles, sm_count, stream); break;
+    }
+    if (e == kStreamDoesNotFit) return 0;
+    *taken = true;
+    return e;
+}
+}  // namespace
+
 int gemm_tc_launch(const GemmArgs& g, int sm_count, cudaStream_t stream) {
+    if (option(W4A16_OPT_GEMM_FORM) == 0) {
+        bool taken = false;
+        const int e = gemm_tc_stream_launch(g, sm_count, stream, &taken);
+        if (taken || e != 0) return e;
+    }
     TcArgs a;
     a.panel = 1;
     const int nt = g.mode == kQkv ? 3 : 1;

@@ -1,0 +1,503 @@
+// Batched-decode W4A16 contraction on tcgen05 (17 to 256 tokens) as a weight-streaming kernel: one launch is about as long
+// as its weights take to arrive.  Included by gemm_tc.cu behind the PTX wrappers.
+//
+// What bounds it: at these token counts a launch reads 1-14 MB of packed weights (0.2-2 us of HBM time) and the rest is
+// latency -- the launch boundary, the dequantisation, the token tile's way from L2, the hand-overs between roles, the
+// K-split exchange.  So what does not depend on the previous kernel is done before the wait for it (barriers, group scales,
+// the ring of weights, the first steps' dequantisation), hand-overs are few (one barrier wait per 128 k in each role), and
+// tokens and K are split over CTAs where the row tiles alone leave SMs idle.
+//
+// D[n][m] = sum_k W[n][k] X[m][k], 128 weight rows on the M side of the MMA, T tokens on its N side, in steps of 128 k (one
+// quantisation group).  A (dequantised weights) goes from registers to tensor memory, a thread owning a weight row = a TMEM
+// lane; B (tokens) comes from shared memory.  With A in tensor memory an MMA of 16..64 tokens takes 12..32 cycles against
+// 40..48 with A in shared memory (measured in a loop), provided the issuing thread is chosen by elect.sync: behind a
+// `lane == 0` branch every operand is moved to a uniform register first and each MMA costs 67.
+//
+//   warps 0..15 : dequantise, four warps a step (steps s % 4), then the epilogue
+//   warp 16     : allocates tensor memory; one thread issues the MMAs (8 per step) behind ONE barrier per slot that counts
+//                 the dequantising warps and the token tile's bytes
+//   warp 17     : one thread loads by TMA: packed weights, 128 rows x 128 k (8 KB) per ring slot, and tokens, T x 128 k per slot
+//
+// Tensor memory: even and odd steps go into accumulators of their own: half as many additions per fp32 sum, which at
+// K = 8192 is the difference between 2.7 and 2 fp16 steps of error.  A slots of 64 columns follow: six up to 64 tokens,
+// four above.
+//
+// K split: every CTA of a cluster finishes its own share of the tokens.  Partials travel as 16-byte asynchronous stores
+// into the owner's shared memory which count themselves on the owner's mbarrier, so the exchange needs no cluster barrier
+// behind it; the one that makes sure that the peers have started is passed before the main loop.  A CTA sends T x 512 bytes
+// at about 18 bytes a cycle, which is why the planner prefers a smaller token tile to a deeper K split.
+constexpr int kStDqWarps = 16;
+constexpr int kStGroups = kStDqWarps / 4;        // groups of four warps = 128 rows
+constexpr int kStDqThreads = kStDqWarps * 32;
+constexpr int kStThreads = kStDqThreads + 2 * 32;
+constexpr int kStRawBytes = kTileRows * 64;      // 128 rows x 128 k of packed nibbles
+constexpr int kStMaxRaw = 24, kStMaxSlots = 6;   // ring slots at most
+constexpr int kStACols = kGroup / 2;             // 128 k of fp16 = 64 columns
+constexpr int kStMaxSplit = 8;                   // portable cluster size
+
+struct StreamArgs {
+    CUtensorMap tmap_w[3];
+    CUtensorMap tmap_x;
+    const __half* scales[3];
+    __half* out[3];
+    int rows[3];
+    int out_ld[3];
+    int tiles[3];
+    const __half* residual;
+    int M, K, T;
+    int ksplit;           // cluster size along grid z
+    int tpr;              // tokens a CTA of the cluster finishes (multiple of 4)
+    int raw_slots;        // multiple of 4: a slot always belongs to the same group of dequantising warps (parity waits)
+    int slots;            // A / token slots, at least 4 (the MMAs complete in order, so a group is never two uses ahead)
+    int x_mem;            // token slots that have memory: `slots`, or the steps of a short K range
+    int part_offset;      // K split: byte offset of the partials in shared memory; 0 = on top of the rings
+    int acc2_col, a_col;  // second accumulator; first column of the A slots
+    __half* peer_out[7];  // PLAIN: the output block's place in other GPUs' matrices
+    int num_peers;
+};
+
+// One thread of the (converged) warp, in a form the compiler knows to be warp-uniform.
+__device__ __forceinline__ bool elect_one() {
+    uint32_t p;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xFFFFFFFF;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(p));
+    return p != 0;
+}
+// D[tmem] (+)= A[tmem] * B[smem]^T, one CTA.
+__device__ __forceinline__ void tc_mma_f16_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t desc_b, uint32_t idesc, uint32_t accumulate) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
+        ::"r"(tmem_d), "r"(tmem_a), "l"(desc_b), "r"(idesc), "r"(accumulate)
+        : "memory");
+}
+__device__ __forceinline__ void tmem_ld8(uint32_t taddr, uint32_t (&r)[8]) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+                 : "r"(taddr)
+                 : "memory");
+}
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+// 16 bytes into a CTA of the cluster; the bytes are counted on the barrier there once they have landed.
+__device__ __forceinline__ void st_async_16(uint32_t cluster_addr, uint32_t cluster_bar, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
+    asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v4.b32 [%0], {%2, %3, %4, %5}, [%1];"
+                 ::"r"(cluster_addr), "r"(cluster_bar), "r"(a), "r"(b), "r"(c), "r"(d) : "memory");
+}
+// Bounded wait that does not look at the abort flag.
+__device__ __forceinline__ bool wait_regardless(uint32_t bar, uint32_t parity, unsigned limit) {
+    for (unsigned it = 0; it < limit; ++it)
+        if (mbar_try_wait(bar, parity)) return true;
+    return false;
+}
+
+// (q - 8) * s of one packed word with one rounding, as dequant_word_fp16, in 11 instructions instead of 15: a nibble at bits
+// 4..7 of a half is the subnormal q * 2^-20, so fma(q * 2^-20, s * 2^20, -8 s) is the whole conversion; both constants are
+// exact while s * 2^20 is finite (s < 0.0624; larger scales take dequant_word_fp16).
+__device__ __forceinline__ void dequant_word_small_scale(uint32_t packed, __half2 s20, __half2 m8s, uint32_t* out) {
+    const uint32_t lo = (packed << 4) & 0xF0F0F0F0u, hi = packed & 0xF0F0F0F0u;
+    const uint32_t h[4] = {__byte_perm(lo, 0, 0x4140), __byte_perm(lo, 0, 0x4342), __byte_perm(hi, 0, 0x4140), __byte_perm(hi, 0, 0x4342)};
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const __half2 v = __hfma2(*reinterpret_cast<const __half2*>(&h[i]), s20, m8s);
+        out[i] = *reinterpret_cast<const uint32_t*>(&v);
+    }
+}
+
+// 8 token columns of this thread's weight row, both accumulators added.
+__device__ __forceinline__ void stream_load_acc(uint32_t taddr, int acc2_col, float (&v)[8]) {
+    uint32_t x[8], y[8];
+    tmem_ld8(taddr, x);
+    tmem_ld8(taddr + static_cast<uint32_t>(acc2_col), y);
+    tmem_ld_wait();
+#pragma unroll
+    for (int j = 0; j < 8; ++j) v[j] = __uint_as_float(x[j]) + __uint_as_float(y[j]);
+}
+
+__device__ __forceinline__ float swiglu_f32(float gate, float up) { return (gate / (1.0f + expf(-gate))) * up; }
+
+// NV tokens m0 .. m0 + NV - 1 of weight row n (acc) to the output.  All lanes of a warp call it with consecutive rows and
+// the same tokens.  SWIGLU: rows 2i / 2i + 1 are gate and up of one output; the lane pair exchanges one value per two
+// tokens, then the even lane finishes the first token and the odd lane the second.
+template <int MODE, int NV>
+__device__ __forceinline__ void stream_store(const StreamArgs& a, int t, int n, bool row_ok, int m0, const float (&acc)[NV], const __half (&res)[NV]) {
+    const size_t ld = static_cast<size_t>(a.out_ld[t]);
+    if constexpr (MODE == kSwiglu) {
+        const int odd = n & 1;
+        __half* out = a.out[t] + static_cast<size_t>(m0 + odd) * ld + (n >> 1);
+#pragma unroll
+        for (int q = 0; q < NV; q += 2) {
+            const float other = __shfl_xor_sync(0xFFFFFFFFu, odd ? acc[q] : acc[q + 1], 1);
+            const float y = odd ? swiglu_f32(other, acc[q + 1]) : swiglu_f32(acc[q], other);
+            if (row_ok && m0 + q + odd < a.M) *out = __float2half_rn(y);
+            out += 2 * ld;
+        }
+    } else {
+        __half* out = a.out[t] + static_cast<size_t>(m0) * ld + n;
+#pragma unroll
+        for (int q = 0; q < NV; ++q) {
+            if (row_ok && m0 + q < a.M) {
+                __half y = __float2half_rn(acc[q]);
+                if constexpr (MODE == kPlain) {
+                    if (a.residual != nullptr) y = __hadd(y, res[q]);
+                }
+                *out = y;
+                if constexpr (MODE == kPlain) {
+                    for (int p = 0; p < a.num_peers; ++p) a.peer_out[p][static_cast<size_t>(m0 + q) * ld + n] = y;
+                }
+            }
+            out += ld;
+        }
+    }
+}
+template <int MODE, int NV>
+__device__ __forceinline__ void stream_load_residual(const StreamArgs& a, int t, int n, bool row_ok, int m0, __half (&res)[NV]) {
+#pragma unroll
+    for (int q = 0; q < NV; ++q) res[q] = __half(0.0f);
+    if constexpr (MODE == kPlain) {
+        if (a.residual != nullptr) {
+#pragma unroll
+            for (int q = 0; q < NV; ++q)
+                if (row_ok && m0 + q < a.M) res[q] = a.residual[static_cast<size_t>(m0 + q) * a.out_ld[t] + n];
+        }
+    }
+}
+
+// All lanes look at the barrier; only if it is still open one lane polls for the warp.
+__device__ __forceinline__ bool group_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag, int lane) {
+    if (__all_sync(0xFFFFFFFFu, mbar_test_wait(bar, parity))) return true;
+    return warp_wait(bar, parity, abort_flag, lane);
+}
+
+template <int MODE>
+__global__ void __launch_bounds__(kStThreads, 1) gemm_w4a16_tc_stream_kernel(const __grid_constant__ StreamArgs a) {
+    extern __shared__ uint8_t smem_raw_base[];
+    uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw_base) + 1023) & ~uintptr_t(1023));
+    const int T = a.T, NS = a.slots, SR = a.raw_slots, K = a.K;
+    const int x_box = T * 128, x_bytes = 2 * x_box;      // a step's tokens: two boxes of 64 k
+    uint8_t* s_x = smem;
+    uint8_t* s_raw = s_x + a.x_mem * x_bytes;
+    uint64_t* s_bar = reinterpret_cast<uint64_t*>(s_raw + SR * kStRawBytes);
+    const uint32_t bar0 = smem_u32(s_bar);
+    auto raw_full = [&](int i) { return bar0 + 8u * i; };
+    auto raw_empty = [&](int i) { return bar0 + 8u * (kStMaxRaw + i); };
+    auto full = [&](int i) { return bar0 + 8u * (2 * kStMaxRaw + i); };          // weights dequantised and tokens landed
+    auto empty = [&](int i) { return bar0 + 8u * (2 * kStMaxRaw + kStMaxSlots + i); };
+    constexpr int kBars = 2 * kStMaxRaw + 2 * kStMaxSlots + 2;
+    const uint32_t accum_full = bar0 + 8u * (kBars - 2), part_full = bar0 + 8u * (kBars - 1);
+    uint32_t* s_tmem = reinterpret_cast<uint32_t*>(s_bar + kBars);
+    volatile int* s_abort = reinterpret_cast<volatile int*>(s_tmem + 1);
+    int* s_issued = reinterpret_cast<int*>(s_tmem + 2);           // steps whose copies were issued: weights, tokens
+    __half* s_scale = reinterpret_cast<__half*>(s_tmem + 4);      // [step][128 rows]
+
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    int t = 0, tile = blockIdx.x;
+    if constexpr (MODE == kQkv) {
+        if (tile >= a.tiles[0]) { tile -= a.tiles[0]; t = 1; }
+        if (t == 1 && tile >= a.tiles[1]) { tile -= a.tiles[1]; t = 2; }
+    }
+    const int n0 = tile * kTileRows, rows_t = a.rows[t], m0 = blockIdx.y * T;
+    // K range: whole steps, spread over the cluster as evenly as they go
+    const int ksplit = a.ksplit, krank = static_cast<int>(blockIdx.z);
+    const int G = K / kGroup, per = G / ksplit, rest = G - per * ksplit;
+    const int st0 = krank * per + min(krank, rest), nst = per + (krank < rest ? 1 : 0);
+
+    // The group scales of the 128 rows are the first loads: behind the weight stream they would arrive last.
+    constexpr int kScaleRegs = 4;
+    const __half* sc = a.scales[t];
+    auto load_scale = [&](int idx) -> __half {
+        const int rr = idx / nst, g = idx - rr * nst, row = n0 + rr;
+        return row < rows_t ? __ldg(sc + static_cast<size_t>(row) * G + st0 + g) : __half(0.0f);
+    };
+    auto store_scale = [&](int idx, __half v) {
+        const int rr = idx / nst, g = idx - rr * nst;
+        s_scale[g * kTileRows + rr] = v;
+    };
+    __half sreg[kScaleRegs];
+    if (warp < kStDqWarps) {
+#pragma unroll
+        for (int q = 0; q < kScaleRegs; ++q)
+            if (tid + q * kStDqThreads < kTileRows * nst) sreg[q] = load_scale(tid + q * kStDqThreads);
+    } else if (warp == kStDqWarps + 1) {
+        // barriers (a lane each), then the ring of packed weights
+        if (lane == 0) { tma_prefetch_desc(&a.tmap_w[t]); *s_abort = 0; s_issued[0] = min(SR, nst); s_issued[1] = 0; }
+        if (lane == 1) tma_prefetch_desc(&a.tmap_x);
+        if (lane < SR) { mbar_init(raw_full(lane), 1); mbar_init(raw_empty(lane), 4); }
+        if (lane < NS) { mbar_init(full(lane), 4 + 1); mbar_init(empty(lane), 1); }
+        if (lane == 31) {
+            mbar_init(accum_full, 1);
+            mbar_init(part_full, 1);
+            const int mine = max(0, min(a.tpr, T - krank * a.tpr));
+            if (ksplit > 1) mbar_arrive_expect_tx(part_full, static_cast<uint32_t>(ksplit * mine * kTileRows * 4));
+        }
+        fence_barrier_init();
+        fence_proxy_async_smem();
+        __syncwarp();
+        if (lane == 0) {
+            const int first = min(SR, nst);
+            for (int i = 0; i < first; ++i) {
+                mbar_arrive_expect_tx(raw_full(i), kStRawBytes);
+                tma_load_2d(smem_u32(s_raw + i * kStRawBytes), &a.tmap_w[t], (st0 + i) * 64, n0, raw_full(i));
+            }
+        }
+        __syncwarp();
+    } else if (warp == kStDqWarps) {
+        // Blocks while a CTA of the previous launch on this SM holds it; the next launch may only follow once every CTA of
+        // this one has its share, or a CTA of the next could take it first and wait for this launch with it.
+        tmem_alloc(smem_u32(s_tmem), 512);
+        tmem_relinquish();
+        pdl_release_dependents();
+    }
+    tc_fence_before();
+    // (the loader only announces its barriers: it goes on to wait for the previous kernel, the others do not)
+    if (warp == kStDqWarps + 1) asm volatile("bar.arrive 2, %0;" ::"n"(kStThreads) : "memory");
+    else asm volatile("bar.sync 2, %0;" ::"n"(kStThreads) : "memory");
+    tc_fence_after();
+    const bool own_part = a.part_offset != 0;      // partials in memory of their own: they may come while the rings are in use
+    if (ksplit > 1 && own_part) cluster_arrive();
+
+    if (warp < kStDqWarps) {
+        const uint32_t tmem_base = *s_tmem;
+#pragma unroll
+        for (int q = 0; q < kScaleRegs; ++q)
+            if (tid + q * kStDqThreads < kTileRows * nst) store_scale(tid + q * kStDqThreads, sreg[q]);
+        for (int idx = tid + kScaleRegs * kStDqThreads; idx < kTileRows * nst; idx += kStDqThreads) store_scale(idx, load_scale(idx));
+        asm volatile("bar.sync 1, %0;" ::"n"(kStDqThreads) : "memory");
+
+        const int r = (warp & 3) * 32 + lane, part = warp >> 2;
+        const uint32_t lane_base = tmem_base + (static_cast<uint32_t>((warp & 3) * 32) << 16);
+        const int swz = (r >> 1) & 3;            // 64-byte swizzle: 16-byte chunk index xor row pair
+        const uint8_t* raw_lane = s_raw + r * 64;
+        bool ok = true;
+        int rs = part;                           // ring slot of this group's next step
+        uint32_t rph = 0;
+        int slot = part;                         // A slot of the step, and the parity its previous use completes
+        uint32_t eph = 1;
+        if (rs >= SR) { rs -= SR; rph ^= 1; }    // (SR is a multiple of 4: never for the first step)
+        for (int s = part; s < nst; s += kStGroups) {
+            const __half sc1 = s_scale[s * kTileRows + r];
+            ok = group_wait(raw_full(rs), rph, s_abort, lane);
+            if (!ok) break;
+            const uint8_t* raw_row = raw_lane + rs * kStRawBytes;
+            ok = group_wait(empty(slot), eph, s_abort, lane);
+            if (!ok) break;
+            tc_fence_after();
+            const uint32_t a_lane = lane_base + static_cast<uint32_t>(a.a_col + slot * kStACols);
+            const __half2 sc2 = __half2half2(sc1);
+            if (__all_sync(0xFFFFFFFFu, __habs(sc1) < __float2half_rn(0.0624f))) {
+                const __half2 k10 = __float2half2_rn(1024.0f);
+                const __half2 s20 = __hmul2(__hmul2(sc2, k10), k10), m8s = __hmul2(sc2, __float2half2_rn(-8.0f));
+#pragma unroll 2
+                for (int c = 0; c < 4; ++c) {
+                    const uint4 w = *reinterpret_cast<const uint4*>(raw_row + ((c ^ swz) << 4));
+                    uint32_t cols[16];
+                    dequant_word_small_scale(w.x, s20, m8s, cols);
+                    dequant_word_small_scale(w.y, s20, m8s, cols + 4);
+                    dequant_word_small_scale(w.z, s20, m8s, cols + 8);
+                    dequant_word_small_scale(w.w, s20, m8s, cols + 12);
+                    tmem_st16(a_lane + 16u * c, cols);
+                }
+            } else {
+#pragma unroll 1
+                for (int c = 0; c < 4; ++c) {
+                    const uint4 w = *reinterpret_cast<const uint4*>(raw_row + ((c ^ swz) << 4));
+                    const uint32_t words[4] = {w.x, w.y, w.z, w.w};
+                    uint32_t cols[16];
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) {
+                        __half2 h[4];
+                        dequant_word_fp16(words[i], sc2, h);
+#pragma unroll
+                        for (int q = 0; q < 4; ++q) cols[4 * i + q] = *reinterpret_cast<const uint32_t*>(&h[q]);
+                    }
+                    tmem_st16(a_lane + 16u * c, cols);
+                }
+            }
+            tmem_st_wait();
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) {
+                mbar_arrive(full(slot));
+                mbar_arrive(raw_empty(rs));
+            }
+            rs += kStGroups;
+            if (rs >= SR) { rs -= SR; rph ^= 1; }
+            slot += kStGroups;
+            if (slot >= NS) { slot -= NS; eph ^= 1; }
+        }
+        // ---------------- epilogue: thread = weight row, registers = tokens ----------------
+        pdl_wait_prior_grids();                  // the previous kernels' reads of the outputs and writes of the residual
+        const int n = n0 + r;
+        const bool row_ok = n < rows_t;
+        if (ksplit == 1) {
+            // eight tokens a round (a loop, not unrolled: this code runs once and its instructions have to be fetched)
+            __half res[8];
+            stream_load_residual<MODE>(a, t, n, row_ok, m0 + part * 8, res);
+            if (ok) ok = warp_wait(accum_full, 0, s_abort, lane);
+            tc_fence_after();
+            if (ok) {
+#pragma unroll 1
+                for (int c0 = part * 8; c0 < T; c0 += 32) {
+                    float acc[8];
+                    stream_load_acc(lane_base + static_cast<uint32_t>(c0), a.acc2_col, acc);
+                    stream_store<MODE>(a, t, n, row_ok, m0 + c0, acc, res);
+                    if (c0 + 32 < T) stream_load_residual<MODE>(a, t, n, row_ok, m0 + c0 + 32, res);
+                }
+            }
+        } else {
+            // Tokens [rank * tpr, (rank + 1) * tpr) are finished by that rank; partials land at [source][token / 4][row][4].
+            // They are sent whatever the waits returned: a peer that waits for them must not be left alone.
+            const int tpr = a.tpr;
+            uint8_t* s_part = smem + a.part_offset;
+            __half res[4];
+            stream_load_residual<MODE>(a, t, n, row_ok && part * 4 < tpr, m0 + krank * tpr + part * 4, res);
+            if (ok) ok = warp_wait(accum_full, 0, s_abort, lane);
+            tc_fence_after();
+            if (!own_part) cluster_arrive();     // this CTA's rings are free
+            cluster_wait();
+            const uint32_t part0 = smem_u32(s_part) + static_cast<uint32_t>(krank * (tpr / 4) * kTileRows + r) * 16u;
+#pragma unroll 1
+            for (int c0 = part * 8; c0 < T; c0 += 32) {
+                float v[8];
+                stream_load_acc(lane_base + static_cast<uint32_t>(c0), a.acc2_col, v);
+#pragma unroll
+                for (int q = 0; q < 8; q += 4) {
+                    const int owner = (c0 + q) / tpr, k = c0 + q - owner * tpr;
+                    st_async_16(cluster_map_shared(part0 + static_cast<uint32_t>((k >> 2) * kTileRows) * 16u, static_cast<uint32_t>(owner)),
+                                cluster_map_shared(part_full, static_cast<uint32_t>(owner)), __float_as_uint(v[q]), __float_as_uint(v[q + 1]),
+                                __float_as_uint(v[q + 2]), __float_as_uint(v[q + 3]));
+                }
+            }
+            bool have = true;
+            if (lane == 0) have = wait_regardless(part_full, 0, 4 * kWaitLimit);
+            have = __shfl_sync(0xFFFFFFFFu, have ? 1 : 0, 0) != 0;
+            if (!have && lane == 0) { *s_abort = 1; atomicAdd(&g_tc_wait_timeouts, 1u); }
+            if (have) {
+#pragma unroll 1
+                for (int k = part * 4; k < tpr; k += 16) {
+                    const int m = krank * tpr + k;
+                    if (m >= T) break;
+                    float acc[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+#pragma unroll
+                    for (int s = 0; s < kStMaxSplit; ++s) {
+                        if (s < ksplit) {
+                            const float4 p = *reinterpret_cast<const float4*>(s_part + static_cast<size_t>((s * (tpr / 4) + (k >> 2)) * kTileRows + r) * 16);
+                            acc[0] += p.x; acc[1] += p.y; acc[2] += p.z; acc[3] += p.w;
+                        }
+                    }
+                    stream_store<MODE>(a, t, n, row_ok, m0 + m, acc, res);
+                    if (k + 16 < tpr) stream_load_residual<MODE>(a, t, n, row_ok, m0 + m + 16, res);
+                }
+            }
+        }
+    } else {
+        if (warp == kStDqWarps) {
+            // ---------------- MMA issue: one thread ----------------
+            const uint32_t tmem_base = *s_tmem;
+            if (elect_one()) {
+                const uint32_t idesc = make_idesc(T);
+                const uint64_t b_desc0 = make_smem_desc(smem_u32(s_x));
+                const uint32_t b_step = static_cast<uint32_t>(x_bytes) >> 4, b_half = static_cast<uint32_t>(x_box) >> 4;
+                int slot = 0;
+                uint32_t ph = 0;
+                uint64_t b_desc = b_desc0;
+                uint32_t a_tmem = tmem_base + static_cast<uint32_t>(a.a_col);
+                bool ready = mbar_test_wait(full(0), 0);
+                for (int s = 0; s < nst; ++s) {
+                    if (!ready && !mbar_wait(full(slot), ph, s_abort)) break;
+                    tc_fence_after();
+                    const uint32_t bar_empty = empty(slot);
+                    const uint32_t tmem_d = tmem_base + ((s & 1) != 0 ? static_cast<uint32_t>(a.acc2_col) : 0u);
+#pragma unroll
+                    for (int ks = 0; ks < kGroup / 16; ++ks)
+                        tc_mma_f16_ts(tmem_d, a_tmem + 8u * ks, b_desc + (ks >= 4 ? b_half : 0u) + static_cast<uint32_t>(2 * (ks & 3)), idesc,
+                                      (ks != 0 || s >= 2) ? 1u : 0u);
+                    tc_commit(bar_empty);
+                    a_tmem += kStACols;
+                    b_desc += b_step;
+                    if (++slot == NS) { slot = 0; ph ^= 1; b_desc = b_desc0; a_tmem = tmem_base + static_cast<uint32_t>(a.a_col); }
+                    ready = mbar_test_wait(full(slot), ph);
+                }
+                tc_commit(accum_full);   // also after a wait that ran out: nothing may be in flight at the end
+            }
+        } else if (lane == 0) {
+            // ---------------- loader: tokens as soon as the previous kernel is through, then both rings as they empty ----------------
+            int iw = min(SR, nst), ix = 0, ws = 0, xs = 0;
+            uint32_t wph = 0, xph = 0;
+            pdl_wait_prior_grids();
+            for (unsigned spins = 0; iw < nst || ix < nst;) {
+                bool moved = false;
+                if (ix < nst && (ix < NS || mbar_test_wait(empty(xs), xph))) {
+                    mbar_arrive_expect_tx(full(xs), static_cast<uint32_t>(x_bytes));
+                    tma_load_2d(smem_u32(s_x + xs * x_bytes), &a.tmap_x, (st0 + ix) * kGroup, m0, full(xs));
+                    tma_load_2d(smem_u32(s_x + xs * x_bytes + x_box), &a.tmap_x, (st0 + ix) * kGroup + kBK, m0, full(xs));
+                    if (++xs == NS) { xs = 0; if (ix >= NS) xph ^= 1; }
+                    ++ix;
+                    moved = true;
+                }
+                if (iw < nst && mbar_test_wait(raw_empty(ws), wph)) {
+                    mbar_arrive_expect_tx(raw_full(ws), kStRawBytes);
+                    tma_load_2d(smem_u32(s_raw + ws * kStRawBytes), &a.tmap_w[t], (st0 + iw) * 64, n0, raw_full(ws));
+                    if (++ws == SR) { ws = 0; wph ^= 1; }
+                    ++iw;
+                    moved = true;
+                }
+                if (moved) { spins = 0; continue; }
+                if (*s_abort) break;
+                if (++spins > 2048) __nanosleep(64);
+                if (spins > kWaitLimit) { *s_abort = 1; atomicAdd(&g_tc_wait_timeouts, 1u); break; }
+            }
+            s_issued[0] = iw;
+            s_issued[1] = ix;
+        }
+        __syncwarp();
+        if (ksplit > 1) {
+            if (!own_part) cluster_arrive();
+            cluster_wait();
+        }
+    }
+    tc_fence_before();
+    __syncthreads();
+    if (*s_abort) {          // a bounded wait ran out: what is in flight has to land before the memory goes (bounded too)
+        if (tid == 0) {
+            for (int i = 0; i < min(SR, s_issued[0]); ++i) wait_regardless(raw_full(i), static_cast<uint32_t>((s_issued[0] - 1 - i) / SR) & 1u, kWaitLimit);
+            wait_regardless(accum_full, 0, kWaitLimit);
+            __nanosleep(100000);     // token copies whose slot never filled up have no barrier phase of their own to wait for
+        }
+        __syncthreads();
+    }
+    if (warp == kStDqWarps) tmem_dealloc(*s_tmem, 512);
+}
+
+// ---- host side of the streaming form ----
+// How a launch is cut: token tiles of T, K split `ksplit` ways, ring sizes.  False where it does not fit.
+bool plan_stream(int steps, StreamArgs* a, size_t* smem) {
+    const int T = a->T;
+    a->slots = T <= 64 ? 6 : 4;
+    a->acc2_col = T <= 64 ? 64 : 128;
+    a->a_col = 2 * a->acc2_col;
+    a->tpr = ((T + a->ksplit - 1) / a->ksplit + 3) & ~3;
+    const size_t part_bytes = a->ksplit > 1 ? static_cast<size_t>(a->ksplit) * a->tpr * kTileRows * 4 : 0;
+    const size_t budget = 226 * 1024;
+    const size_t fixed = 1024 + (2 * kStMaxRaw + 2 * kStMaxSlots + 2) * 8 + 16 + static_cast<size_t>(steps) * kTileRows * 2;
+    for (; a->slots >= 4; a->slots -= 2) {
+        a->x_mem = std::min(a->slots, steps);
+        const size_t x_bytes = static_cast<size_t>(a->x_mem) * T * 256;
+        for (int own = part_bytes ? 1 : 0; own >= 0; --own) {
+            const size_t extra = own ? part_bytes + 128 : 0;
+            int raw = std::min(kStMaxRaw, (steps + 3) & ~3);
+            while (raw > 4 && fixed + extra + x_bytes + static_cast<size_t>(raw) * kStRawBytes > budget) raw -= 4;
+            const size_t ring = x_bytes + static_cast<size_t>(raw) * kStRawBytes;
+            if (fixed + extra + ring > budget) continue;
+            if (!own && ring < part_bytes) continue;     // the partials go on top of the rings
+            a->raw_slots = raw;
+            const size_t used = (fixed - 1024 + ring + 127) / 128 * 128;
+            a->part_offset = own ? static_cast<int>(used) : 0;
+            // At least half an SM, so that no SM gets two CTAs of a launch: smaller ones pile up on the SMs that the previous
+            // launch leaves idle (measured on one layer at 47 tokens: 33 instead of 29 us).
+            *smem = std::max<size_t>(1024 + used + (own ? part_bytes : 0), 116 * 1024);
+            return true;
+        }
+    }
+    return false;
+}

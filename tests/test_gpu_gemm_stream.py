@@ -1,0 +1,59 @@
+"""The weight-streaming tcgen05 kernel (17-256 tokens) at the edges of its tiles: token tiles of 16 to 128, one and two of
+them, K ranges of two steps and of many, split and not, rows past the last whole tile, scales on both sides of the limit
+of the short dequantisation."""
+import numpy as np
+import pytest
+
+import oracle
+from tests import util
+
+pytestmark = pytest.mark.gpu
+torch = pytest.importorskip("torch")
+
+
+@pytest.mark.parametrize("M,N,K,scale_max,res", [
+    (17, 128, 256, 0.02, False), (47, 1536, 8960, 0.02, True), (48, 520, 512, 0.5, True), (64, 2048, 1536, 0.02, False),
+    (65, 20000, 256, 0.02, True), (112, 384, 2304, 0.07, True), (115, 1536, 1536, 0.02, True), (128, 17920, 768, 0.02, False),
+    (129, 1536, 1536, 0.5, True), (203, 17920, 1536, 0.02, False), (255, 132, 8960, 0.02, True), (256, 300, 1024, 0.02, False),
+])
+def test_stream_kernel_matches_oracle(M, N, K, scale_max, res):
+    import qwen_engine_b200 as ops
+    from qwen_engine_b200 import synth
+    seed = M * 31 + N + K
+    rng = np.random.default_rng(seed)
+    qw, x = synth.packed_weights(seed, "s", N, K), synth.activations(seed, "s", M, K)
+    sc = rng.uniform(0.002, scale_max, size=(N, K // 128)).astype(np.float16)
+    r = rng.standard_normal((M, N)).astype(np.float16) if res else None
+    y = torch.full((M * N + 64,), float("nan"), dtype=torch.float16, device="cuda")
+    ops.launch_gemm_prefill_w4a16(util.to_dev(qw), util.to_dev(sc), util.to_dev(x), util.to_dev(r) if res else None, y, M, N, K)
+    torch.cuda.synchronize()
+    got = util.to_np(y)
+    assert np.isnan(got[M * N:]).all(), "wrote past the output"
+    pick = lambda n: np.unique(np.concatenate([[0, n - 1], rng.choice(n, size=min(n, 24), replace=False)])).astype(np.int32)  # noqa: E731
+    m_idx, n_idx = pick(M), pick(N)
+    ref64, _ = oracle.gemm_prefill(qw, sc, x, m_idx, n_idx, residual=r)
+    acc = ref64 - r[np.ix_(m_idx, n_idx)].astype(np.float64) if res else None
+    util.assert_fp16_close(got[:M * N].reshape(M, N)[np.ix_(m_idx, n_idx)], ref64, what=f"{M}x{N}x{K}", magnitude=acc)
+    assert ops.debug_counter(0) == 0
+
+
+@pytest.mark.parametrize("M", [33, 130])
+def test_stream_kernel_swiglu_and_qkv_routing(M):
+    import qwen_engine_b200 as ops
+    from qwen_engine_b200 import synth
+    H, I = 512, 640
+    x = synth.activations(M, "x", M, H)
+    qw, sc = synth.packed_weights(M, "gu", 2 * I, H), synth.scales(M, "gu", 2 * I, H)
+    y = torch.empty((M, I), dtype=torch.float16, device="cuda")
+    ops.launch_gemm_prefill_dual_gate_up_swiglu_w4a16(util.to_dev(qw), util.to_dev(sc), util.to_dev(x), y, M, None, H, I)
+    m_idx, n_idx = np.arange(0, M, 7, dtype=np.int32), np.arange(0, I, 13, dtype=np.int32)
+    ref64, _ = oracle.gemm_prefill(qw, sc, x, m_idx, n_idx, swiglu=True)
+    util.assert_fp16_close(util.to_np(y)[np.ix_(m_idx, n_idx)], ref64, what="swiglu")
+    # q, k, v as three tensors of 384, 128 and 128 rows = the rows of one
+    qkv = [(util.to_dev(qw[a:b].copy()), util.to_dev(sc[a:b].copy()), torch.empty((M, b - a), dtype=torch.float16, device="cuda"))
+           for a, b in ((0, 384), (384, 512), (512, 640))]
+    ops.launch_gemm_prefill_qkv_w4a16(ops.QKVProjectionView(*[t for p in qkv for t in p]), util.to_dev(x), M, None, H, 3, 1, 128)
+    n_idx = np.arange(0, 640, 11, dtype=np.int32)
+    ref64, _ = oracle.gemm_prefill(qw, sc, x, m_idx, n_idx)
+    got = np.concatenate([util.to_np(p[2]) for p in qkv], axis=1)
+    util.assert_fp16_close(got[np.ix_(m_idx, n_idx)], ref64, what="qkv")

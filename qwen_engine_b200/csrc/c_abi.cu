@@ -30,6 +30,20 @@ int option(int which) {
     init_options();
     return (which > 0 && which < W4A16_OPT_COUNT_) ? g_options[which].load(std::memory_order_relaxed) : 0;
 }
+int max_active_clusters(const void* kernel, int block, size_t smem, int cluster) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(static_cast<unsigned>(cluster));
+    cfg.blockDim = dim3(static_cast<unsigned>(block));
+    cfg.dynamicSmemBytes = smem;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = static_cast<unsigned>(cluster); attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    int n = 0;
+    if (cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) != cudaSuccess) { cudaGetLastError(); n = 0; }
+    return n;
+}
 bool pdl_enabled() { return option(W4A16_OPT_PDL) != 0; }
 
 int ensure_device_ready(const DeviceInfo** out) {
@@ -610,7 +624,13 @@ int w4a16_gemv_group_dots(const uint32_t* qweight, const int8_t* input_q8, const
 int w4a16_debug_counter(int which, unsigned int* out) {
     if (!out) return W4A16_ERR_INVALID_ARG;
     if (int st = ensure_device_ready(nullptr)) return st;
-    if (which == 0) return gemm_tc_timeouts(out);
+    if (which == 0) {
+        unsigned int tc = 0, mma = 0;
+        if (int st = gemm_tc_timeouts(&tc)) return st;
+        if (int st = gemm_mma_timeouts(&mma)) return st;
+        *out = tc + mma;
+        return 0;
+    }
     if (which == 1) return gemv_copy_timeouts(out);
     return W4A16_ERR_INVALID_ARG;
 }

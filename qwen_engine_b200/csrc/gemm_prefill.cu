@@ -79,71 +79,73 @@ bool plan_v2(const GemmArgs& g, int units, int sm_count, SmallMPlan* out, int* U
 }
 
 // ---- few-token mma.sync form (gemm_smallm_mma_kernel) ----
-template <int MODE, int U>
-cudaError_t launch_mma_nt(const SmallMArgs& a, const SmallMmaPlan& p, int NT, dim3 grid, dim3 block, size_t smem, cudaStream_t stream) {
-    const bool pdl = pdl_enabled();
-    if (NT == 1) return launch_kernel(gemm_smallm_mma_kernel<MODE, U, 1>, grid, block, smem, stream, pdl, a, p);
-    if (NT == 2) return launch_kernel(gemm_smallm_mma_kernel<MODE, U, 2>, grid, block, smem, stream, pdl, a, p);
-    return launch_kernel(gemm_smallm_mma_kernel<MODE, U, 4>, grid, block, smem, stream, pdl, a, p);
-}
+constexpr size_t kMmaMaxSmem = 200 * 1024;
+using MmaKernel = void (*)(const SmallMArgs, const SmallMmaPlan);
 template <int MODE>
-cudaError_t launch_mma(const SmallMArgs& a, const SmallMmaPlan& p, int U, int NT, dim3 grid, dim3 block, size_t smem, cudaStream_t stream) {
-    if (U == 4) return launch_mma_nt<MODE, 4>(a, p, NT, grid, block, smem, stream);
-    return launch_mma_nt<MODE, 8>(a, p, NT, grid, block, smem, stream);
+MmaKernel mma_kernel_nt(int NT) {
+    return NT == 1 ? gemm_smallm_mma_kernel<MODE, 1> : gemm_smallm_mma_kernel<MODE, 2>;
 }
-template <int MODE, int U, int NT>
+MmaKernel mma_kernel(int mode, int NT) {
+    return mode == kPlain ? mma_kernel_nt<kPlain>(NT) : mode == kQkv ? mma_kernel_nt<kQkv>(NT) : mma_kernel_nt<kSwiglu>(NT);
+}
 cudaError_t raise_mma() {
-    return cudaFuncSetAttribute(gemm_smallm_mma_kernel<MODE, U, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-}
-template <int MODE>
-cudaError_t raise_mma_mode() {
-    cudaError_t e = raise_mma<MODE, 4, 1>();
-    if (e == cudaSuccess) e = raise_mma<MODE, 4, 2>();
-    if (e == cudaSuccess) e = raise_mma<MODE, 4, 4>();
-    if (e == cudaSuccess) e = raise_mma<MODE, 8, 1>();
-    if (e == cudaSuccess) e = raise_mma<MODE, 8, 2>();
-    if (e == cudaSuccess) e = raise_mma<MODE, 8, 4>();
-    return e;
+    for (int mode : {static_cast<int>(kPlain), static_cast<int>(kQkv), static_cast<int>(kSwiglu)})
+        for (int NT : {1, 2}) {
+            cudaError_t e = cudaFuncSetAttribute(reinterpret_cast<const void*>(mma_kernel(mode, NT)), cudaFuncAttributeMaxDynamicSharedMemorySize, kMmaMaxSmem);
+            if (e != cudaSuccess) return e;
+            // the same carve-out for every kernel of a layer: CTAs of two launches share an SM only if they agree on it
+            e = cudaFuncSetAttribute(reinterpret_cast<const void*>(mma_kernel(mode, NT)), cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
+            if (e != cudaSuccess) return e;
+        }
+    return cudaSuccess;
 }
 
-// CTA shape of the mma.sync form.  A warp = 16 MMA rows x one K slice of at most 8 steps of 128; enough slices that
-// about 8 warps per SM exist where the matrix is short, row groups per CTA so that a CTA has up to 8-16 warps while
-// the grid still covers the SMs.  False when the shape does not fit (rows not in whole groups, shared memory).
-bool plan_mma(const GemmArgs& g, int units, int sm_count, SmallMmaPlan* out, int* U, int* NT, size_t* smem) {
-    const int uw = g.mode == kSwiglu ? 8 : 16;
-    if (units % uw) return false;
-    if (g.mode == kQkv && (g.rows[0] % 16 || g.rows[1] % 16 || g.rows[2] % 16)) return false;
-    const int steps = g.K / kGroup;
-    const int groups_total = units / uw;
-    // slices of at most 4 steps where 16 warps allow it (the 4-step form has registers to spare for the token loads)
-    int ksplit = std::max((steps + 3) / 4, (8 * sm_count + groups_total - 1) / groups_total);
-    ksplit = std::min(ksplit, std::min(steps, 16));
-    int per = (steps + ksplit - 1) / ksplit;
-    ksplit = (steps + per - 1) / per;
-    // the whole grid must be resident (16 warps per SM at 128 registers): deeper slices where it would not be
-    while (static_cast<long long>(groups_total) * ksplit > 16LL * sm_count && per < 8) {
-        ++per;
-        ksplit = (steps + per - 1) / per;
-    }
-    if (per > 8 || static_cast<long long>(groups_total) * ksplit > 16LL * sm_count) return false;
-    // every CTA stages all the tokens, so fewer and larger CTAs mean less traffic for them: up to 16 warps per CTA
-    // as long as about one CTA per SM remains
-    int gpc = std::max(1, std::min(8, 16 / ksplit));
-    while (gpc > 1 && groups_total / gpc < (sm_count * 9) / 10) gpc /= 2;
-    int nt = g.M <= 8 ? 1 : (g.M <= 16 ? 2 : 4);
-    auto bytes = [&](int n) {
-        return static_cast<size_t>(g.K / 4) * (8 * n) * 8 + static_cast<size_t>(ksplit) * gpc * n * 4 * 32 * sizeof(float);
-    };
-    while (nt > 1 && bytes(nt) > 100 * 1024) nt /= 2;
-    if (bytes(nt) > 200 * 1024) return false;
-    out->groups_per_cta = gpc;
-    out->ksplit = ksplit;
-    out->steps_per_split = per;
-    out->passes_tokens = 8 * nt;
-    *U = per <= 4 ? 4 : 8;
-    *NT = nt;
-    *smem = bytes(nt);
-    return true;
+struct MmaLaunch {
+    SmallMmaPlan plan{};
+    int NT = 0, grid = 0, block = 0;
+    size_t smem = 0;
+    bool ok = false;
+};
+// How the rows and K are cut: the cheapest of all cuts that keep the whole grid resident (16 warps per SM) by an estimate in
+// cycles: per warp and step 34 + 3 NT issue slots or 16 NT tensor-core cycles, whichever is more, and 300 of latency per
+// step of the chain; the staging of a CTA's tokens at 25 bytes a cycle; 900 for an exchange over a cluster, 1200 more where
+// the clusters would fill nearly every SM (the GPCs' sizes are not multiples of theirs, so the last ones wait: down at 4
+// tokens 6.0 us as 24 clusters of 6, 5.0 as 24 of 5); 500 per further CTA on an SM (they stand in the way of the
+// next launch's); the owner's addition of the slices.
+MmaLaunch plan_mma(int mode, int units, int M, int K, int sm_count) {
+    MmaLaunch best;
+    const int uw = mode == kSwiglu ? 8 : 16, groups = units / uw, G = K / kGroup;
+    if (M > 16) return best;
+    const int NT = M <= 8 ? 1 : 2;
+    double best_cost = 0;
+    for (int rg : {1, 2, 4, 8})
+        for (int ks : {1, 2, 4, 8, 16}) {
+            const int warps = rg * ks;
+            if (warps > 16) continue;
+            for (int S = 1; S <= kMmaMaxCluster; ++S) {
+                const int slices = ks * S, per = (G + slices - 1) / slices;
+                if (slices > G || per > 16) continue;
+                const int blocks = (groups + rg - 1) / rg, ctas = blocks * S, per_sm = (ctas + sm_count - 1) / sm_count;
+                if (per_sm * warps > 16) continue;
+                const int cta_steps = std::min(G, ks * per), own = (rg + S - 1) / S;
+                MmaLaunch c;
+                c.plan.row_groups = rg; c.plan.kslices = ks; c.plan.cluster = S; c.plan.steps = per;
+                c.plan.x_pitch = cta_steps * 256 + 64;
+                c.plan.x_offset = warps * per * kMmaSlot;
+                c.plan.part_offset = c.plan.x_offset + M * c.plan.x_pitch;
+                c.smem = static_cast<size_t>(c.plan.part_offset) + static_cast<size_t>(own) * slices * NT * 512;
+                if (c.smem * per_sm > kMmaMaxSmem) continue;
+                const double cost = static_cast<double>(per_sm) * warps * per * std::max(34.0 + 3 * NT, 16.0 * NT) + 300.0 * per +
+                                    static_cast<double>(per_sm) * M * cta_steps * 256 / 25 + 12.0 * slices * ((own * NT + warps - 1) / warps) +
+                                    (S == 1 ? 0.0 : ctas > 0.85 * per_sm * sm_count ? 2100.0 : 900.0) + 500.0 * (per_sm - 1);
+                if (best.ok && cost >= best_cost) continue;
+                c.NT = NT; c.grid = ctas; c.block = 32 * warps; c.ok = true;
+                if (S > 1 && max_active_clusters(reinterpret_cast<const void*>(mma_kernel(mode, NT)), c.block, c.smem, S) < blocks) continue;
+                best = c;
+                best_cost = cost;
+            }
+        }
+    return best;
 }
 
 }  // namespace
@@ -152,11 +154,13 @@ int gemm_set_attributes() {
     cudaError_t e = raise_v2_mode<kPlain>();
     if (e == cudaSuccess) e = raise_v2_mode<kQkv>();
     if (e == cudaSuccess) e = raise_v2_mode<kSwiglu>();
-    if (e == cudaSuccess) e = raise_mma_mode<kPlain>();
-    if (e == cudaSuccess) e = raise_mma_mode<kQkv>();
-    if (e == cudaSuccess) e = raise_mma_mode<kSwiglu>();
+    if (e == cudaSuccess) e = raise_mma();
     if (e != cudaSuccess) return static_cast<int>(e);
     return gemm_tc_set_attributes();
+}
+
+int gemm_mma_timeouts(unsigned int* out) {
+    return static_cast<int>(cudaMemcpyFromSymbol(out, g_mma_wait_timeouts, sizeof(unsigned int)));
 }
 
 int gemm_launch(GemmArgs g, cudaStream_t stream) {
@@ -183,27 +187,19 @@ int gemm_launch(GemmArgs g, cudaStream_t stream) {
     bool aligned = reinterpret_cast<uintptr_t>(g.x) % 16 == 0;
     for (int t = 0; t < (g.mode == kQkv ? 3 : 1); ++t) aligned = aligned && reinterpret_cast<uintptr_t>(g.qweight[t]) % 16 == 0;
 
-    // Two to sixteen tokens: the weight-streaming kernel with the warp-level MMA (no fixed tcgen05 costs).  Measured on
-    // B200 against the other two forms: faster from 2 tokens on every Qwen shape (QKV: equal to the CUDA-core form up
-    // to 4), and up to 16 tokens as long as they are staged in one pass (K = 8960 holds 8 tokens per pass: from 9 the
-    // tcgen05 kernel wins there).
+    // Two to sixteen tokens: the weight-streaming kernel with the warp-level MMA (no fixed tcgen05 costs).  Rows in whole groups
+    // of 16 (a group of QKV rows from one tensor).
     const int mma_max_opt = option(W4A16_OPT_GEMM_MMA_MAX_TOKENS);
     const int mma_max_m = mma_max_opt > 0 ? mma_max_opt : 16;
-    if (aligned && g.num_peers == 0 && g.M >= std::max(2, tc_min_m_opt) && g.M <= mma_max_m) {
-        SmallMmaPlan mp;
-        int mU = 8, mNT = 1;
-        size_t msmem = 0;
-        if (plan_mma(g, a.units, dev->sm_count, &mp, &mU, &mNT, &msmem) && (mma_max_opt > 0 || g.M <= mp.passes_tokens)) {
-            const dim3 mgrid((a.units / (g.mode == kSwiglu ? 8 : 16) + mp.groups_per_cta - 1) / mp.groups_per_cta);
-            const dim3 mblock(32 * mp.groups_per_cta * mp.ksplit);
-            cudaError_t me;
-            switch (g.mode) {
-                case kPlain: me = launch_mma<kPlain>(a, mp, mU, mNT, mgrid, mblock, msmem, stream); break;
-                case kQkv: me = launch_mma<kQkv>(a, mp, mU, mNT, mgrid, mblock, msmem, stream); break;
-                default: me = launch_mma<kSwiglu>(a, mp, mU, mNT, mgrid, mblock, msmem, stream); break;
-            }
-            return static_cast<int>(me);
-        }
+    const bool whole_groups = a.units % (g.mode == kSwiglu ? 8 : 16) == 0 && (g.mode != kQkv || (g.rows[0] % 16 == 0 && g.rows[1] % 16 == 0 && g.rows[2] % 16 == 0));
+    bool scale_pairs = true;
+    for (int t = 0; t < (g.mode == kQkv ? 3 : 1); ++t) scale_pairs = scale_pairs && reinterpret_cast<uintptr_t>(g.scales[t]) % 4 == 0;
+    if (aligned && scale_pairs && whole_groups && g.num_peers == 0 && g.M >= std::max(2, tc_min_m_opt) && g.M <= std::min(mma_max_m, 16)) {
+        static PlanCache<MmaLaunch> plans;
+        const MmaLaunch m = plans.get(plan_key(g.mode, g.M, g.K, a.units), [&] { return plan_mma(g.mode, a.units, g.M, g.K, dev->sm_count); });
+        if (m.ok)
+            return static_cast<int>(launch_kernel_cluster(mma_kernel(g.mode, m.NT), dim3(m.grid), dim3(m.block), m.smem, stream, pdl_enabled(),
+                                                          dim3(static_cast<unsigned>(m.plan.cluster), 1, 1), a, m.plan));
     }
     if ((g.M >= tc_min_m || g.num_peers > 0) && gemm_tc_supported(g)) return gemm_tc_launch(g, dev->sm_count, stream);
     if (g.num_peers > 0) return W4A16_ERR_SHAPE;   // peer stores exist in the tensor-core form only

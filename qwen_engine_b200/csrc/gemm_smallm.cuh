@@ -31,6 +31,19 @@ __device__ __forceinline__ void dequant_word_fp16(uint32_t packed, __half2 scale
     out[3] = __hmul2(__hsub2(*reinterpret_cast<__half2*>(&h67), bias), scale2);
 }
 
+// (q - 8) * s of one packed word with one rounding, as dequant_word_fp16, in 11 instructions instead of 15: a nibble at bits
+// 4..7 of a half is the subnormal q * 2^-20, so fma(q * 2^-20, s * 2^20, -8 s) is the whole conversion; both constants are
+// exact while s * 2^20 is finite (s < 0.0624; larger scales take dequant_word_fp16).
+__device__ __forceinline__ void dequant_word_small_scale(uint32_t packed, __half2 s20, __half2 m8s, uint32_t* out) {
+    const uint32_t lo = (packed << 4) & 0xF0F0F0F0u, hi = packed & 0xF0F0F0F0u;
+    const uint32_t h[4] = {__byte_perm(lo, 0, 0x4140), __byte_perm(lo, 0, 0x4342), __byte_perm(hi, 0, 0x4140), __byte_perm(hi, 0, 0x4342)};
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const __half2 v = __hfma2(*reinterpret_cast<const __half2*>(&h[i]), s20, m8s);
+        out[i] = *reinterpret_cast<const uint32_t*>(&v);
+    }
+}
+
 struct SmallMArgs {
     GemmArgs g;
     int units;          // output rows (PLAIN/QKV) or pairs (SWIGLU)

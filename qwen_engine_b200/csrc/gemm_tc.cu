@@ -1140,63 +1140,39 @@ bool gemm_tc_supported(const GemmArgs& g) {
 namespace {
 constexpr int kStreamDoesNotFit = -1000;     // a K range whose group scales and rings are beyond a CTA's shared memory
 template <int MODE>
-int stream_active_clusters(int ksplit, size_t smem) {
-    static std::mutex mu;
-    static std::vector<std::pair<uint64_t, int>> cache;
-    int dev = 0;
-    cudaGetDevice(&dev);
-    const uint64_t key = (static_cast<uint64_t>(dev) << 48) ^ (static_cast<uint64_t>(ksplit) << 32) ^ static_cast<uint64_t>(smem);
-    std::lock_guard<std::mutex> lock(mu);
-    for (const auto& kv : cache)
-        if (kv.first == key) return kv.second;
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(1, 1, static_cast<unsigned>(ksplit));
-    cfg.blockDim = dim3(kStThreads);
-    cfg.dynamicSmemBytes = smem;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = 1; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = static_cast<unsigned>(ksplit);
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    int n = 0;
-    if (cudaOccupancyMaxActiveClusters(&n, gemm_w4a16_tc_stream_kernel<MODE>, &cfg) != cudaSuccess) { cudaGetLastError(); n = 0; }
-    cache.emplace_back(key, n);
-    return n;
-}
-template <int MODE>
 int launch_stream(StreamArgs& a, const __half* x, int tiles, int sm_count, cudaStream_t stream) {
     // Token tiles and K slices, two steps each at least, within one CTA per SM where that is possible.  Estimated cycles of a
     // CTA, from measurements on B200: 400 a step of dequantisation or 4 T of MMA, whichever is longer; the exchange of
     // partials at 18 bytes a cycle with its latency; 25 a token for the epilogue.
-    const int steps = a.K / kGroup;
-    StreamArgs best = a;
-    size_t smem = 0, best_smem = 0;
-    double best_cost = 0;
-    const int ts_min = (a.M + 127) / 128, ts_max = (a.M + 15) / 16;
-    for (int ts = ts_min; ts <= ts_max; ++ts) {
-        const int T = ((a.M + ts - 1) / ts + 15) & ~15;
-        if (ts > ts_min && ((a.M + T - 1) / T != ts || tiles * ts > sm_count)) continue;
-        for (int split = std::max(1, std::min({kStMaxSplit, sm_count / (tiles * ts), steps / 2})); split >= 1; --split) {
-            a.T = T;
-            a.ksplit = split;
-            const int per = (steps + split - 1) / split;
-            const double cost = per * std::max(400.0, 4.0 * T) + (split > 1 ? 1500.0 + T * 512.0 * (split - 1) / split / 18.0 + 25.0 * T / split : 25.0 * T);
-            if (best_smem != 0 && cost >= best_cost) continue;
-            if (!plan_stream(per, &a, &smem)) continue;
-            if (split > 1 && stream_active_clusters<MODE>(split, smem) < tiles * ts) continue;
-            best = a;
-            best_smem = smem;
-            best_cost = cost;
+    static PlanCache<StreamPlan> plans;
+    const StreamPlan plan = plans.get(plan_key(MODE, a.M, a.K, tiles), [&] {
+        const int steps = a.K / kGroup;
+        StreamPlan best;
+        double best_cost = 0;
+        const int ts_min = (a.M + 127) / 128, ts_max = (a.M + 15) / 16;
+        for (int ts = ts_min; ts <= ts_max; ++ts) {
+            const int T = ((a.M + ts - 1) / ts + 15) & ~15;
+            if (ts > ts_min && ((a.M + T - 1) / T != ts || tiles * ts > sm_count)) continue;
+            for (int split = std::max(1, std::min({kStMaxSplit, sm_count / (tiles * ts), steps / 2})); split >= 1; --split) {
+                const int per = (steps + split - 1) / split;
+                const double cost = per * std::max(400.0, 4.0 * T) + (split > 1 ? 1500.0 + T * 512.0 * (split - 1) / split / 18.0 + 25.0 * T / split : 25.0 * T);
+                if (best.smem != 0 && cost >= best_cost) continue;
+                StreamPlan p;
+                if (!plan_stream(T, split, per, &p)) continue;
+                if (split > 1 && max_active_clusters(reinterpret_cast<const void*>(gemm_w4a16_tc_stream_kernel<MODE>), kStThreads, p.smem, split) < tiles * ts) continue;
+                best = p;
+                best_cost = cost;
+            }
         }
-    }
-    if (best_smem == 0) return kStreamDoesNotFit;
-    a = best;
-    smem = best_smem;
+        return best;
+    });
+    if (plan.smem == 0) return kStreamDoesNotFit;
+    a.p = plan;
     if (!encode_2d(&a.tmap_x, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, x, static_cast<uint64_t>(a.K), static_cast<uint64_t>(a.M),
-                   static_cast<uint64_t>(a.K) * 2, kBK, static_cast<uint32_t>(a.T)))
+                   static_cast<uint64_t>(a.K) * 2, kBK, static_cast<uint32_t>(plan.T)))
         return W4A16_ERR_INVALID_ARG;
-    return static_cast<int>(launch_kernel_cluster(gemm_w4a16_tc_stream_kernel<MODE>, dim3(tiles, (a.M + a.T - 1) / a.T, a.ksplit), dim3(kStThreads), smem,
-                                                  stream, pdl_enabled(), dim3(1, 1, static_cast<unsigned>(a.ksplit)), a));
+    return static_cast<int>(launch_kernel_cluster(gemm_w4a16_tc_stream_kernel<MODE>, dim3(tiles, (a.M + plan.T - 1) / plan.T, plan.ksplit), dim3(kStThreads),
+                                                  plan.smem, stream, pdl_enabled(), dim3(1, 1, static_cast<unsigned>(plan.ksplit)), a));
 }
 // The streaming form; *taken says whether it applies (up to 256 tokens, K range within a CTA's staging).
 int gemm_tc_stream_launch(const GemmArgs& g, int sm_count, cudaStream_t stream, bool* taken) {

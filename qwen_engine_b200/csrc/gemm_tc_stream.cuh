@@ -35,6 +35,18 @@ constexpr int kStMaxRaw = 24, kStMaxSlots = 6;   // ring slots at most
 constexpr int kStACols = kGroup / 2;             // 128 k of fp16 = 64 columns
 constexpr int kStMaxSplit = 8;                   // portable cluster size
 
+// How a launch is cut.
+struct StreamPlan {
+    int T;                // tokens of a CTA's tile
+    int ksplit;           // cluster size along grid z
+    int tpr;              // tokens a CTA of the cluster finishes (multiple of 4)
+    int raw_slots;        // multiple of 4: a slot always belongs to the same group of dequantising warps (parity waits)
+    int slots;            // A / token slots, at least 4 (the MMAs complete in order, so a group is never two uses ahead)
+    int x_mem;            // token slots that have memory: `slots`, or the steps of a short K range
+    int part_offset;      // K split: byte offset of the partials in shared memory; 0 = on top of the rings
+    int acc2_col, a_col;  // second accumulator; first column of the A slots
+    size_t smem = 0;      // 0: does not fit
+};
 struct StreamArgs {
     CUtensorMap tmap_w[3];
     CUtensorMap tmap_x;
@@ -44,14 +56,8 @@ struct StreamArgs {
     int out_ld[3];
     int tiles[3];
     const __half* residual;
-    int M, K, T;
-    int ksplit;           // cluster size along grid z
-    int tpr;              // tokens a CTA of the cluster finishes (multiple of 4)
-    int raw_slots;        // multiple of 4: a slot always belongs to the same group of dequantising warps (parity waits)
-    int slots;            // A / token slots, at least 4 (the MMAs complete in order, so a group is never two uses ahead)
-    int x_mem;            // token slots that have memory: `slots`, or the steps of a short K range
-    int part_offset;      // K split: byte offset of the partials in shared memory; 0 = on top of the rings
-    int acc2_col, a_col;  // second accumulator; first column of the A slots
+    int M, K;
+    StreamPlan p;
     __half* peer_out[7];  // PLAIN: the output block's place in other GPUs' matrices
     int num_peers;
 };
@@ -89,19 +95,6 @@ __device__ __forceinline__ bool wait_regardless(uint32_t bar, uint32_t parity, u
     for (unsigned it = 0; it < limit; ++it)
         if (mbar_try_wait(bar, parity)) return true;
     return false;
-}
-
-// (q - 8) * s of one packed word with one rounding, as dequant_word_fp16, in 11 instructions instead of 15: a nibble at bits
-// 4..7 of a half is the subnormal q * 2^-20, so fma(q * 2^-20, s * 2^20, -8 s) is the whole conversion; both constants are
-// exact while s * 2^20 is finite (s < 0.0624; larger scales take dequant_word_fp16).
-__device__ __forceinline__ void dequant_word_small_scale(uint32_t packed, __half2 s20, __half2 m8s, uint32_t* out) {
-    const uint32_t lo = (packed << 4) & 0xF0F0F0F0u, hi = packed & 0xF0F0F0F0u;
-    const uint32_t h[4] = {__byte_perm(lo, 0, 0x4140), __byte_perm(lo, 0, 0x4342), __byte_perm(hi, 0, 0x4140), __byte_perm(hi, 0, 0x4342)};
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        const __half2 v = __hfma2(*reinterpret_cast<const __half2*>(&h[i]), s20, m8s);
-        out[i] = *reinterpret_cast<const uint32_t*>(&v);
-    }
 }
 
 // 8 token columns of this thread's weight row, both accumulators added.
@@ -173,10 +166,10 @@ template <int MODE>
 __global__ void __launch_bounds__(kStThreads, 1) gemm_w4a16_tc_stream_kernel(const __grid_constant__ StreamArgs a) {
     extern __shared__ uint8_t smem_raw_base[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw_base) + 1023) & ~uintptr_t(1023));
-    const int T = a.T, NS = a.slots, SR = a.raw_slots, K = a.K;
+    const int T = a.p.T, NS = a.p.slots, SR = a.p.raw_slots, K = a.K;
     const int x_box = T * 128, x_bytes = 2 * x_box;      // a step's tokens: two boxes of 64 k
     uint8_t* s_x = smem;
-    uint8_t* s_raw = s_x + a.x_mem * x_bytes;
+    uint8_t* s_raw = s_x + a.p.x_mem * x_bytes;
     uint64_t* s_bar = reinterpret_cast<uint64_t*>(s_raw + SR * kStRawBytes);
     const uint32_t bar0 = smem_u32(s_bar);
     auto raw_full = [&](int i) { return bar0 + 8u * i; };
@@ -198,7 +191,7 @@ __global__ void __launch_bounds__(kStThreads, 1) gemm_w4a16_tc_stream_kernel(con
     }
     const int n0 = tile * kTileRows, rows_t = a.rows[t], m0 = blockIdx.y * T;
     // K range: whole steps, spread over the cluster as evenly as they go
-    const int ksplit = a.ksplit, krank = static_cast<int>(blockIdx.z);
+    const int ksplit = a.p.ksplit, krank = static_cast<int>(blockIdx.z);
     const int G = K / kGroup, per = G / ksplit, rest = G - per * ksplit;
     const int st0 = krank * per + min(krank, rest), nst = per + (krank < rest ? 1 : 0);
 
@@ -227,7 +220,7 @@ __global__ void __launch_bounds__(kStThreads, 1) gemm_w4a16_tc_stream_kernel(con
         if (lane == 31) {
             mbar_init(accum_full, 1);
             mbar_init(part_full, 1);
-            const int mine = max(0, min(a.tpr, T - krank * a.tpr));
+            const int mine = max(0, min(a.p.tpr, T - krank * a.p.tpr));
             if (ksplit > 1) mbar_arrive_expect_tx(part_full, static_cast<uint32_t>(ksplit * mine * kTileRows * 4));
         }
         fence_barrier_init();
@@ -253,7 +246,7 @@ __global__ void __launch_bounds__(kStThreads, 1) gemm_w4a16_tc_stream_kernel(con
     if (warp == kStDqWarps + 1) asm volatile("bar.arrive 2, %0;" ::"n"(kStThreads) : "memory");
     else asm volatile("bar.sync 2, %0;" ::"n"(kStThreads) : "memory");
     tc_fence_after();
-    const bool own_part = a.part_offset != 0;      // partials in memory of their own: they may come while the rings are in use
+    const bool own_part = a.p.part_offset != 0;      // partials in memory of their own: they may come while the rings are in use
     if (ksplit > 1 && own_part) cluster_arrive();
 
     if (warp < kStDqWarps) {
@@ -282,7 +275,7 @@ __global__ void __launch_bounds__(kStThreads, 1) gemm_w4a16_tc_stream_kernel(con
             ok = group_wait(empty(slot), eph, s_abort, lane);
             if (!ok) break;
             tc_fence_after();
-            const uint32_t a_lane = lane_base + static_cast<uint32_t>(a.a_col + slot * kStACols);
+            const uint32_t a_lane = lane_base + static_cast<uint32_t>(a.p.a_col + slot * kStACols);
             const __half2 sc2 = __half2half2(sc1);
             if (__all_sync(0xFFFFFFFFu, __habs(sc1) < __float2half_rn(0.0624f))) {
                 const __half2 k10 = __float2half2_rn(1024.0f);
@@ -339,7 +332,7 @@ __global__ void __launch_bounds__(kStThreads, 1) gemm_w4a16_tc_stream_kernel(con
 #pragma unroll 1
                 for (int c0 = part * 8; c0 < T; c0 += 32) {
                     float acc[8];
-                    stream_load_acc(lane_base + static_cast<uint32_t>(c0), a.acc2_col, acc);
+                    stream_load_acc(lane_base + static_cast<uint32_t>(c0), a.p.acc2_col, acc);
                     stream_store<MODE>(a, t, n, row_ok, m0 + c0, acc, res);
                     if (c0 + 32 < T) stream_load_residual<MODE>(a, t, n, row_ok, m0 + c0 + 32, res);
                 }
@@ -347,8 +340,8 @@ __global__ void __launch_bounds__(kStThreads, 1) gemm_w4a16_tc_stream_kernel(con
         } else {
             // Tokens [rank * tpr, (rank + 1) * tpr) are finished by that rank; partials land at [source][token / 4][row][4].
             // They are sent whatever the waits returned: a peer that waits for them must not be left alone.
-            const int tpr = a.tpr;
-            uint8_t* s_part = smem + a.part_offset;
+            const int tpr = a.p.tpr;
+            uint8_t* s_part = smem + a.p.part_offset;
             __half res[4];
             stream_load_residual<MODE>(a, t, n, row_ok && part * 4 < tpr, m0 + krank * tpr + part * 4, res);
             if (ok) ok = warp_wait(accum_full, 0, s_abort, lane);
@@ -359,7 +352,7 @@ __global__ void __launch_bounds__(kStThreads, 1) gemm_w4a16_tc_stream_kernel(con
 #pragma unroll 1
             for (int c0 = part * 8; c0 < T; c0 += 32) {
                 float v[8];
-                stream_load_acc(lane_base + static_cast<uint32_t>(c0), a.acc2_col, v);
+                stream_load_acc(lane_base + static_cast<uint32_t>(c0), a.p.acc2_col, v);
 #pragma unroll
                 for (int q = 0; q < 8; q += 4) {
                     const int owner = (c0 + q) / tpr, k = c0 + q - owner * tpr;
@@ -401,13 +394,13 @@ __global__ void __launch_bounds__(kStThreads, 1) gemm_w4a16_tc_stream_kernel(con
                 int slot = 0;
                 uint32_t ph = 0;
                 uint64_t b_desc = b_desc0;
-                uint32_t a_tmem = tmem_base + static_cast<uint32_t>(a.a_col);
+                uint32_t a_tmem = tmem_base + static_cast<uint32_t>(a.p.a_col);
                 bool ready = mbar_test_wait(full(0), 0);
                 for (int s = 0; s < nst; ++s) {
                     if (!ready && !mbar_wait(full(slot), ph, s_abort)) break;
                     tc_fence_after();
                     const uint32_t bar_empty = empty(slot);
-                    const uint32_t tmem_d = tmem_base + ((s & 1) != 0 ? static_cast<uint32_t>(a.acc2_col) : 0u);
+                    const uint32_t tmem_d = tmem_base + ((s & 1) != 0 ? static_cast<uint32_t>(a.p.acc2_col) : 0u);
 #pragma unroll
                     for (int ks = 0; ks < kGroup / 16; ++ks)
                         tc_mma_f16_ts(tmem_d, a_tmem + 8u * ks, b_desc + (ks >= 4 ? b_half : 0u) + static_cast<uint32_t>(2 * (ks & 3)), idesc,
@@ -415,7 +408,7 @@ __global__ void __launch_bounds__(kStThreads, 1) gemm_w4a16_tc_stream_kernel(con
                     tc_commit(bar_empty);
                     a_tmem += kStACols;
                     b_desc += b_step;
-                    if (++slot == NS) { slot = 0; ph ^= 1; b_desc = b_desc0; a_tmem = tmem_base + static_cast<uint32_t>(a.a_col); }
+                    if (++slot == NS) { slot = 0; ph ^= 1; b_desc = b_desc0; a_tmem = tmem_base + static_cast<uint32_t>(a.p.a_col); }
                     ready = mbar_test_wait(full(slot), ph);
                 }
                 tc_commit(accum_full);   // also after a wait that ran out: nothing may be in flight at the end
@@ -470,9 +463,10 @@ __global__ void __launch_bounds__(kStThreads, 1) gemm_w4a16_tc_stream_kernel(con
 }
 
 // ---- host side of the streaming form ----
-// How a launch is cut: token tiles of T, K split `ksplit` ways, ring sizes.  False where it does not fit.
-bool plan_stream(int steps, StreamArgs* a, size_t* smem) {
-    const int T = a->T;
+// Ring sizes for token tiles of T and K split `ksplit` ways, `steps` steps each at most.  False where it does not fit.
+bool plan_stream(int T, int ksplit, int steps, StreamPlan* a) {
+    a->T = T;
+    a->ksplit = ksplit;
     a->slots = T <= 64 ? 6 : 4;
     a->acc2_col = T <= 64 ? 64 : 128;
     a->a_col = 2 * a->acc2_col;
@@ -495,7 +489,7 @@ bool plan_stream(int steps, StreamArgs* a, size_t* smem) {
             a->part_offset = own ? static_cast<int>(used) : 0;
             // At least half an SM, so that no SM gets two CTAs of a launch: smaller ones pile up on the SMs that the previous
             // launch leaves idle (measured on one layer at 47 tokens: 33 instead of 29 us).
-            *smem = std::max<size_t>(1024 + used + (own ? part_bytes : 0), 116 * 1024);
+            a->smem = std::max<size_t>(1024 + used + (own ? part_bytes : 0), 116 * 1024);
             return true;
         }
     }

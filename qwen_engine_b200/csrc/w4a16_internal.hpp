@@ -3,6 +3,8 @@
 
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
+#include <mutex>
+#include <unordered_map>
 #include <utility>
 
 #include <cstdint>
@@ -52,6 +54,34 @@ template <typename... KArgs, typename... Args>
 inline cudaError_t launch_kernel(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
                                  bool pdl, Args&&... args) {
     return launch_kernel_cluster(kernel, grid, block, smem, stream, pdl, dim3(1, 1, 1), std::forward<Args>(args)...);
+}
+
+// Clusters of `cluster` CTAs of a kernel that can be resident at once on the current device (0 where the runtime cannot say).
+int max_active_clusters(const void* kernel, int block, size_t smem, int cluster);
+
+// How a launch of a shape is cut, worked out once per shape (bounded: a host that goes through many shapes starts over).
+template <typename V>
+class PlanCache {
+public:
+    template <typename F>
+    V get(uint64_t key, F&& make) {
+        std::lock_guard<std::mutex> lock(mu_);
+        auto it = map_.find(key);
+        if (it != map_.end()) return it->second;
+        if (map_.size() >= 4096) map_.clear();
+        return map_.emplace(key, make()).first->second;
+    }
+
+private:
+    std::mutex mu_;
+    std::unordered_map<uint64_t, V> map_;
+};
+// device | mode | tokens | K / 128 | rows
+inline uint64_t plan_key(int mode, int tokens, int K, int rows) {
+    int dev = 0;
+    cudaGetDevice(&dev);
+    return (static_cast<uint64_t>(dev) << 58) | (static_cast<uint64_t>(mode & 3) << 56) | (static_cast<uint64_t>(tokens & 0xFFF) << 44) |
+           (static_cast<uint64_t>((K / 128) & 0xFFFF) << 28) | static_cast<uint64_t>(rows & 0xFFFFFFF);
 }
 
 // ---- Q8_1 quantisers (q8_1_quantize.cu) ----
@@ -191,6 +221,7 @@ bool gemm_tc_supported(const GemmArgs& g);
 int gemm_tc_launch(const GemmArgs& g, int sm_count, cudaStream_t stream);
 int gemm_tc_set_attributes();
 int gemm_tc_timeouts(unsigned int* out);
+int gemm_mma_timeouts(unsigned int* out);    // the exchange of the few-token form
 
 // ---- persistent one-kernel decode sweep (sweep_persistent.cu) ----
 struct PSweepArgs {

@@ -1,0 +1,531 @@
+// Prefill W4A16 contraction on CTA pairs (tcgen05.mma.cta_group::2).  Included by gemm_tc.cu behind the PTX wrappers.
+//
+// Two CTAs of a cluster -- two SMs -- share a tile of 256 weight rows x T tokens: each dequantises ITS 128 weight rows
+// (the A operand, M = 256 split over the pair) into its tensor memory and loads ITS T / 2 tokens (half of the B operand)
+// into its shared memory; one thread of the leading CTA issues the MMAs, which accumulate into both CTAs' tensor memory.
+// A does not pass through shared memory: with it there the operand reads alone exceed what shared memory delivers beside
+// the loads (measured on a one-CTA form: 0.57 of the bf16 peak).  Steps are 128 k, one quantisation group.
+//
+// What bounds it: the tensor pipe on long K (28672 x 8192), the work around a tile on short K (K = 1536 gives 12 steps per
+// tile).  So the epilogue has warps of its own, and tensor memory holds two accumulators of up to 128 token columns: a tile
+// of up to 128 tokens uses one of them in turn with the next tile's, a larger one both as its two halves.  The epilogue
+// takes a half into registers and gives it back at once, and the MMAs of the next tile's first half run ahead meanwhile.
+// The rest of tensor memory are four A slots of one step.  Arrivals on the leader's barriers carry no cluster-scope release:
+// with one the peer's dequantising warps waited for their own prefetched loads at every step (1400 cycles a step, 930 of
+// them for nothing).
+//
+//   warps 0..7  : dequantise; group g = warp / 4 takes the steps g, g + 2, ...  A step is in registers as fp16 before its
+//                 slot is free, so a slot is refilled one store after the MMA that read it.
+//   warps 8..23 : epilogue, 128 rows of a finished accumulator (four warps per 32 rows, a quarter of the tokens each)
+//   warp 24     : tensor memory; in the leading CTA one thread issues the MMAs
+//   warp 25     : TMA of the packed weights, 128 rows x 128 k per slot (private ring, before the wait for the previous kernel)
+//   warp 26     : TMA of this CTA's half of the token tile, T / 2 x 128 k per slot
+//   warp 27     : none (whole warpgroups, for the register split)
+//
+// Synchronisation: one "full" barrier per slot in the leader counts the dequantising warps of both CTAs and the bytes
+// of both token halves; one "done" barrier per slot in both CTAs (tcgen05.commit with a CTA mask) frees the A slot and
+// the token slot.  Two "accumulator full" barriers in both CTAs, two "accumulator empty" ones in the leader.
+constexpr int kPairGroups = 2;
+constexpr int kPairDqWarps = 4 * kPairGroups, kPairEpiWarps = 16;
+constexpr int kPairThreads = (kPairDqWarps + kPairEpiWarps + 4) * 32;
+constexpr int kPairAccCols = 128;            // one accumulator
+constexpr int kPairACol = 2 * kPairAccCols, kPairACols = kGroup / 2;   // A slots behind the two accumulators
+constexpr int kPairSlots = 4;                // A and token slots; a multiple of the groups (parity waits)
+constexpr int kPairRawSlots = 8;             // packed weights; likewise
+constexpr int kPairRawBytes = kTileRows * 64;
+// Registers a thread: 72 at launch (28 warps), then by role; the sum over the warps stays what was launched with.
+constexpr int kPairRegsLaunch = 72, kPairRegsDq = 88, kPairRegsEpi = 64, kPairRegsRest = 72;
+static_assert(kPairDqWarps * kPairRegsDq + kPairEpiWarps * kPairRegsEpi + 4 * kPairRegsRest <= (kPairThreads / 32) * kPairRegsLaunch, "register split");
+
+struct PairArgs {
+    CUtensorMap tmap_w[3];
+    CUtensorMap tmap_x;
+    const __half* scales[3];
+    __half* out[3];
+    int rows[3];
+    int out_ld[3];
+    int tiles[3];
+    const __half* residual;
+    int M, K;
+    int halves, n_half;      // accumulators of a tile and tokens of each: T = halves * n_half
+    int vec_ok;              // outputs (and residual) can be written two rows at a time: even strides, 4-byte aligned
+    int panel;               // token tiles per panel of the tile order
+    __half* peer_out[7];     // PLAIN: the output block's place in other GPUs' matrices
+    int num_peers;
+};
+
+__device__ __forceinline__ uint32_t cluster_cta_rank() {
+    uint32_t r;
+    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+    return r;
+}
+// Arrival on a barrier of the other CTA.  What it announces lies in tensor memory, ordered by the tcgen05 fences and waits
+// on both sides.
+__device__ __forceinline__ void mbar_arrive_remote(uint32_t cluster_addr) {
+    asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
+}
+__device__ __forceinline__ void tma_load_2d_pair(uint32_t dst, const CUtensorMap* map, int x, int y, uint32_t leader_bar) {
+    asm volatile(
+        "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
+        ::"r"(dst), "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(leader_bar)
+        : "memory");
+}
+__device__ __forceinline__ void tmem_alloc_pair(uint32_t dst_smem, uint32_t cols) {
+    asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(dst_smem), "r"(cols) : "memory");
+}
+__device__ __forceinline__ void tmem_relinquish_pair() {
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void tmem_dealloc_pair(uint32_t taddr, uint32_t cols) {
+    asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(cols) : "memory");
+}
+// arrives on the barrier at this shared-memory offset in both CTAs of the pair once the MMAs issued so far are done
+__device__ __forceinline__ void tc_commit_pair(uint32_t bar) {
+    asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;"
+                 ::"r"(bar), "h"(static_cast<uint16_t>(3)) : "memory");
+}
+// Instruction descriptor of the pair: D fp32, A/B fp16, both K-major, M = 256 (128 rows per CTA), N = n.
+__device__ __forceinline__ uint32_t make_idesc_pair(int n) {
+    return (1u << 4) | (static_cast<uint32_t>(n >> 3) << 17) | (static_cast<uint32_t>(256 >> 4) << 24);
+}
+// D[tmem] (+)= A[tmem] * B[smem]^T over the CTA pair.
+__device__ __forceinline__ void tc_mma_f16_pair_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t desc_b, uint32_t idesc,
+                                                   uint32_t accumulate) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::2.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
+        ::"r"(tmem_d), "r"(tmem_a), "l"(desc_b), "r"(idesc), "r"(accumulate)
+        : "memory");
+}
+
+// Which 128-row tile of which tensor, and which tokens, a pair tile index stands for (this CTA's half).
+struct PairTile {
+    int t, n0, m0;
+};
+__device__ __forceinline__ PairTile pair_tile(const PairArgs& a, int pt, int n_pairs, int rank, bool qkv) {
+    PairTile r;
+    // Tile order: panels of a.panel token tiles; inside a panel the token tile runs fastest.  With a panel of 4 the
+    // tiles in flight at one time (one per CTA pair) cover 4 token tiles x about 18 row-tile pairs, and both the
+    // token slabs and the packed weight rows are re-used out of L2; a panel of 1 (row tiles fastest) shares one
+    // token slab among all tiles in flight but streams the whole weight matrix once per token tile, which is
+    // right only while the matrix stays in L2 (the host picks).
+    const int T = a.halves * a.n_half;
+    const int m_tiles = (a.M + T - 1) / T;
+    const int per_panel = a.panel * n_pairs;
+    const int panel = pt / per_panel;
+    const int q = pt - panel * per_panel;
+    const int w = min(a.panel, m_tiles - panel * a.panel);
+    const int m_idx = panel * a.panel + q % w;
+    int tile = 2 * (q / w) + rank;      // consecutive 128-row tiles form a pair; an odd last one is paired with rows past the end
+    r.t = 0;
+    if (qkv) {
+        if (tile >= a.tiles[0]) { tile -= a.tiles[0]; r.t = 1; }
+        if (r.t == 1 && tile >= a.tiles[1]) { tile -= a.tiles[1]; r.t = 2; }
+    }
+    r.n0 = tile * kTileRows;
+    r.m0 = m_idx * T;
+    return r;
+}
+
+// Eight tokens m0 .. m0 + 7 of weight row n.  All lanes of a warp call it with consecutive rows and the same tokens.  The
+// even lane of a pair finishes the first token of two, the odd lane the second: SWIGLU has its gate in the even and its
+// up in the odd row, the others store both rows of a token as one word.
+template <int MODE>
+__device__ __forceinline__ void pair_store8(const PairArgs& a, int t, int n, int m0, const float (&acc)[8]) {
+    const int odd = n & 1, ne = n & ~1, rows = a.rows[t];
+    const size_t ld = static_cast<size_t>(a.out_ld[t]);
+#pragma unroll
+    for (int q = 0; q < 8; q += 2) {
+        const float other = __shfl_xor_sync(0xFFFFFFFFu, odd ? acc[q] : acc[q + 1], 1);
+        const float even_row = odd ? other : acc[q], odd_row = odd ? acc[q + 1] : other;
+        const int m = m0 + q + odd;
+        if (m >= a.M || ne >= rows) continue;
+        if constexpr (MODE == kSwiglu) {
+            a.out[t][static_cast<size_t>(m) * ld + (n >> 1)] = __float2half_rn(swiglu_f32(even_row, odd_row));
+        } else {
+            const size_t off = static_cast<size_t>(m) * ld + ne;
+            __half y[2] = {__float2half_rn(even_row), __float2half_rn(odd_row)};
+            for (int i = 0; i < (ne + 1 < rows ? 2 : 1); ++i) {
+                if constexpr (MODE == kPlain) {
+                    if (a.residual != nullptr) y[i] = __hadd(y[i], a.residual[off + i]);
+                }
+                a.out[t][off + i] = y[i];
+            }
+            if constexpr (MODE == kPlain) {
+                for (int p = 0; p < a.num_peers; ++p) {
+                    if (a.vec_ok && ne + 1 < rows) {
+                        *reinterpret_cast<__half2*>(a.peer_out[p] + off) = __halves2half2(y[0], y[1]);
+                    } else {
+                        a.peer_out[p][off] = y[0];
+                        if (ne + 1 < rows) a.peer_out[p][off + 1] = y[1];
+                    }
+                }
+            }
+        }
+    }
+}
+// The same for a tile that lies inside the output, addresses given: this lane's first token and output, `step` bytes from
+// one of its tokens to the next.
+template <int MODE>
+__device__ __forceinline__ void pair_store8_inside(char* out, size_t step, int odd, const float (&acc)[8], const __half2 (&res)[4], bool add) {
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+        const float other = __shfl_xor_sync(0xFFFFFFFFu, odd ? acc[2 * q] : acc[2 * q + 1], 1);
+        const float even_row = odd ? other : acc[2 * q], odd_row = odd ? acc[2 * q + 1] : other;
+        if constexpr (MODE == kSwiglu) {
+            *reinterpret_cast<__half*>(out) = __float2half_rn(swiglu_f32(even_row, odd_row));
+        } else {
+            __half2 y = __floats2half2_rn(even_row, odd_row);
+            if (MODE == kPlain && add) y = __hadd2(y, res[q]);
+            *reinterpret_cast<__half2*>(out) = y;
+        }
+        out += step;
+    }
+}
+
+template <int MODE>
+__global__ void __launch_bounds__(kPairThreads, 1) gemm_w4a16_tc_pair_kernel(const __grid_constant__ PairArgs a) {
+    constexpr int kEpi0 = kPairDqWarps, kMmaWarp = kEpi0 + kPairEpiWarps, kRawWarp = kMmaWarp + 1;
+    extern __shared__ uint8_t smem_raw_base[];
+    uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw_base) + 1023) & ~uintptr_t(1023));
+    const int H = a.halves, NH = a.n_half, T = H * NH, K = a.K, G = K / kGroup;
+    const int b_box = (NH / 2) * 128, b_bytes = 2 * H * b_box;      // [accumulator][64 k]: half of each accumulator's tokens
+    uint8_t* s_b = smem;
+    uint8_t* s_raw = s_b + kPairSlots * b_bytes;
+    uint64_t* s_bar = reinterpret_cast<uint64_t*>(s_raw + kPairRawSlots * kPairRawBytes);
+    const uint32_t bar0 = smem_u32(s_bar);
+    auto raw_full = [&](int i) { return bar0 + 8u * i; };
+    auto raw_empty = [&](int i) { return bar0 + 8u * (kPairRawSlots + i); };
+    auto full = [&](int i) { return bar0 + 8u * (2 * kPairRawSlots + i); };
+    auto done = [&](int i) { return bar0 + 8u * (2 * kPairRawSlots + kPairSlots + i); };
+    auto acc_full = [&](int i) { return bar0 + 8u * (2 * kPairRawSlots + 2 * kPairSlots + i); };
+    auto acc_empty = [&](int i) { return bar0 + 8u * (2 * kPairRawSlots + 2 * kPairSlots + 2 + i); };
+    constexpr int kBars = 2 * kPairRawSlots + 2 * kPairSlots + 4;
+    uint32_t* s_tmem = reinterpret_cast<uint32_t*>(s_bar + kBars);
+    volatile int* s_abort = reinterpret_cast<volatile int*>(s_tmem + 1);
+
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int rank = static_cast<int>(cluster_cta_rank());
+    const bool leader = rank == 0;
+    const int pair_id = blockIdx.x >> 1, num_pairs = gridDim.x >> 1;
+    const int n_pairs = (a.tiles[0] + a.tiles[1] + a.tiles[2] + 1) / 2;
+    const int total_pt = n_pairs * ((a.M + T - 1) / T);
+
+    if (warp == kRawWarp) {
+        if (lane < kPairRawSlots) { mbar_init(raw_full(lane), 1); mbar_init(raw_empty(lane), 4); }
+        // full: four dequantising warps of each CTA and the leader's expect_tx arrival
+        if (lane < kPairSlots) { mbar_init(full(lane), 2 * 4 + 1); mbar_init(done(lane), 1); }
+        if (lane < 2) { mbar_init(acc_full(lane), 1); mbar_init(acc_empty(lane), 2 * kPairEpiWarps); }
+        if (lane == 0) { *s_abort = 0; tma_prefetch_desc(&a.tmap_x); tma_prefetch_desc(&a.tmap_w[0]); }
+        fence_barrier_init();
+        fence_proxy_async_smem();
+        __syncwarp();
+    }
+    if (warp == kMmaWarp) {          // the same warp in both CTAs, the same shared-memory offset for the result
+        tmem_alloc_pair(smem_u32(s_tmem), 512);
+        tmem_relinquish_pair();
+        pdl_release_dependents();    // not before: a CTA of the next launch must not take this one's tensor memory
+    }
+    tc_fence_before();
+    __syncthreads();
+    cluster_sync_all();              // the peer's barriers exist before anything arrives on them from here
+    tc_fence_after();
+    const uint32_t tmem_base = *s_tmem;
+    if (warp < kPairDqWarps) asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kPairRegsDq));
+    else if (warp < kMmaWarp) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kPairRegsEpi));
+    else asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kPairRegsRest));
+
+    if (warp < kPairDqWarps) {
+        // ================= dequantise: thread = weight row = tensor-memory lane =================
+        const int r = (warp & 3) * 32 + lane, g = warp >> 2;
+        const int swz = (r >> 1) & 3;            // 64-byte swizzle: 16-byte chunk index xor row pair
+        const uint32_t a_lane = tmem_base + (static_cast<uint32_t>((warp & 3) * 32) << 16) + static_cast<uint32_t>(kPairACol);
+        const uint32_t leader_full0 = cluster_map_shared(full(0), 0);
+        bool ok = true;
+        // The walk over (tile, step) pairs is one sequence: a group's next step after a tile's last one lies in the next tile.
+        const int my_tiles = pair_id < total_pt ? (total_pt - pair_id + num_pairs - 1) / num_pairs : 0;
+        const int total = my_tiles * G;
+        int rs = g, slot = g;                    // ring positions of this group's next step
+        uint32_t rph = 0, dph = 1;               // parities: raw slot filled; slot freed by its previous use
+        int it = 0, st = g;                      // tile iteration and step in it
+        PairTile pt = my_tiles > 0 ? pair_tile(a, pair_id, n_pairs, rank, MODE == kQkv) : PairTile{0, 0, 0};
+        auto settle = [&]() {                    // (it, st) back into range after st moved on
+            while (st >= G) {
+                st -= G;
+                if (++it < my_tiles) pt = pair_tile(a, pair_id + it * num_pairs, n_pairs, rank, MODE == kQkv);
+            }
+        };
+        auto load_scale = [&]() -> __half {
+            const int row = pt.n0 + r;
+            return row < a.rows[pt.t] ? __ldg(a.scales[pt.t] + static_cast<size_t>(row) * G + st) : __half(0.0f);
+        };
+        settle();
+        __half sc_next = g < total ? load_scale() : __half(0.0f);
+        for (int i = g; i < total; i += kPairGroups) {
+            const __half sc = sc_next;
+            st += kPairGroups;
+            settle();
+            if (i + kPairGroups < total) sc_next = load_scale();     // the next step's, one visit ahead
+            ok = group_wait(raw_full(rs), rph, s_abort, lane);
+            if (!ok) break;
+            const uint8_t* raw_row = s_raw + rs * kPairRawBytes + r * 64;
+            const __half2 sc2 = __half2half2(sc);
+            uint32_t cols[2][32];
+            if (__all_sync(0xFFFFFFFFu, __habs(sc) < __float2half_rn(0.0624f))) {
+                const __half2 k10 = __float2half2_rn(1024.0f);
+                const __half2 s20 = __hmul2(__hmul2(sc2, k10), k10), m8s = __hmul2(sc2, __float2half2_rn(-8.0f));
+#pragma unroll
+                for (int c = 0; c < 4; ++c) {
+                    const uint4 w = *reinterpret_cast<const uint4*>(raw_row + ((c ^ swz) << 4));
+                    uint32_t* o = &cols[c >> 1][16 * (c & 1)];
+                    dequant_word_small_scale(w.x, s20, m8s, o);
+                    dequant_word_small_scale(w.y, s20, m8s, o + 4);
+                    dequant_word_small_scale(w.z, s20, m8s, o + 8);
+                    dequant_word_small_scale(w.w, s20, m8s, o + 12);
+                }
+            } else {
+#pragma unroll
+                for (int c = 0; c < 4; ++c) {
+                    const uint4 w = *reinterpret_cast<const uint4*>(raw_row + ((c ^ swz) << 4));
+                    const uint32_t words[4] = {w.x, w.y, w.z, w.w};
+#pragma unroll
+                    for (int k = 0; k < 4; ++k) {
+                        __half2 h[4];
+                        dequant_word_fp16(words[k], sc2, h);
+#pragma unroll
+                        for (int q = 0; q < 4; ++q) cols[c >> 1][16 * (c & 1) + 4 * k + q] = *reinterpret_cast<const uint32_t*>(&h[q]);
+                    }
+                }
+            }
+            __syncwarp();
+            if (lane == 0) mbar_arrive(raw_empty(rs));
+            ok = group_wait(done(slot), dph, s_abort, lane);
+            if (!ok) break;
+            tc_fence_after();
+            tmem_st32(a_lane + static_cast<uint32_t>(slot * kPairACols), cols[0]);
+            tmem_st32(a_lane + static_cast<uint32_t>(slot * kPairACols + 32), cols[1]);
+            tmem_st_wait();
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) {
+                if (leader) mbar_arrive(full(slot));
+                else mbar_arrive_remote(leader_full0 + 8u * slot);
+            }
+            rs += kPairGroups;
+            if (rs >= kPairRawSlots) { rs -= kPairRawSlots; rph ^= 1; }
+            slot += kPairGroups;
+            if (slot >= kPairSlots) { slot -= kPairSlots; dph ^= 1; }
+        }
+    } else if (warp < kMmaWarp) {
+        // ================= epilogue: thread = weight row, registers = tokens =================
+        const int part = (warp - kEpi0) >> 2, r = (warp & 3) * 32 + lane, odd = lane & 1;
+        const uint32_t lane_base = tmem_base + (static_cast<uint32_t>((warp & 3) * 32) << 16) + static_cast<uint32_t>(8 * part);
+        const uint32_t leader_empty0 = cluster_map_shared(acc_empty(0), 0);
+        constexpr int kMaxGroups = kPairAccCols / 32;          // this warp's groups of eight tokens: part, part + 4, ...
+        const int n_groups = (NH / 8 - part + 3) / 4;
+        const bool add = MODE == kPlain && a.residual != nullptr;
+        bool ok = true;
+        int buf = 0;
+        uint32_t ph = 0;
+        pdl_wait_prior_grids();                  // the previous kernels' reads of the outputs and writes of the residual
+        for (int pt_i = pair_id; pt_i < total_pt && ok; pt_i += num_pairs) {
+            const PairTile pt = pair_tile(a, pt_i, n_pairs, rank, MODE == kQkv);
+            for (int h = 0; h < H; ++h) {
+                const int m0 = pt.m0 + h * NH + 8 * part;
+                const bool inside = a.vec_ok && pt.n0 + kTileRows <= a.rows[pt.t] && pt.m0 + (h + 1) * NH <= a.M && (MODE != kPlain || a.num_peers == 0);
+                const size_t ld = static_cast<size_t>(a.out_ld[pt.t]);
+                const size_t off = static_cast<size_t>(m0 + odd) * ld + (MODE == kSwiglu ? (pt.n0 + r) >> 1 : (pt.n0 + r) & ~1);
+                // the residual of the first groups while the tensor core is still at it
+                __half2 res[2][4];
+                auto load_res = [&](int i) {
+#pragma unroll
+                    for (int q = 0; q < 4; ++q) res[i & 1][q] = *reinterpret_cast<const __half2*>(a.residual + off + static_cast<size_t>(32 * i + 2 * q) * ld);
+                };
+                if (add && inside) {
+#pragma unroll
+                    for (int i = 0; i < 2; ++i)
+                        if (i < n_groups) load_res(i);
+                }
+                ok = group_wait(acc_full(buf), ph, s_abort, lane);
+                if (!ok) break;
+                tc_fence_after();
+                // this warp's columns into registers, then the accumulator goes back
+                uint32_t v[kMaxGroups][8];
+#pragma unroll
+                for (int i = 0; i < kMaxGroups; ++i)
+                    if (i < n_groups) tmem_ld8(lane_base + static_cast<uint32_t>(buf * kPairAccCols + 32 * i), v[i]);
+                tmem_ld_wait();
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) {
+                    if (leader) mbar_arrive(acc_empty(buf));
+                    else mbar_arrive_remote(leader_empty0 + 8u * buf);
+                }
+                char* out = reinterpret_cast<char*>(a.out[pt.t] + off);
+#pragma unroll
+                for (int i = 0; i < kMaxGroups; ++i) {
+                    if (i < n_groups) {
+                        float acc[8];
+#pragma unroll
+                        for (int q = 0; q < 8; ++q) acc[q] = __uint_as_float(v[i][q]);
+                        if (inside) {
+                            pair_store8_inside<MODE>(out, 4 * ld, odd, acc, res[i & 1], add);
+                            if (add && i + 2 < n_groups) load_res(i + 2);
+                            out += 64 * ld;
+                        } else if (m0 + 32 * i < a.M) {
+                            pair_store8<MODE>(a, pt.t, pt.n0 + r, m0 + 32 * i, acc);
+                        }
+                    }
+                }
+                buf ^= 1;
+                if (buf == 0) ph ^= 1;
+            }
+        }
+    } else if (warp == kMmaWarp) {
+        // ================= MMA issue: one thread of the leading CTA =================
+        if (leader && elect_one()) {
+            const uint32_t idesc = make_idesc_pair(NH);
+            const uint64_t b_desc0 = make_smem_desc(smem_u32(s_b));
+            const uint32_t b_step = static_cast<uint32_t>(b_bytes) >> 4, b_boxd = static_cast<uint32_t>(b_box) >> 4;
+            int slot = 0, buf = 0;
+            uint32_t ph = 0, eph = 1;            // eph: parity that frees an accumulator (fresh barriers pass)
+            bool ok = true;
+            // the eight MMAs of one step into one accumulator
+            auto issue = [&](int sl, int half, int buffer, bool fresh) {
+                const uint32_t a_tmem = tmem_base + static_cast<uint32_t>(kPairACol + sl * kPairACols);
+                const uint64_t b_desc = b_desc0 + static_cast<uint32_t>(sl) * b_step + static_cast<uint32_t>(half) * 2u * b_boxd;
+                const uint32_t tmem_d = tmem_base + static_cast<uint32_t>(buffer * kPairAccCols);
+#pragma unroll
+                for (int ks = 0; ks < kGroup / 16; ++ks)
+                    tc_mma_f16_pair_ts(tmem_d, a_tmem + 8u * ks, b_desc + (ks >= 4 ? b_boxd : 0u) + static_cast<uint32_t>(2 * (ks & 3)), idesc,
+                                       (ks != 0 || !fresh) ? 1u : 0u);
+            };
+            auto advance = [&](int& sl, uint32_t& p) {
+                if (++sl == kPairSlots) { sl = 0; p ^= 1; }
+            };
+            bool ready = mbar_test_wait(full(0), 0);
+            for (int pt_i = pair_id; pt_i < total_pt && ok; pt_i += num_pairs) {
+                if (!mbar_wait(acc_empty(buf), eph, s_abort)) break;
+                tc_fence_after();
+                int st = 0;
+                bool first_half_committed = false;
+                if (H == 2) {
+                    // the first half runs ahead while the epilogue still has the second
+                    int ahead = 0, sl = slot;
+                    uint32_t p = ph;
+                    const int most = min(kPairSlots, G);
+                    while (ahead < most && !mbar_test_wait(acc_empty(1), eph)) {
+                        if (!mbar_wait(full(sl), p, s_abort)) { ok = false; break; }
+                        tc_fence_after();
+                        issue(sl, 0, 0, ahead == 0);
+                        advance(sl, p);
+                        ++ahead;
+                    }
+                    if (!ok || !mbar_wait(acc_empty(1), eph, s_abort)) break;
+                    tc_fence_after();
+                    for (; st < ahead; ++st) {
+                        issue(slot, 1, 1, st == 0);
+                        tc_commit_pair(done(slot));
+                        advance(slot, ph);
+                    }
+                    if (ahead > 0) ready = st < G && mbar_test_wait(full(slot), ph);
+                }
+                for (; st < G; ++st) {
+                    if (!ready && !mbar_wait(full(slot), ph, s_abort)) { ok = false; break; }
+                    tc_fence_after();
+                    const int sl = slot;
+                    advance(slot, ph);
+                    ready = mbar_test_wait(full(slot), ph);      // the answer arrives while the MMAs below are issued
+                    issue(sl, 0, H == 2 ? 0 : buf, st == 0);
+                    if (H == 2) {
+                        if (st == G - 1) { tc_commit_pair(acc_full(0)); first_half_committed = true; }
+                        issue(sl, 1, 1, st == 0);
+                    }
+                    tc_commit_pair(done(sl));
+                }
+                if (!ok) break;
+                if (H == 2) {
+                    if (!first_half_committed) tc_commit_pair(acc_full(0));   // (all of a short tile was issued ahead)
+                    tc_commit_pair(acc_full(1));
+                    eph ^= 1;
+                } else {
+                    tc_commit_pair(acc_full(buf));
+                    buf ^= 1;
+                    if (buf == 0) eph ^= 1;
+                }
+            }
+        }
+        __syncwarp();
+    } else if (warp == kRawWarp) {
+        // ================= TMA: raw packed weights of this CTA's 128 rows (private ring) =================
+        if (lane == 0) {
+            int rs = 0;
+            uint32_t rph = 1;
+            bool ok = true;
+            for (int pt_i = pair_id; pt_i < total_pt && ok; pt_i += num_pairs) {
+                const PairTile pt = pair_tile(a, pt_i, n_pairs, rank, MODE == kQkv);
+                for (int s = 0; s < G; ++s) {
+                    if (!mbar_wait(raw_empty(rs), rph, s_abort)) { ok = false; break; }
+                    mbar_arrive_expect_tx(raw_full(rs), kPairRawBytes);
+                    tma_load_2d(smem_u32(s_raw + rs * kPairRawBytes), &a.tmap_w[pt.t], s * 64, pt.n0, raw_full(rs));
+                    if (++rs == kPairRawSlots) { rs = 0; rph ^= 1; }
+                }
+            }
+        }
+        __syncwarp();
+    } else if (warp == kRawWarp + 1) {
+        // ================= TMA: this CTA's half of the token tile; bytes counted on the LEADER's barrier =================
+        if (lane == 0) {
+            int slot = 0;
+            uint32_t dph = 1;
+            bool ok = true;
+            const uint32_t leader_full0 = cluster_map_shared(full(0), 0);
+            pdl_wait_prior_grids();
+            for (int pt_i = pair_id; pt_i < total_pt && ok; pt_i += num_pairs) {
+                const PairTile pt = pair_tile(a, pt_i, n_pairs, rank, MODE == kQkv);
+                for (int s = 0; s < G; ++s) {
+                    if (!mbar_wait(done(slot), dph, s_abort)) { ok = false; break; }
+                    if (leader) mbar_arrive_expect_tx(full(slot), static_cast<uint32_t>(2 * b_bytes));
+                    uint32_t dst = smem_u32(s_b + slot * b_bytes);
+                    for (int h = 0; h < H; ++h)
+                        for (int kk = 0; kk < 2; ++kk, dst += b_box)
+                            tma_load_2d_pair(dst, &a.tmap_x, s * kGroup + kk * kBK, pt.m0 + h * NH + rank * (NH / 2), leader_full0 + 8u * slot);
+                    if (++slot == kPairSlots) { slot = 0; dph ^= 1; }
+                }
+            }
+        }
+        __syncwarp();
+    }
+
+    // Neither CTA may leave (or free its tensor memory) while the other's instructions can still touch its
+    // shared memory, barriers or accumulators.
+    tc_fence_before();
+    __syncthreads();
+    if (*s_abort) __nanosleep(500000);      // a bounded wait ran out: what is in flight lands before the memory goes
+    cluster_sync_all();
+    if (warp == kMmaWarp) tmem_dealloc_pair(tmem_base, 512);
+}
+
+// ---- host side ----
+size_t tc_pair_smem_bytes(int T) {
+    return 1024 + static_cast<size_t>(kPairSlots) * T * 128 + static_cast<size_t>(kPairRawSlots) * kPairRawBytes +
+           (2 * kPairRawSlots + 2 * kPairSlots + 4) * 8 + 16;
+}
+// Estimated cycles of a launch with token tiles of T, from measurements on B200: a step takes 4 T of MMA or 950 of
+// dequantisation, whichever is more; a tile of two accumulators waits 2500 for the second one to be drained; the first fill,
+// the exchange at the start and the last tile's epilogue are not overlapped.
+double pair_cost(int M, int n_pairs, int steps, int pairs, int T) {
+    const int tiles = n_pairs * ((M + T - 1) / T), rounds = (tiles + pairs - 1) / pairs;
+    return rounds * (steps * std::max(4.0 * T, 950.0) + (T > kPairAccCols ? 2500.0 : 0.0)) + 6000.0 + 25.0 * T;
+}
+// The token tile for `n_pairs` pairs of row tiles on `pairs` pairs of SMs: one accumulator of 16..128 or two of 80..128.
+int pair_token_tile(int M, int n_pairs, int steps, int pairs) {
+    int best = 16;
+    double best_cost = 0;
+    for (int T = 16; T <= 2 * kPairAccCols; T += T < kPairAccCols ? 16 : 32) {
+        const double cost = pair_cost(M, n_pairs, steps, pairs, T);
+        if (best_cost == 0 || cost < best_cost) { best = T; best_cost = cost; }
+    }
+    return best;
+}

@@ -80,8 +80,8 @@ private:
 inline uint64_t plan_key(int mode, int tokens, int K, int rows) {
     int dev = 0;
     cudaGetDevice(&dev);
-    return (static_cast<uint64_t>(dev) << 58) | (static_cast<uint64_t>(mode & 3) << 56) | (static_cast<uint64_t>(tokens & 0xFFF) << 44) |
-           (static_cast<uint64_t>((K / 128) & 0xFFFF) << 28) | static_cast<uint64_t>(rows & 0xFFFFFFF);
+    return (static_cast<uint64_t>(dev) << 58) | (static_cast<uint64_t>(mode & 3) << 56) | (static_cast<uint64_t>(tokens & 0xFFFF) << 40) |
+           (static_cast<uint64_t>((K / 128) & 0xFFFF) << 24) | static_cast<uint64_t>(rows & 0xFFFFFF);
 }
 
 // ---- Q8_1 quantisers (q8_1_quantize.cu) ----

@@ -127,6 +127,13 @@ __device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t (&r)[32
           "r"(r[29]), "r"(r[30]), "r"(r[31])
         : "memory");
 }
+__device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&r)[16]) {
+    asm volatile(
+        "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};"
+        ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]),
+          "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
+        : "memory");
+}
 __device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 
 // Shared-memory matrix descriptor: K-major tile, 128-byte swizzle, rows 128 B apart, 8-row groups
@@ -229,9 +236,11 @@ int gemm_tc_set_attributes() {
     raise_pair(gemm_w4a16_tc_stream_kernel<kPlain>);
     raise_pair(gemm_w4a16_tc_stream_kernel<kQkv>);
     raise_pair(gemm_w4a16_tc_stream_kernel<kSwiglu>);
-    raise_pair(gemm_w4a16_tc_pair_kernel<kPlain>);
-    raise_pair(gemm_w4a16_tc_pair_kernel<kQkv>);
-    raise_pair(gemm_w4a16_tc_pair_kernel<kSwiglu>);
+    raise_pair(gemm_w4a16_tc_pair_kernel<kPlain, true>);
+    raise_pair(gemm_w4a16_tc_pair_kernel<kPlain, false>);
+    raise_pair(gemm_w4a16_tc_pair_kernel<kQkv, true>);
+    raise_pair(gemm_w4a16_tc_pair_kernel<kQkv, false>);
+    raise_pair(gemm_w4a16_tc_pair_kernel<kSwiglu, true>);
     return static_cast<int>(e);
 }
 
@@ -247,41 +256,45 @@ bool gemm_tc_supported(const GemmArgs& g) {
 }
 
 namespace {
-constexpr int kStreamDoesNotFit = -1000;     // a K range whose group scales and rings are beyond a CTA's shared memory
+// The streaming kernel's cut of a shape: token tiles and K slices, two steps each at least, within one CTA per SM where that is
+// possible.  The cut is chosen by what a CTA has to do, in cycles: 400 a step of dequantisation or 4 T of MMA, whichever is
+// longer; the exchange of partials at 18 bytes a cycle after its latency; 25 a token for the epilogue.  What a launch takes (the
+// plan's cost) is more than that: 8.6 T a step, the token tile's way from L2 (measured at 128 tokens, 96 CTAs: 0.58 us a
+// step), and 5500 of start and end, for every wave of CTAs.
 template <int MODE>
-int launch_stream(StreamArgs& a, const __half* x, int tiles, int sm_count, cudaStream_t stream) {
-    // Token tiles and K slices, two steps each at least, within one CTA per SM where that is possible.  Estimated cycles of a
-    // CTA, from measurements on B200: 400 a step of dequantisation or 4 T of MMA, whichever is longer; the exchange of
-    // partials at 18 bytes a cycle with its latency; 25 a token for the epilogue.
+StreamPlan stream_plan(int M, int K, int tiles, int sm_count) {
     static PlanCache<StreamPlan> plans;
-    const StreamPlan plan = plans.get(plan_key(MODE, a.M, a.K, tiles), [&] {
-        const int steps = a.K / kGroup;
+    return plans.get(plan_key(MODE, M, K, tiles), [&] {
+        const int steps = K / kGroup;
         StreamPlan best;
-        double best_cost = 0;
-        const int ts_min = (a.M + 127) / 128, ts_max = (a.M + 15) / 16;
+        double best_work = 0;
+        const int ts_min = (M + 127) / 128, ts_max = (M + 15) / 16;
         for (int ts = ts_min; ts <= ts_max; ++ts) {
-            const int T = ((a.M + ts - 1) / ts + 15) & ~15;
-            if (ts > ts_min && ((a.M + T - 1) / T != ts || tiles * ts > sm_count)) continue;
+            const int T = ((M + ts - 1) / ts + 15) & ~15;
+            if (ts > ts_min && static_cast<long long>(tiles) * ts > sm_count) break;
+            if (ts > ts_min && (M + T - 1) / T != ts) continue;
             for (int split = std::max(1, std::min({kStMaxSplit, sm_count / (tiles * ts), steps / 2})); split >= 1; --split) {
-                const int per = (steps + split - 1) / split;
-                const double cost = per * std::max(400.0, 4.0 * T) + (split > 1 ? 1500.0 + T * 512.0 * (split - 1) / split / 18.0 + 25.0 * T / split : 25.0 * T);
-                if (best.smem != 0 && cost >= best_cost) continue;
+                const int per = (steps + split - 1) / split, waves = (tiles * ts * split + sm_count - 1) / sm_count;
+                const double ends = split > 1 ? 1500.0 + T * 512.0 * (split - 1) / split / 18.0 + 25.0 * T / split : 25.0 * T;
+                const double work = per * std::max(400.0, 4.0 * T) + ends;
+                if (best.smem != 0 && work >= best_work) continue;
                 StreamPlan p;
                 if (!plan_stream(T, split, per, &p)) continue;
                 if (split > 1 && max_active_clusters(reinterpret_cast<const void*>(gemm_w4a16_tc_stream_kernel<MODE>), kStThreads, p.smem, split) < tiles * ts) continue;
                 best = p;
-                best_cost = cost;
+                best.cost = waves * (5500.0 + per * std::max(450.0, 8.6 * T) + ends);
+                best_work = work;
             }
         }
         return best;
     });
-    if (plan.smem == 0) return kStreamDoesNotFit;
-    a.p = plan;
-    if (!encode_2d(&a.tmap_x, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, x, static_cast<uint64_t>(a.K), static_cast<uint64_t>(a.M),
-                   static_cast<uint64_t>(a.K) * 2, kBK, static_cast<uint32_t>(plan.T)))
-        return W4A16_ERR_INVALID_ARG;
-    return static_cast<int>(launch_kernel_cluster(gemm_w4a16_tc_stream_kernel<MODE>, dim3(tiles, (a.M + plan.T - 1) / plan.T, plan.ksplit), dim3(kStThreads),
-                                                  plan.smem, stream, pdl_enabled(), dim3(1, 1, static_cast<unsigned>(plan.ksplit)), a));
+}
+StreamPlan stream_plan(const GemmArgs& g, int tiles, int sm_count) {
+    switch (g.mode) {
+        case kPlain: return stream_plan<kPlain>(g.M, g.K, tiles, sm_count);
+        case kQkv: return stream_plan<kQkv>(g.M, g.K, tiles, sm_count);
+        default: return stream_plan<kSwiglu>(g.M, g.K, tiles, sm_count);
+    }
 }
 // What both kernels' arguments have in common.
 template <typename Args>
@@ -310,14 +323,22 @@ int fill_args(const GemmArgs& g, Args* a, int* total_tiles) {
     for (int t = nt; t < 3; ++t) a->tmap_w[t] = a->tmap_w[0];
     return 0;
 }
-int stream_launch(const GemmArgs& g, int sm_count, cudaStream_t stream) {
+int stream_launch(const GemmArgs& g, const StreamPlan& plan, cudaStream_t stream) {
     StreamArgs a;
     int tiles = 0;
     if (int e = fill_args(g, &a, &tiles)) return e;
+    a.p = plan;
+    if (!encode_2d(&a.tmap_x, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, g.x, static_cast<uint64_t>(g.K), static_cast<uint64_t>(g.M),
+                   static_cast<uint64_t>(g.K) * 2, kBK, static_cast<uint32_t>(plan.T)))
+        return W4A16_ERR_INVALID_ARG;
+    auto launch = [&](auto* kernel) {
+        return static_cast<int>(launch_kernel_cluster(kernel, dim3(tiles, (g.M + plan.T - 1) / plan.T, plan.ksplit), dim3(kStThreads), plan.smem, stream,
+                                                      pdl_enabled(), dim3(1, 1, static_cast<unsigned>(plan.ksplit)), a));
+    };
     switch (g.mode) {
-        case kPlain: return launch_stream<kPlain>(a, g.x, tiles, sm_count, stream);
-        case kQkv: return launch_stream<kQkv>(a, g.x, tiles, sm_count, stream);
-        default: return launch_stream<kSwiglu>(a, g.x, tiles, sm_count, stream);
+        case kPlain: return launch(gemm_w4a16_tc_stream_kernel<kPlain>);
+        case kQkv: return launch(gemm_w4a16_tc_stream_kernel<kQkv>);
+        default: return launch(gemm_w4a16_tc_stream_kernel<kSwiglu>);
     }
 }
 int pair_launch(const GemmArgs& g, int sm_count, cudaStream_t stream) {
@@ -325,15 +346,13 @@ int pair_launch(const GemmArgs& g, int sm_count, cudaStream_t stream) {
     int tiles = 0;
     if (int e = fill_args(g, &a, &tiles)) return e;
     const int n_pairs = (tiles + 1) / 2, pairs = std::max(1, sm_count / 2);
-    const int T = pair_token_tile(g.M, n_pairs, g.K / kGroup, pairs);
+    const int T = pair_token_tile(g.M, n_pairs, g.K / kGroup, pairs, nullptr);
     a.halves = T > kPairAccCols ? 2 : 1;
     a.n_half = T / a.halves;
-    // Two rows of an output as one word.
+    // Two rows of an output as one word: even strides and rows, 4-byte aligned; peers get value by value stores.
     auto word = [](const void* p) { return reinterpret_cast<uintptr_t>(p) % 4 == 0; };
-    a.vec_ok = 1;
-    for (int t = 0; t < (g.mode == kQkv ? 3 : 1); ++t) a.vec_ok = a.vec_ok && a.out_ld[t] % 2 == 0 && word(a.out[t]);
-    a.vec_ok = a.vec_ok && word(a.residual);
-    for (int p = 0; p < a.num_peers; ++p) a.vec_ok = a.vec_ok && word(a.peer_out[p]);
+    bool words = a.num_peers == 0 && word(a.residual);
+    for (int t = 0; t < (g.mode == kQkv ? 3 : 1); ++t) words = words && a.out_ld[t] % 2 == 0 && a.rows[t] % 2 == 0 && word(a.out[t]);
     // weight matrices that do not stay in L2 next to the tokens and outputs: panels of 4 token tiles (measured on
     // 28672 x 8192 at 4096 tokens: 1.62 -> 1.56 ms, DRAM reads 1.77 -> under 1 GB); smaller ones: row tiles fastest
     a.panel = static_cast<size_t>(tiles) * kTileRows * (g.K / 2) > (48u << 20) ? 4 : 1;
@@ -347,19 +366,25 @@ int pair_launch(const GemmArgs& g, int sm_count, cudaStream_t stream) {
         return static_cast<int>(launch_kernel_cluster(kernel, dim3(grid), dim3(kPairThreads), smem, stream, pdl_enabled(), dim3(2, 1, 1), a));
     };
     switch (g.mode) {
-        case kPlain: return launch(gemm_w4a16_tc_pair_kernel<kPlain>);
-        case kQkv: return launch(gemm_w4a16_tc_pair_kernel<kQkv>);
-        default: return launch(gemm_w4a16_tc_pair_kernel<kSwiglu>);
+        case kPlain: return words ? launch(gemm_w4a16_tc_pair_kernel<kPlain, true>) : launch(gemm_w4a16_tc_pair_kernel<kPlain, false>);
+        case kQkv: return words ? launch(gemm_w4a16_tc_pair_kernel<kQkv, true>) : launch(gemm_w4a16_tc_pair_kernel<kQkv, false>);
+        default: return launch(gemm_w4a16_tc_pair_kernel<kSwiglu, true>);
     }
 }
 }  // namespace
 
-// Up to 256 tokens the streaming kernel (more CTAs, K split), above that CTA pairs; W4A16_OPT_GEMM_FORM = 1 / 2 asks for one of them.
+// Up to 256 tokens the streaming kernel (more CTAs, K split), above that whichever of the two is estimated to be faster: thin
+// matrices stay with the streaming kernel up to about 1024 tokens (QKV at 1024: 9.4 us against 11.7 on pairs), gate_up goes to
+// pairs at once (300 tokens: 29.7 against 23.2 us).  W4A16_OPT_GEMM_FORM = 1 / 2 asks for one of them.
 int gemm_tc_launch(const GemmArgs& g, int sm_count, cudaStream_t stream) {
     const int form = option(W4A16_OPT_GEMM_FORM);
-    if (form == 1 || (form == 0 && g.M <= 256)) {
-        const int e = stream_launch(g, sm_count, stream);
-        if (e != kStreamDoesNotFit) return e;
+    if (form != 2) {
+        int tiles = 0;
+        for (int t = 0; t < (g.mode == kQkv ? 3 : 1); ++t) tiles += (g.rows[t] + kTileRows - 1) / kTileRows;
+        const StreamPlan plan = stream_plan(g, tiles, sm_count);
+        double pairs_cost = 0;
+        if (form == 0 && g.M > 256) pair_token_tile(g.M, (tiles + 1) / 2, g.K / kGroup, std::max(1, sm_count / 2), &pairs_cost);
+        if (plan.smem != 0 && (form == 1 || g.M <= 256 || plan.cost < pairs_cost)) return stream_launch(g, plan, stream);
     }
     return pair_launch(g, sm_count, stream);
 }

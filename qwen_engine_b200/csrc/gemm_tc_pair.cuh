@@ -48,7 +48,6 @@ struct PairArgs {
     const __half* residual;
     int M, K;
     int halves, n_half;      // accumulators of a tile and tokens of each: T = halves * n_half
-    int vec_ok;              // outputs (and residual) can be written two rows at a time: even strides, 4-byte aligned
     int panel;               // token tiles per panel of the tile order
     __half* peer_out[7];     // PLAIN: the output block's place in other GPUs' matrices
     int num_peers;
@@ -128,63 +127,22 @@ __device__ __forceinline__ PairTile pair_tile(const PairArgs& a, int pt, int n_p
     return r;
 }
 
-// Eight tokens m0 .. m0 + 7 of weight row n.  All lanes of a warp call it with consecutive rows and the same tokens.  The
-// even lane of a pair finishes the first token of two, the odd lane the second: SWIGLU has its gate in the even and its
-// up in the odd row, the others store both rows of a token as one word.
-template <int MODE>
-__device__ __forceinline__ void pair_store8(const PairArgs& a, int t, int n, int m0, const float (&acc)[8]) {
-    const int odd = n & 1, ne = n & ~1, rows = a.rows[t];
-    const size_t ld = static_cast<size_t>(a.out_ld[t]);
-#pragma unroll
-    for (int q = 0; q < 8; q += 2) {
-        const float other = __shfl_xor_sync(0xFFFFFFFFu, odd ? acc[q] : acc[q + 1], 1);
-        const float even_row = odd ? other : acc[q], odd_row = odd ? acc[q + 1] : other;
-        const int m = m0 + q + odd;
-        if (m >= a.M || ne >= rows) continue;
-        if constexpr (MODE == kSwiglu) {
-            a.out[t][static_cast<size_t>(m) * ld + (n >> 1)] = __float2half_rn(swiglu_f32(even_row, odd_row));
-        } else {
-            const size_t off = static_cast<size_t>(m) * ld + ne;
-            __half y[2] = {__float2half_rn(even_row), __float2half_rn(odd_row)};
-            for (int i = 0; i < (ne + 1 < rows ? 2 : 1); ++i) {
-                if constexpr (MODE == kPlain) {
-                    if (a.residual != nullptr) y[i] = __hadd(y[i], a.residual[off + i]);
-                }
-                a.out[t][off + i] = y[i];
-            }
-            if constexpr (MODE == kPlain) {
-                for (int p = 0; p < a.num_peers; ++p) {
-                    if (a.vec_ok && ne + 1 < rows) {
-                        *reinterpret_cast<__half2*>(a.peer_out[p] + off) = __halves2half2(y[0], y[1]);
-                    } else {
-                        a.peer_out[p][off] = y[0];
-                        if (ne + 1 < rows) a.peer_out[p][off + 1] = y[1];
-                    }
-                }
-            }
-        }
-    }
-}
-// The same for a tile that lies inside the output, addresses given: this lane's first token and output, `step` bytes from
-// one of its tokens to the next.
-template <int MODE>
-__device__ __forceinline__ void pair_store8_inside(char* out, size_t step, int odd, const float (&acc)[8], const __half2 (&res)[4], bool add) {
+// Eight tokens of a weight row.  All lanes of a warp call it with consecutive rows and the same tokens.  The even lane of a
+// pair finishes the first token of two, the odd lane the second: SWIGLU has its gate in the even and its up in the odd row,
+// the others hold both rows of a token.  `take(q, even_row, odd_row)` gets token pair q.
+template <typename F>
+__device__ __forceinline__ void pair_exchange8(int odd, const uint32_t (&v)[8], F&& take) {
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
-        const float other = __shfl_xor_sync(0xFFFFFFFFu, odd ? acc[2 * q] : acc[2 * q + 1], 1);
-        const float even_row = odd ? other : acc[2 * q], odd_row = odd ? acc[2 * q + 1] : other;
-        if constexpr (MODE == kSwiglu) {
-            *reinterpret_cast<__half*>(out) = __float2half_rn(swiglu_f32(even_row, odd_row));
-        } else {
-            __half2 y = __floats2half2_rn(even_row, odd_row);
-            if (MODE == kPlain && add) y = __hadd2(y, res[q]);
-            *reinterpret_cast<__half2*>(out) = y;
-        }
-        out += step;
+        const float a = __uint_as_float(v[2 * q]), b = __uint_as_float(v[2 * q + 1]);
+        const float other = __shfl_xor_sync(0xFFFFFFFFu, odd ? a : b, 1);
+        take(q, odd ? other : a, odd ? b : other);
     }
 }
 
-template <int MODE>
+// WORDS: both rows of an output lie in one aligned word and nothing goes to peers (the host checks); the other form stores
+// value by value.
+template <int MODE, bool WORDS>
 __global__ void __launch_bounds__(kPairThreads, 1) gemm_w4a16_tc_pair_kernel(const __grid_constant__ PairArgs a) {
     constexpr int kEpi0 = kPairDqWarps, kMmaWarp = kEpi0 + kPairEpiWarps, kRawWarp = kMmaWarp + 1;
     extern __shared__ uint8_t smem_raw_base[];
@@ -204,6 +162,7 @@ __global__ void __launch_bounds__(kPairThreads, 1) gemm_w4a16_tc_pair_kernel(con
     constexpr int kBars = 2 * kPairRawSlots + 2 * kPairSlots + 4;
     uint32_t* s_tmem = reinterpret_cast<uint32_t*>(s_bar + kBars);
     volatile int* s_abort = reinterpret_cast<volatile int*>(s_tmem + 1);
+    volatile int* s_epi_ok = reinterpret_cast<volatile int*>(s_tmem + 2);
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int rank = static_cast<int>(cluster_cta_rank());
@@ -249,18 +208,21 @@ __global__ void __launch_bounds__(kPairThreads, 1) gemm_w4a16_tc_pair_kernel(con
         int rs = g, slot = g;                    // ring positions of this group's next step
         uint32_t rph = 0, dph = 1;               // parities: raw slot filled; slot freed by its previous use
         int it = 0, st = g;                      // tile iteration and step in it
-        PairTile pt = my_tiles > 0 ? pair_tile(a, pair_id, n_pairs, rank, MODE == kQkv) : PairTile{0, 0, 0};
+        const __half* sc_row = nullptr;          // scales of this thread's row; null past the tensor
+        auto row_of = [&](int iteration) {
+            const PairTile pt = pair_tile(a, pair_id + iteration * num_pairs, n_pairs, rank, MODE == kQkv);
+            const int row = pt.n0 + r;
+            sc_row = row < a.rows[pt.t] ? a.scales[pt.t] + static_cast<size_t>(row) * G : nullptr;
+        };
         auto settle = [&]() {                    // (it, st) back into range after st moved on
             while (st >= G) {
                 st -= G;
-                if (++it < my_tiles) pt = pair_tile(a, pair_id + it * num_pairs, n_pairs, rank, MODE == kQkv);
+                if (++it < my_tiles) row_of(it);
             }
         };
-        auto load_scale = [&]() -> __half {
-            const int row = pt.n0 + r;
-            return row < a.rows[pt.t] ? __ldg(a.scales[pt.t] + static_cast<size_t>(row) * G + st) : __half(0.0f);
-        };
+        if (my_tiles > 0) row_of(0);
         settle();
+        auto load_scale = [&]() -> __half { return sc_row != nullptr ? __ldg(sc_row + st) : __half(0.0f); };
         __half sc_next = g < total ? load_scale() : __half(0.0f);
         for (int i = g; i < total; i += kPairGroups) {
             const __half sc = sc_next;
@@ -271,10 +233,11 @@ __global__ void __launch_bounds__(kPairThreads, 1) gemm_w4a16_tc_pair_kernel(con
             if (!ok) break;
             const uint8_t* raw_row = s_raw + rs * kPairRawBytes + r * 64;
             const __half2 sc2 = __half2half2(sc);
-            uint32_t cols[2][32];
+            const uint32_t a_slot = a_lane + static_cast<uint32_t>(slot * kPairACols);
             if (__all_sync(0xFFFFFFFFu, __habs(sc) < __float2half_rn(0.0624f))) {
                 const __half2 k10 = __float2half2_rn(1024.0f);
                 const __half2 s20 = __hmul2(__hmul2(sc2, k10), k10), m8s = __hmul2(sc2, __float2half2_rn(-8.0f));
+                uint32_t cols[2][32];
 #pragma unroll
                 for (int c = 0; c < 4; ++c) {
                     const uint4 w = *reinterpret_cast<const uint4*>(raw_row + ((c ^ swz) << 4));
@@ -284,31 +247,35 @@ __global__ void __launch_bounds__(kPairThreads, 1) gemm_w4a16_tc_pair_kernel(con
                     dequant_word_small_scale(w.z, s20, m8s, o + 8);
                     dequant_word_small_scale(w.w, s20, m8s, o + 12);
                 }
+                ok = group_wait(done(slot), dph, s_abort, lane);
+                if (!ok) break;
+                tc_fence_after();
+                tmem_st32(a_slot, cols[0]);
+                tmem_st32(a_slot + 32u, cols[1]);
             } else {
-#pragma unroll
+                ok = group_wait(done(slot), dph, s_abort, lane);
+                if (!ok) break;
+                tc_fence_after();
+#pragma unroll 1
                 for (int c = 0; c < 4; ++c) {
                     const uint4 w = *reinterpret_cast<const uint4*>(raw_row + ((c ^ swz) << 4));
                     const uint32_t words[4] = {w.x, w.y, w.z, w.w};
+                    uint32_t cols[16];
 #pragma unroll
                     for (int k = 0; k < 4; ++k) {
                         __half2 h[4];
                         dequant_word_fp16(words[k], sc2, h);
 #pragma unroll
-                        for (int q = 0; q < 4; ++q) cols[c >> 1][16 * (c & 1) + 4 * k + q] = *reinterpret_cast<const uint32_t*>(&h[q]);
+                        for (int q = 0; q < 4; ++q) cols[4 * k + q] = *reinterpret_cast<const uint32_t*>(&h[q]);
                     }
+                    tmem_st16(a_slot + 16u * c, cols);
                 }
             }
-            __syncwarp();
-            if (lane == 0) mbar_arrive(raw_empty(rs));
-            ok = group_wait(done(slot), dph, s_abort, lane);
-            if (!ok) break;
-            tc_fence_after();
-            tmem_st32(a_lane + static_cast<uint32_t>(slot * kPairACols), cols[0]);
-            tmem_st32(a_lane + static_cast<uint32_t>(slot * kPairACols + 32), cols[1]);
             tmem_st_wait();
             tc_fence_before();
             __syncwarp();
             if (lane == 0) {
+                mbar_arrive(raw_empty(rs));
                 if (leader) mbar_arrive(full(slot));
                 else mbar_arrive_remote(leader_full0 + 8u * slot);
             }
@@ -331,23 +298,28 @@ __global__ void __launch_bounds__(kPairThreads, 1) gemm_w4a16_tc_pair_kernel(con
         pdl_wait_prior_grids();                  // the previous kernels' reads of the outputs and writes of the residual
         for (int pt_i = pair_id; pt_i < total_pt && ok; pt_i += num_pairs) {
             const PairTile pt = pair_tile(a, pt_i, n_pairs, rank, MODE == kQkv);
+            const int ne = (pt.n0 + r) & ~1, rows = a.rows[pt.t];
             for (int h = 0; h < H; ++h) {
-                const int m0 = pt.m0 + h * NH + 8 * part;
-                const bool inside = a.vec_ok && pt.n0 + kTileRows <= a.rows[pt.t] && pt.m0 + (h + 1) * NH <= a.M && (MODE != kPlain || a.num_peers == 0);
+                const int m0 = pt.m0 + h * NH + 8 * part + odd;        // this lane's first token
                 const size_t ld = static_cast<size_t>(a.out_ld[pt.t]);
-                const size_t off = static_cast<size_t>(m0 + odd) * ld + (MODE == kSwiglu ? (pt.n0 + r) >> 1 : (pt.n0 + r) & ~1);
-                // the residual of the first groups while the tensor core is still at it
-                __half2 res[2][4];
+                const size_t off = static_cast<size_t>(m0) * ld + (MODE == kSwiglu ? ne >> 1 : ne);
+                const int left = ne < rows ? a.M - m0 : 0;             // this lane's tokens are 0, 2, 4, .. below that
+                // the residual of the first group while the tensor core is still at it
+                __half2 res[4];
                 auto load_res = [&](int i) {
 #pragma unroll
-                    for (int q = 0; q < 4; ++q) res[i & 1][q] = *reinterpret_cast<const __half2*>(a.residual + off + static_cast<size_t>(32 * i + 2 * q) * ld);
+                    for (int q = 0; q < 4; ++q)
+                        if (32 * i + 2 * q < left) res[q] = *reinterpret_cast<const __half2*>(a.residual + off + static_cast<size_t>(32 * i + 2 * q) * ld);
                 };
-                if (add && inside) {
-#pragma unroll
-                    for (int i = 0; i < 2; ++i)
-                        if (i < n_groups) load_res(i);
+                if (WORDS && add) load_res(0);
+                // One warp polls, the others wait at a block barrier: sixteen polling warps slow the dequantising ones down.
+                // Its answer goes through one word per buffer, rewritten only after everybody has read it.
+                if (warp == kEpi0) {
+                    ok = group_wait(acc_full(buf), ph, s_abort, lane);
+                    if (lane == 0) s_epi_ok[buf] = ok ? 1 : 0;
                 }
-                ok = group_wait(acc_full(buf), ph, s_abort, lane);
+                asm volatile("bar.sync 1, %0;" ::"n"(kPairEpiWarps * 32) : "memory");
+                ok = s_epi_ok[buf] != 0;
                 if (!ok) break;
                 tc_fence_after();
                 // this warp's columns into registers, then the accumulator goes back
@@ -362,20 +334,34 @@ __global__ void __launch_bounds__(kPairThreads, 1) gemm_w4a16_tc_pair_kernel(con
                     if (leader) mbar_arrive(acc_empty(buf));
                     else mbar_arrive_remote(leader_empty0 + 8u * buf);
                 }
-                char* out = reinterpret_cast<char*>(a.out[pt.t] + off);
+                __half* out = a.out[pt.t] + off;
 #pragma unroll
                 for (int i = 0; i < kMaxGroups; ++i) {
                     if (i < n_groups) {
-                        float acc[8];
-#pragma unroll
-                        for (int q = 0; q < 8; ++q) acc[q] = __uint_as_float(v[i][q]);
-                        if (inside) {
-                            pair_store8_inside<MODE>(out, 4 * ld, odd, acc, res[i & 1], add);
-                            if (add && i + 2 < n_groups) load_res(i + 2);
-                            out += 64 * ld;
-                        } else if (m0 + 32 * i < a.M) {
-                            pair_store8<MODE>(a, pt.t, pt.n0 + r, m0 + 32 * i, acc);
-                        }
+                        pair_exchange8(odd, v[i], [&](int q, float even_row, float odd_row) {
+                            const bool on = 32 * i + 2 * q < left;
+                            if constexpr (MODE == kSwiglu) {
+                                const __half y = __float2half_rn(swiglu_f32(even_row, odd_row));
+                                if (on) *out = y;
+                            } else if constexpr (WORDS) {
+                                __half2 y = __floats2half2_rn(even_row, odd_row);
+                                if (add) y = __hadd2(y, res[q]);
+                                if (on) *reinterpret_cast<__half2*>(out) = y;
+                            } else if (on) {
+                                const size_t o = static_cast<size_t>(out - a.out[pt.t]);
+                                for (int k = 0; k < (ne + 1 < rows ? 2 : 1); ++k) {
+                                    __half y = __float2half_rn(k == 0 ? even_row : odd_row);
+                                    if constexpr (MODE == kPlain) {
+                                        if (add) y = __hadd(y, a.residual[o + k]);
+                                        for (int p = 0; p < a.num_peers; ++p) a.peer_out[p][o + k] = y;
+                                    }
+                                    out[k] = y;
+                                }
+                            }
+                            out += 2 * ld;
+                        });
+                        out += 24 * ld;          // the groups of the other three warps
+                        if (WORDS && add && i + 1 < n_groups) load_res(i + 1);
                     }
                 }
                 buf ^= 1;
@@ -520,12 +506,13 @@ double pair_cost(int M, int n_pairs, int steps, int pairs, int T) {
     return rounds * (steps * std::max(4.0 * T, 950.0) + (T > kPairAccCols ? 2500.0 : 0.0)) + 6000.0 + 25.0 * T;
 }
 // The token tile for `n_pairs` pairs of row tiles on `pairs` pairs of SMs: one accumulator of 16..128 or two of 80..128.
-int pair_token_tile(int M, int n_pairs, int steps, int pairs) {
+int pair_token_tile(int M, int n_pairs, int steps, int pairs, double* estimate) {
     int best = 16;
     double best_cost = 0;
     for (int T = 16; T <= 2 * kPairAccCols; T += T < kPairAccCols ? 16 : 32) {
         const double cost = pair_cost(M, n_pairs, steps, pairs, T);
         if (best_cost == 0 || cost < best_cost) { best = T; best_cost = cost; }
     }
+    if (estimate != nullptr) *estimate = best_cost;
     return best;
 }

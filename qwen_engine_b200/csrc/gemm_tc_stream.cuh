@@ -46,6 +46,7 @@ struct StreamPlan {
     int part_offset;      // K split: byte offset of the partials in shared memory; 0 = on top of the rings
     int acc2_col, a_col;  // second accumulator; first column of the A slots
     size_t smem = 0;      // 0: does not fit
+    double cost = 0;      // estimated cycles
 };
 struct StreamArgs {
     CUtensorMap tmap_w[3];

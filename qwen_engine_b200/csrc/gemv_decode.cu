@@ -640,9 +640,13 @@ __global__ void __launch_bounds__(kMaxThreads, 2) gemv_w4_stream_kernel(const Ge
             seq_pos = static_cast<uint32_t>(c->seq_pos);
         }
     }
-    if constexpr (XIN == kXFp16Norm) stage_x_from_fp16_rmsnorm(a.x_fp16, a.gamma, K, kRmsEps, s_q8, s_seed, s_scale);
-    else if constexpr (XIN == kXFp16) stage_x_from_fp16(a.x_fp16, K, s_q8, s_seed, s_scale);
-    else stage_x_from_q8_1(a.q8, a.xscale, a.sum8, K, a.vec_ok != 0, s_q8, s_seed, s_scale);
+    if constexpr (XIN == kXFp16Norm) {
+        stage_x_from_fp16_rmsnorm(a.x_fp16, a.gamma, K, kRmsEps, s_q8, s_seed, s_scale);
+    } else if constexpr (XIN == kXFp16) {
+        stage_x_from_fp16(a.x_fp16, K, s_q8, s_seed, s_scale);
+    } else if (!stage_x_from_q8_1_regs<STEPS == 8>(a.q8, a.xscale, a.sum8, K, a.vec_ok != 0, s_q8, s_seed, s_scale)) {
+        stage_x_from_q8_1(a.q8, a.xscale, a.sum8, K, a.vec_ok != 0, s_q8, s_seed, s_scale);
+    }
     __syncthreads();
 
     uint4 xa[STEPS], xb[STEPS];
@@ -798,8 +802,8 @@ __global__ void __launch_bounds__(kMaxThreads, 2) gemv_w4_stream_kernel(const Ge
 // activation read from shared memory (a lane's share of an 8192-element vector would not fit registers).
 // A row's chunks are accumulated in K order by the same lane as in gemv_w4_kernel without a K split, so the
 // two agree bit for bit.  PLAIN mode, 16-byte aligned weights.
-template <int XIN, bool FULL>     // FULL: K is a multiple of 2048, every slice has all 8 steps (no guards in the loops)
-__global__ void __launch_bounds__(kMaxThreads, 2) gemv_w4_stream_longk_kernel(const GemvArgs a, const int num_blocks) {
+template <int XIN, bool FULL, int THREADS>     // FULL: K is a multiple of 2048, every slice has all 8 steps (no guards in the loops)
+__global__ void __launch_bounds__(THREADS, 2) gemv_w4_stream_longk_kernel(const GemvArgs a, const int num_blocks) {
     constexpr int STEPS = 8;
     extern __shared__ __align__(16) uint8_t smem[];
     const int K = a.K;
@@ -816,7 +820,7 @@ __global__ void __launch_bounds__(kMaxThreads, 2) gemv_w4_stream_longk_kernel(co
         if (++sl == nslices) { sl = 0; blk += gridDim.x; }
     };
     auto issue = [&](uint4 (&w)[STEPS], uint16_t (&sb)[STEPS], int blk, int sl) {
-        const int row = min(blk * kMaxSubwarps + sub, N - 1);      // rows past the end re-read the last row; never stored
+        const int row = min(blk * (THREADS / kSubwarp) + sub, N - 1);      // rows past the end re-read the last row; never stored
         const uint32_t* wp = a.qweight[0] + static_cast<size_t>(row) * words + (sl * STEPS * kSubwarp + l) * 4;
         const __half* sp = a.scales[0] + static_cast<size_t>(row) * groups + 2 * sl * STEPS + (l >> 2);
 #pragma unroll
@@ -849,7 +853,7 @@ __global__ void __launch_bounds__(kMaxThreads, 2) gemv_w4_stream_longk_kernel(co
             acc += __shfl_xor_sync(0xFFFFFFFFu, acc, 4);
             acc += __shfl_xor_sync(0xFFFFFFFFu, acc, 2);
             acc += __shfl_xor_sync(0xFFFFFFFFu, acc, 1);
-            const int row = blk * kMaxSubwarps + sub;
+            const int row = blk * (THREADS / kSubwarp) + sub;
             if (l == 0 && row < N) {
                 float y = acc;
                 if (a.residual != nullptr) y += __half2float(a.residual[row]);
@@ -867,9 +871,13 @@ __global__ void __launch_bounds__(kMaxThreads, 2) gemv_w4_stream_longk_kernel(co
     if (blk < num_blocks) issue(w0, sb0, blk, 0);
     pdl_release_dependents();
     pdl_wait_prior_grids();
-    if constexpr (XIN == kXFp16Norm) stage_x_from_fp16_rmsnorm(a.x_fp16, a.gamma, K, kRmsEps, s_q8, s_seed, s_scale);
-    else if constexpr (XIN == kXFp16) stage_x_from_fp16(a.x_fp16, K, s_q8, s_seed, s_scale);
-    else stage_x_from_q8_1(a.q8, a.xscale, a.sum8, K, a.vec_ok != 0, s_q8, s_seed, s_scale);
+    if constexpr (XIN == kXFp16Norm) {
+        stage_x_from_fp16_rmsnorm(a.x_fp16, a.gamma, K, kRmsEps, s_q8, s_seed, s_scale);
+    } else if constexpr (XIN == kXFp16) {
+        stage_x_from_fp16(a.x_fp16, K, s_q8, s_seed, s_scale);
+    } else if (!stage_x_from_q8_1_regs<true>(a.q8, a.xscale, a.sum8, K, a.vec_ok != 0, s_q8, s_seed, s_scale)) {
+        stage_x_from_q8_1(a.q8, a.xscale, a.sum8, K, a.vec_ok != 0, s_q8, s_seed, s_scale);
+    }
     __syncthreads();
     // two register sets used in turn: the next unit's words are in flight while this one is multiplied
     while (blk < num_blocks) {
@@ -1095,12 +1103,18 @@ int gemv_set_attributes() {
     if (e == cudaSuccess) e = raise_smem_mode<kSwiglu, 4>();
     if (e == cudaSuccess) e = raise_smem_mode<kSwiglu, 8>();
     if (e == cudaSuccess) e = raise_smem(gemv_group_dots_kernel);
-    if (e == cudaSuccess) e = raise_smem(gemv_w4_stream_longk_kernel<kXQ8, true>);
-    if (e == cudaSuccess) e = raise_smem(gemv_w4_stream_longk_kernel<kXQ8, false>);
-    if (e == cudaSuccess) e = raise_smem(gemv_w4_stream_longk_kernel<kXFp16, true>);
-    if (e == cudaSuccess) e = raise_smem(gemv_w4_stream_longk_kernel<kXFp16, false>);
-    if (e == cudaSuccess) e = raise_smem(gemv_w4_stream_longk_kernel<kXFp16Norm, true>);
-    if (e == cudaSuccess) e = raise_smem(gemv_w4_stream_longk_kernel<kXFp16Norm, false>);
+    if (e == cudaSuccess) e = raise_smem(gemv_w4_stream_longk_kernel<kXQ8, true, 256>);
+    if (e == cudaSuccess) e = raise_smem(gemv_w4_stream_longk_kernel<kXQ8, true, 288>);
+    if (e == cudaSuccess) e = raise_smem(gemv_w4_stream_longk_kernel<kXQ8, false, 256>);
+    if (e == cudaSuccess) e = raise_smem(gemv_w4_stream_longk_kernel<kXQ8, false, 288>);
+    if (e == cudaSuccess) e = raise_smem(gemv_w4_stream_longk_kernel<kXFp16, true, 256>);
+    if (e == cudaSuccess) e = raise_smem(gemv_w4_stream_longk_kernel<kXFp16, true, 288>);
+    if (e == cudaSuccess) e = raise_smem(gemv_w4_stream_longk_kernel<kXFp16, false, 256>);
+    if (e == cudaSuccess) e = raise_smem(gemv_w4_stream_longk_kernel<kXFp16, false, 288>);
+    if (e == cudaSuccess) e = raise_smem(gemv_w4_stream_longk_kernel<kXFp16Norm, true, 256>);
+    if (e == cudaSuccess) e = raise_smem(gemv_w4_stream_longk_kernel<kXFp16Norm, true, 288>);
+    if (e == cudaSuccess) e = raise_smem(gemv_w4_stream_longk_kernel<kXFp16Norm, false, 256>);
+    if (e == cudaSuccess) e = raise_smem(gemv_w4_stream_longk_kernel<kXFp16Norm, false, 288>);
     if (e == cudaSuccess) e = prepare_bulk_mode<kPlain>();
     if (e == cudaSuccess) e = prepare_bulk_mode<kQkv>();
     if (e == cudaSuccess) e = prepare_bulk_mode<kSwiglu>();
@@ -1178,13 +1192,20 @@ int gemv_launch(GemvMode mode, GemvArgs a, cudaStream_t stream) {
     if (mode == kPlain && !q8_epilogue && !sampling && !handoff && aligned16 && steps > 8 && a.x_f32 == nullptr &&
         static_cast<long long>(num_blocks) * ((steps + 7) / 8) >= 8LL * 2 * dev->sm_count &&
         staged_x_bytes(a.K) <= 160 * 1024 && option(W4A16_OPT_GEMV_FORM) != 2) {
-        const dim3 sgrid(std::min(num_blocks, 2 * dev->sm_count)), sblock(kMaxThreads);
+        // Nine warps per CTA where that saves a round: the CTAs walk in rounds of (2 x SMs) x 32 or 36 rows, and a round for a
+        // handful of rows costs the latency of all of a row's slices (28672 rows: 3.03 rounds of 32, 2.69 of 36).
+        const int ctas = 2 * dev->sm_count;
+        const bool nine = (a.units + ctas * 36 - 1) / (ctas * 36) < (a.units + ctas * 32 - 1) / (ctas * 32);
+        const int threads_l = nine ? 288 : 256, blocks_l = (a.units + threads_l / kSubwarp - 1) / (threads_l / kSubwarp);
+        const dim3 sgrid(std::min(blocks_l, ctas)), sblock(threads_l);
         const size_t ssmem = staged_x_bytes(a.K);
         const bool pdl = pdl_enabled();
-#define W4_LONGK(XINV) (steps % 8 == 0 ? launch_kernel(gemv_w4_stream_longk_kernel<XINV, true>, sgrid, sblock, ssmem, stream, pdl, a, num_blocks) \
-                                       : launch_kernel(gemv_w4_stream_longk_kernel<XINV, false>, sgrid, sblock, ssmem, stream, pdl, a, num_blocks))
+#define W4_LONGK2(XINV, F) (nine ? launch_kernel(gemv_w4_stream_longk_kernel<XINV, F, 288>, sgrid, sblock, ssmem, stream, pdl, a, blocks_l) \
+                                 : launch_kernel(gemv_w4_stream_longk_kernel<XINV, F, 256>, sgrid, sblock, ssmem, stream, pdl, a, blocks_l))
+#define W4_LONGK(XINV) (steps % 8 == 0 ? W4_LONGK2(XINV, true) : W4_LONGK2(XINV, false))
         if (a.x_fp16 != nullptr) e = a.gamma != nullptr ? W4_LONGK(kXFp16Norm) : W4_LONGK(kXFp16);
         else e = W4_LONGK(kXQ8);
+#undef W4_LONGK2
 #undef W4_LONGK
         return static_cast<int>(e);
     }

@@ -91,6 +91,67 @@ __global__ void __launch_bounds__(kNormThreads) rmsnorm_q8_1_kernel(const __half
     }
 }
 
+// The same for vectors a CTA can hold in registers (hidden <= 8192, 16-byte aligned): eight elements a thread, a half-warp per
+// group of 128.  A launch of one CTA is latency only, so there is one global round trip behind the wait (the gain, a weight,
+// is fetched before it), one barrier, and every warp finishes the sum of squares itself; nothing passes through shared memory
+// but the warps' sums.  @RMS@
+__global__ void __launch_bounds__(1024) rmsnorm_q8_1_regs_kernel(const __half* __restrict__ in, const __half* __restrict__ gamma,
+                                                                 __half* __restrict__ out_opt, int8_t* __restrict__ q8,
+                                                                 float* __restrict__ scale, int32_t* __restrict__ sum8, int hidden,
+                                                                 float eps) {
+    __shared__ double s_warp[32];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, hl = tid & 15;
+    const bool on = tid * 8 < hidden;
+    uint4 gr = make_uint4(0, 0, 0, 0), xr = make_uint4(0, 0, 0, 0);
+    if (on) gr = __ldg(reinterpret_cast<const uint4*>(gamma) + tid);
+    pdl_release_dependents();
+    pdl_wait_prior_grids();
+    if (on) xr = reinterpret_cast<const uint4*>(in)[tid];
+    const __half2* xh = reinterpret_cast<const __half2*>(&xr);
+    const __half2* gh = reinterpret_cast<const __half2*>(&gr);
+    double ss = 0.0;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        const float2 f = __half22float2(xh[k]);
+        // (a square of an fp16 value is exact in fp32; the sums are in double)
+        ss += static_cast<double>(f.x * f.x) + static_cast<double>(f.y * f.y);
+    }
+#pragma unroll
+    for (int m = 16; m > 0; m >>= 1) ss += __shfl_xor_sync(0xFFFFFFFFu, ss, m);
+    if (lane == 0) s_warp[warp] = ss;
+    __syncthreads();
+    double t = lane < (static_cast<int>(blockDim.x) >> 5) ? s_warp[lane] : 0.0;
+#pragma unroll
+    for (int m = 16; m > 0; m >>= 1) t += __shfl_xor_sync(0xFFFFFFFFu, t, m);
+    const __half2 inv2 = __float2half2_rn(inv_rms_from_sumsq(t, hidden, eps));
+    __half2 y[4];
+    float v[8];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        y[k] = __hmul2(__hmul2(xh[k], inv2), gh[k]);
+        const float2 f = __half22float2(y[k]);
+        v[2 * k] = f.x;
+        v[2 * k + 1] = f.y;
+    }
+    float m = 0.0f;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) m = fmaxf(m, fabsf(v[j]));
+#pragma unroll
+    for (int mask = 8; mask > 0; mask >>= 1) m = fmaxf(m, __shfl_xor_sync(0xFFFFFFFFu, m, mask));
+    const float d = fmaxf(__fdiv_rn(m, 127.0f), 1e-8f), inv_d = __fdiv_rn(1.0f, d);
+    uint32_t packed[2] = {0, 0};
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+        const int q = max(-127, min(127, __float2int_rn(__fmul_rn(v[j], inv_d))));
+        packed[j >> 2] |= (static_cast<uint32_t>(q) & 0xFFu) << (8 * (j & 3));
+    }
+    if (!on) return;
+    reinterpret_cast<uint2*>(q8)[tid] = make_uint2(packed[0], packed[1]);
+    sum8[tid] = -8 * (byte_sum(packed[0]) + byte_sum(packed[1]));
+    if (hl == 0) scale[tid >> 4] = d;
+    if (out_opt != nullptr) reinterpret_cast<uint4*>(out_opt)[tid] = *reinterpret_cast<const uint4*>(y);
+}
+
 // Q8_1 of attention heads from their fp32 accumulators (the epilogue of the reference's flash-decode combine
 // kernel, src/kernels/attention_gqa.cu:258-310, as a kernel of its own): one half-warp per head of 128.
 // Also writes fp16(acc) -- the reference's attn_out -- when out_fp16_opt is given.
@@ -153,6 +214,10 @@ int quantize_fp16_to_q8_1(const __half* x, int8_t* q8, float* scale, int32_t* su
 int rmsnorm_q8_1(const __half* in, const __half* gamma, __half* out_opt, int8_t* q8, float* scale, int32_t* sum8,
                  int hidden, cudaStream_t stream) {
     constexpr float kEps = 1e-6f;  // reference include/config.cuh:20 RMS_NORM_EPS
+    const uintptr_t all = reinterpret_cast<uintptr_t>(in) | reinterpret_cast<uintptr_t>(gamma) | reinterpret_cast<uintptr_t>(out_opt);
+    if (hidden <= 8192 && all % 16 == 0 && reinterpret_cast<uintptr_t>(q8) % 8 == 0)
+        return static_cast<int>(launch_kernel(rmsnorm_q8_1_regs_kernel, dim3(1), dim3((hidden / 8 + 31) / 32 * 32), 0, stream, pdl_enabled(), in,
+                                              gamma, out_opt, q8, scale, sum8, hidden, kEps));
     const size_t smem = static_cast<size_t>(hidden) * sizeof(__half);
     cudaError_t e = launch_kernel(rmsnorm_q8_1_kernel, dim3(1), dim3(kNormThreads), smem, stream, pdl_enabled(), in,
                                   gamma, out_opt, q8, scale, sum8, hidden, kEps);

@@ -573,6 +573,27 @@ __global__ void __maxnreg__(64) gemv_w4_bulk_kernel(const GemvArgs a) {
 
 namespace {
 
+// The group scales of up to eight steps of a sub-warp's row.  A step of 256 has two groups: lanes 0..3 need the first, lanes
+// 4..7 the second.  Lane l = 4 h + q fetches the scale of group h of the steps q and q + 4, multiplies it with the activation's
+// there, and a step's product reaches the other lanes by one shuffle: two loads and two products a lane where a load and a
+// product per lane and step made the scales, 3% of the bytes, half of the requests (lm_head with token selection 25.3 ->
+// 22.7 us, 28672 x 8192 22.6 -> 20.2 us on B200, 0.9 of what a plain read of the same bytes takes).
+struct ScalePair {
+    uint16_t bits[2];
+};
+// row_scales: the first step's two groups; n: steps there are
+__device__ __forceinline__ ScalePair load_scale_pair(const __half* row_scales, int n, int l) {
+    const int q = l & 3, h = l >> 2;
+    ScalePair s;
+    s.bits[0] = q < n ? ld_scale_bits(row_scales + 2 * q + h) : 0;
+    s.bits[1] = q + 4 < n ? ld_scale_bits(row_scales + 2 * (q + 4) + h) : 0;
+    return s;
+}
+// The product of step i for this lane, from the two products each lane of the sub-warp holds (whole warps call it).
+__device__ __forceinline__ float product_of_step(const float (&p)[2], int i, int l) {
+    return __shfl_sync(0xFFFFFFFFu, p[i >> 2], (l & 4) | (i & 3), kSubwarp);
+}
+
 // Streaming form for very tall matrices (lm_head): a persistent grid, each CTA walks row blocks of 32 with
 // the weights of the NEXT block already in flight while the current one is reduced, and the lane's share
 // of the quantised activation lives in registers for the whole launch (a lane always meets the same
@@ -595,8 +616,8 @@ __global__ void __launch_bounds__(kMaxThreads, 2) gemv_w4_stream_kernel(const Ge
     const int N = SWIGLU ? 2 * a.units : a.units;   // weight rows (SwiGLU: gate/up pairs = adjacent sub-warps)
 
     uint4 w0[STEPS], w1[STEPS];
-    uint16_t sb0[STEPS], sb1[STEPS];
-    auto issue = [&](uint4 (&w)[STEPS], uint16_t (&sb)[STEPS], int blk) {
+    ScalePair sp0 = {}, sp1 = {};
+    auto issue = [&](uint4 (&w)[STEPS], ScalePair& sp, int blk) {
         const int row = blk * kMaxSubwarps + sub;
         const bool on_row = row < N;
         const uint32_t* wrow = a.qweight[0] + static_cast<size_t>(on_row ? row : 0) * words;
@@ -605,16 +626,15 @@ __global__ void __launch_bounds__(kMaxThreads, 2) gemv_w4_stream_kernel(const Ge
         for (int i = 0; i < STEPS; ++i) {
             if (on_row && i < steps) {
                 w[i] = ld_weights_16(wrow + (i * kSubwarp + l) * 4);
-                sb[i] = ld_scale_bits(srow + 2 * i + (l >> 2));
             } else {
                 w[i] = make_uint4(0, 0, 0, 0);
-                sb[i] = 0;
             }
         }
+        sp = load_scale_pair(srow, on_row ? steps : 0, l);
     };
 
     int blk = blockIdx.x;
-    if (blk < num_blocks) issue(w0, sb0, blk);
+    if (blk < num_blocks) issue(w0, sp0, blk);
     pdl_release_dependents();
     pdl_wait_prior_grids();
 
@@ -651,24 +671,26 @@ __global__ void __launch_bounds__(kMaxThreads, 2) gemv_w4_stream_kernel(const Ge
 
     uint4 xa[STEPS], xb[STEPS];
     int32_t seed[STEPS];
-    float xs[STEPS];
+    float xs[2];                     // scales of the groups whose weight scales this lane fetches
+#pragma unroll
+    for (int j = 0; j < 2; ++j) xs[j] = (l & 3) + 4 * j < steps ? s_scale[2 * ((l & 3) + 4 * j) + (l >> 2)] : 0.0f;
 #pragma unroll
     for (int i = 0; i < STEPS; ++i) {
         const int c = (i < steps ? i : 0) * kSubwarp + l;
         xa[i] = reinterpret_cast<const uint4*>(s_q8)[q8_slot(c, 0)];
         xb[i] = reinterpret_cast<const uint4*>(s_q8)[q8_slot(c, 1)];
         seed[i] = s_seed[c];
-        xs[i] = i < steps ? s_scale[c >> 2] : 0.0f;     // a zero factor switches an unused slot off
     }
 
     for (; blk < num_blocks; blk += gridDim.x) {
         const int nxt = blk + gridDim.x;
-        if (nxt < num_blocks) issue(w1, sb1, nxt);
+        if (nxt < num_blocks) issue(w1, sp1, nxt);
         float acc = 0.0f;
+        const float prod[2] = {__half2float(__ushort_as_half(sp0.bits[0])) * xs[0], __half2float(__ushort_as_half(sp0.bits[1])) * xs[1]};
 #pragma unroll
         for (int i = 0; i < STEPS; ++i) {
             const int32_t d = chunk_dot(w0[i], xa[i], xb[i], seed[i]);
-            acc = fmaf(static_cast<float>(d), __half2float(__ushort_as_half(sb0[i])) * xs[i], acc);
+            acc = fmaf(static_cast<float>(d), product_of_step(prod, i, l), acc);
         }
         acc += __shfl_xor_sync(0xFFFFFFFFu, acc, 4);
         acc += __shfl_xor_sync(0xFFFFFFFFu, acc, 2);
@@ -721,7 +743,8 @@ __global__ void __launch_bounds__(kMaxThreads, 2) gemv_w4_stream_kernel(const Ge
             }
         }
 #pragma unroll
-        for (int i = 0; i < STEPS; ++i) { w0[i] = w1[i]; sb0[i] = sb1[i]; }
+        for (int i = 0; i < STEPS; ++i) w0[i] = w1[i];
+        sp0 = sp1;
     }
     if constexpr (SIGNAL) {
         // "last block" pattern: the storing lanes fence, the CTA counts itself; the CTA that completes the count
@@ -802,8 +825,8 @@ __global__ void __launch_bounds__(kMaxThreads, 2) gemv_w4_stream_kernel(const Ge
 // activation read from shared memory (a lane's share of an 8192-element vector would not fit registers).
 // A row's chunks are accumulated in K order by the same lane as in gemv_w4_kernel without a K split, so the
 // two agree bit for bit.  PLAIN mode, 16-byte aligned weights.
-template <int XIN, bool FULL, int THREADS>     // FULL: K is a multiple of 2048, every slice has all 8 steps (no guards in the loops)
-__global__ void __launch_bounds__(THREADS, 2) gemv_w4_stream_longk_kernel(const GemvArgs a, const int num_blocks) {
+template <int XIN, bool FULL>     // FULL: K is a multiple of 2048, every slice has all 8 steps (no guards in the loops)
+__global__ void __launch_bounds__(kMaxThreads, 2) gemv_w4_stream_longk_kernel(const GemvArgs a, const int num_blocks) {
     constexpr int STEPS = 8;
     extern __shared__ __align__(16) uint8_t smem[];
     const int K = a.K;
@@ -819,41 +842,44 @@ __global__ void __launch_bounds__(THREADS, 2) gemv_w4_stream_longk_kernel(const 
     auto next_unit = [&](int& blk, int& sl) {
         if (++sl == nslices) { sl = 0; blk += gridDim.x; }
     };
-    auto issue = [&](uint4 (&w)[STEPS], uint16_t (&sb)[STEPS], int blk, int sl) {
-        const int row = min(blk * (THREADS / kSubwarp) + sub, N - 1);      // rows past the end re-read the last row; never stored
+    auto issue = [&](uint4 (&w)[STEPS], ScalePair& sp, int blk, int sl) {
+        const int row = min(blk * kMaxSubwarps + sub, N - 1);      // rows past the end re-read the last row; never stored
         const uint32_t* wp = a.qweight[0] + static_cast<size_t>(row) * words + (sl * STEPS * kSubwarp + l) * 4;
-        const __half* sp = a.scales[0] + static_cast<size_t>(row) * groups + 2 * sl * STEPS + (l >> 2);
 #pragma unroll
         for (int i = 0; i < STEPS; ++i) {
             if (FULL || sl * STEPS + i < steps) {
                 w[i] = ld_weights_16(wp + i * (kSubwarp * 4));
-                sb[i] = ld_scale_bits(sp + 2 * i);
             } else {
                 w[i] = make_uint4(0, 0, 0, 0);
-                sb[i] = 0;       // a zero scale switches an unused slot off
             }
         }
+        sp = load_scale_pair(a.scales[0] + static_cast<size_t>(row) * groups + 2 * sl * STEPS, min(STEPS, steps - sl * STEPS), l);
     };
     float acc = 0.0f;
     // one unit: 8 chunks of this lane against the staged activation; at a row's last slice reduce and store
-    auto consume = [&](const uint4 (&w)[STEPS], const uint16_t (&sb)[STEPS], int blk, int sl) {
+    auto consume = [&](const uint4 (&w)[STEPS], const ScalePair& sp, int blk, int sl) {
         const uint4* xq = reinterpret_cast<const uint4*>(s_q8) + q8_slot(sl * STEPS * kSubwarp + l, 0);   // chunk-interleaved
         const int32_t* xseed = s_seed + sl * STEPS * kSubwarp + l;
-        const float* xscale = s_scale + 2 * sl * STEPS + (l >> 2);
+        float prod[2];
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+            const int st = sl * STEPS + (l & 3) + 4 * j;
+            prod[j] = __half2float(__ushort_as_half(sp.bits[j])) * (FULL || st < steps ? s_scale[2 * st + (l >> 2)] : 0.0f);
+        }
 #pragma unroll
         for (int i = 0; i < STEPS; ++i) {
             if (FULL || sl * STEPS + i < steps) {
                 const uint4 xa = xq[16 * i];        // chunk + 8 i: the next block of eight chunks
                 const uint4 xb = xq[16 * i + 8];
                 const int32_t d = chunk_dot(w[i], xa, xb, xseed[i * kSubwarp]);
-                acc = fmaf(static_cast<float>(d), __half2float(__ushort_as_half(sb[i])) * xscale[2 * i], acc);
+                acc = fmaf(static_cast<float>(d), product_of_step(prod, i, l), acc);
             }
         }
         if (sl == nslices - 1) {
             acc += __shfl_xor_sync(0xFFFFFFFFu, acc, 4);
             acc += __shfl_xor_sync(0xFFFFFFFFu, acc, 2);
             acc += __shfl_xor_sync(0xFFFFFFFFu, acc, 1);
-            const int row = blk * (THREADS / kSubwarp) + sub;
+            const int row = blk * kMaxSubwarps + sub;
             if (l == 0 && row < N) {
                 float y = acc;
                 if (a.residual != nullptr) y += __half2float(a.residual[row]);
@@ -866,9 +892,9 @@ __global__ void __launch_bounds__(THREADS, 2) gemv_w4_stream_longk_kernel(const 
     };
 
     uint4 w0[STEPS], w1[STEPS];
-    uint16_t sb0[STEPS], sb1[STEPS];
+    ScalePair sp0 = {}, sp1 = {};
     int blk = blockIdx.x, sl = 0;
-    if (blk < num_blocks) issue(w0, sb0, blk, 0);
+    if (blk < num_blocks) issue(w0, sp0, blk, 0);
     pdl_release_dependents();
     pdl_wait_prior_grids();
     if constexpr (XIN == kXFp16Norm) {
@@ -883,13 +909,13 @@ __global__ void __launch_bounds__(THREADS, 2) gemv_w4_stream_longk_kernel(const 
     while (blk < num_blocks) {
         int nblk = blk, nsl = sl;
         next_unit(nblk, nsl);
-        if (nblk < num_blocks) issue(w1, sb1, nblk, nsl);
-        consume(w0, sb0, blk, sl);
+        if (nblk < num_blocks) issue(w1, sp1, nblk, nsl);
+        consume(w0, sp0, blk, sl);
         if (nblk >= num_blocks) break;
         blk = nblk; sl = nsl;
         next_unit(nblk, nsl);
-        if (nblk < num_blocks) issue(w0, sb0, nblk, nsl);
-        consume(w1, sb1, blk, sl);
+        if (nblk < num_blocks) issue(w0, sp0, nblk, nsl);
+        consume(w1, sp1, blk, sl);
         blk = nblk; sl = nsl;
     }
 }
@@ -1103,18 +1129,12 @@ int gemv_set_attributes() {
     if (e == cudaSuccess) e = raise_smem_mode<kSwiglu, 4>();
     if (e == cudaSuccess) e = raise_smem_mode<kSwiglu, 8>();
     if (e == cudaSuccess) e = raise_smem(gemv_group_dots_kernel);
-    if (e == cudaSuccess) e = raise_smem(gemv_w4_stream_longk_kernel<kXQ8, true, 256>);
-    if (e == cudaSuccess) e = raise_smem(gemv_w4_stream_longk_kernel<kXQ8, true, 288>);
-    if (e == cudaSuccess) e = raise_smem(gemv_w4_stream_longk_kernel<kXQ8, false, 256>);
-    if (e == cudaSuccess) e = raise_smem(gemv_w4_stream_longk_kernel<kXQ8, false, 288>);
-    if (e == cudaSuccess) e = raise_smem(gemv_w4_stream_longk_kernel<kXFp16, true, 256>);
-    if (e == cudaSuccess) e = raise_smem(gemv_w4_stream_longk_kernel<kXFp16, true, 288>);
-    if (e == cudaSuccess) e = raise_smem(gemv_w4_stream_longk_kernel<kXFp16, false, 256>);
-    if (e == cudaSuccess) e = raise_smem(gemv_w4_stream_longk_kernel<kXFp16, false, 288>);
-    if (e == cudaSuccess) e = raise_smem(gemv_w4_stream_longk_kernel<kXFp16Norm, true, 256>);
-    if (e == cudaSuccess) e = raise_smem(gemv_w4_stream_longk_kernel<kXFp16Norm, true, 288>);
-    if (e == cudaSuccess) e = raise_smem(gemv_w4_stream_longk_kernel<kXFp16Norm, false, 256>);
-    if (e == cudaSuccess) e = raise_smem(gemv_w4_stream_longk_kernel<kXFp16Norm, false, 288>);
+    if (e == cudaSuccess) e = raise_smem(gemv_w4_stream_longk_kernel<kXQ8, true>);
+    if (e == cudaSuccess) e = raise_smem(gemv_w4_stream_longk_kernel<kXQ8, false>);
+    if (e == cudaSuccess) e = raise_smem(gemv_w4_stream_longk_kernel<kXFp16, true>);
+    if (e == cudaSuccess) e = raise_smem(gemv_w4_stream_longk_kernel<kXFp16, false>);
+    if (e == cudaSuccess) e = raise_smem(gemv_w4_stream_longk_kernel<kXFp16Norm, true>);
+    if (e == cudaSuccess) e = raise_smem(gemv_w4_stream_longk_kernel<kXFp16Norm, false>);
     if (e == cudaSuccess) e = prepare_bulk_mode<kPlain>();
     if (e == cudaSuccess) e = prepare_bulk_mode<kQkv>();
     if (e == cudaSuccess) e = prepare_bulk_mode<kSwiglu>();
@@ -1192,20 +1212,13 @@ int gemv_launch(GemvMode mode, GemvArgs a, cudaStream_t stream) {
     if (mode == kPlain && !q8_epilogue && !sampling && !handoff && aligned16 && steps > 8 && a.x_f32 == nullptr &&
         static_cast<long long>(num_blocks) * ((steps + 7) / 8) >= 8LL * 2 * dev->sm_count &&
         staged_x_bytes(a.K) <= 160 * 1024 && option(W4A16_OPT_GEMV_FORM) != 2) {
-        // Nine warps per CTA where that saves a round: the CTAs walk in rounds of (2 x SMs) x 32 or 36 rows, and a round for a
-        // handful of rows costs the latency of all of a row's slices (28672 rows: 3.03 rounds of 32, 2.69 of 36).
-        const int ctas = 2 * dev->sm_count;
-        const bool nine = (a.units + ctas * 36 - 1) / (ctas * 36) < (a.units + ctas * 32 - 1) / (ctas * 32);
-        const int threads_l = nine ? 288 : 256, blocks_l = (a.units + threads_l / kSubwarp - 1) / (threads_l / kSubwarp);
-        const dim3 sgrid(std::min(blocks_l, ctas)), sblock(threads_l);
+        const dim3 sgrid(std::min(num_blocks, 2 * dev->sm_count)), sblock(kMaxThreads);
         const size_t ssmem = staged_x_bytes(a.K);
         const bool pdl = pdl_enabled();
-#define W4_LONGK2(XINV, F) (nine ? launch_kernel(gemv_w4_stream_longk_kernel<XINV, F, 288>, sgrid, sblock, ssmem, stream, pdl, a, blocks_l) \
-                                 : launch_kernel(gemv_w4_stream_longk_kernel<XINV, F, 256>, sgrid, sblock, ssmem, stream, pdl, a, blocks_l))
-#define W4_LONGK(XINV) (steps % 8 == 0 ? W4_LONGK2(XINV, true) : W4_LONGK2(XINV, false))
+#define W4_LONGK(XINV) (steps % 8 == 0 ? launch_kernel(gemv_w4_stream_longk_kernel<XINV, true>, sgrid, sblock, ssmem, stream, pdl, a, num_blocks) \
+                                       : launch_kernel(gemv_w4_stream_longk_kernel<XINV, false>, sgrid, sblock, ssmem, stream, pdl, a, num_blocks))
         if (a.x_fp16 != nullptr) e = a.gamma != nullptr ? W4_LONGK(kXFp16Norm) : W4_LONGK(kXFp16);
         else e = W4_LONGK(kXQ8);
-#undef W4_LONGK2
 #undef W4_LONGK
         return static_cast<int>(e);
     }

@@ -203,11 +203,11 @@ __device__ __forceinline__ void stage_x_from_fp16(const __half* __restrict__ g_x
 // RMSNorm fused in front of the quantiser, per CTA: y = fp16(fp16(x * inv_rms) * gamma) with
 // inv_rms = 1 / sqrt(mean(x^2) + eps) rounded to fp16 -- the arithmetic of the stand-alone
 // rmsnorm_q8_1 kernel (mean of squares in double), so both give the same Q8_1 arrays.
-// Needs blockDim.x to be a multiple of 32 and at most 512.
+// Needs blockDim.x to be a multiple of 32 and at most 256.
 __device__ __forceinline__ void stage_x_from_fp16_rmsnorm(const __half* __restrict__ g_x,
                                                           const __half* __restrict__ g_gamma, int K, float eps,
                                                           int8_t* s_q8, int32_t* s_seed, float* s_scale) {
-    __shared__ double s_red[16];
+    __shared__ double s_red[8];
     __shared__ float s_inv;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
     double ss = 0.0;

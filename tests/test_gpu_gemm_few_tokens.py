@@ -1,0 +1,58 @@
+"""The few-token kernel (2-16 tokens) at the edges of its cut: one CTA per row block and clusters, K of one step pair and of many,
+row groups that do not fill a CTA, scales on both sides of the limit of the short dequantisation; and the RMSNorm + Q8_1 launch
+at the ends of its register form."""
+import numpy as np
+import pytest
+
+import oracle
+from tests import util
+
+pytestmark = pytest.mark.gpu
+torch = pytest.importorskip("torch")
+
+
+@pytest.mark.parametrize("M,N,K,scale_max", [(2, 16, 256, 0.02), (3, 48, 8960, 0.5), (7, 1536, 8960, 0.02), (8, 2064, 1536, 0.07),
+                                             (9, 17920, 1536, 0.02), (13, 272, 4096, 0.5), (16, 1536, 8960, 0.02), (16, 30000, 512, 0.02)])
+def test_few_token_kernel_matches_oracle(M, N, K, scale_max):
+    import qwen_engine_b200 as ops
+    from qwen_engine_b200 import synth
+    seed = M * 31 + N + K
+    rng = np.random.default_rng(seed)
+    qw, x = synth.packed_weights(seed, "f", N, K), synth.activations(seed, "f", M, K)
+    sc = rng.uniform(0.002, scale_max, size=(N, K // 128)).astype(np.float16)
+    r = rng.standard_normal((M, N)).astype(np.float16)
+    y = torch.full((M * N + 64,), float("nan"), dtype=torch.float16, device="cuda")
+    y[:M * N] = util.to_dev(r).reshape(-1)
+    ops.launch_gemm_prefill_w4a16(util.to_dev(qw), util.to_dev(sc), util.to_dev(x), y, y, M, N, K)
+    torch.cuda.synchronize()
+    got = util.to_np(y)
+    assert np.isnan(got[M * N:]).all(), "wrote past the output"
+    n_idx = np.unique(np.concatenate([[0, N - 1], rng.choice(N, size=min(N, 48), replace=False)])).astype(np.int32)
+    m_idx = np.arange(M, dtype=np.int32)
+    ref64, _ = oracle.gemm_prefill(qw, sc, x, m_idx, n_idx, residual=r)
+    util.assert_fp16_close(got[:M * N].reshape(M, N)[:, n_idx], ref64, what=f"{M}x{N}x{K}",
+                           magnitude=ref64 - r[:, n_idx].astype(np.float64))
+    assert ops.debug_counter(0) == 0
+
+
+@pytest.mark.parametrize("hidden,offset", [(128, 0), (1536, 0), (1664, 0), (8192, 0), (8320, 0), (1536, 4)])
+def test_rmsnorm_q8_1_sizes(hidden, offset):
+    """offset: elements by which the input misses its 16-byte alignment (the shared-memory form takes it)."""
+    import qwen_engine_b200 as ops
+    from qwen_engine_b200 import synth
+    x = (synth.activations(hidden, "r", hidden).astype(np.float32) * 3).astype(np.float16)
+    g = (1 + 0.1 * synth.activations(hidden, "g", hidden).astype(np.float32)).astype(np.float16)
+    d_x = torch.empty(hidden + offset, dtype=torch.float16, device="cuda")[offset:]
+    d_x.copy_(util.to_dev(x))
+    q8 = torch.empty(hidden, dtype=torch.int8, device="cuda")
+    xs = torch.empty(hidden // 128, dtype=torch.float32, device="cuda")
+    s8 = torch.empty(hidden // 8, dtype=torch.int32, device="cuda")
+    y = torch.empty(hidden, dtype=torch.float16, device="cuda")
+    ops.launch_rmsnorm_q8_1(d_x, util.to_dev(g), y, q8, xs, s8, None, hidden)
+    torch.cuda.synchronize()
+    # the normed vector, then the quantiser the oracle has for it
+    inv = np.float16(np.float32(1) / np.sqrt(np.float32(np.mean(x.astype(np.float64) ** 2)) + np.float32(1e-6)))
+    want = ((x * inv).astype(np.float16) * g).astype(np.float16)
+    assert np.array_equal(util.to_np(y).view(np.uint16), want.view(np.uint16))
+    w8, ws, wsum = oracle.quantize_q8_1(want)
+    assert np.array_equal(util.to_np(q8), w8) and np.array_equal(util.to_np(xs), ws) and np.array_equal(util.to_np(s8), wsum)

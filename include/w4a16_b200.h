@@ -91,10 +91,11 @@ enum {
                                         Same output bits in every form. */
     W4A16_OPT_GEMM_MIN_TOKENS_TENSOR_CORE = 4, /* token count from which the M-token contraction runs on the
                                         tensor cores; 0 (default): the measured crossover (4 or 5 tokens) */
-    W4A16_OPT_GEMM_FORM = 5,         /* tensor-core form of the M-token contraction: 0 (default) chosen by token
-                                        count, 1 one CTA per tile, 2 CTA pairs (cta_group::2) */
+    W4A16_OPT_GEMM_FORM = 5,         /* tensor-core form of the M-token contraction: 0 (default) chosen by tokens and
+                                        shape, 1 weight streaming (one CTA per tile and K slice), 2 CTA pairs */
     W4A16_OPT_GEMM_MMA_MAX_TOKENS = 6, /* largest token count that takes the weight-streaming mma.sync kernel instead of
-                                        the tcgen05 kernels: 0 (default) the measured crossover, 1 never, n up to n */
+                                        the tcgen05 kernels: 0 (default) the measured crossover (16), 1 never, n up to
+                                        n (at most 16) */
     W4A16_OPT_COUNT_ = 7
 };
 W4A16_API int w4a16_set_option(int option, int value);

@@ -236,11 +236,12 @@ int gemm_tc_set_attributes() {
     raise_pair(gemm_w4a16_tc_stream_kernel<kPlain>);
     raise_pair(gemm_w4a16_tc_stream_kernel<kQkv>);
     raise_pair(gemm_w4a16_tc_stream_kernel<kSwiglu>);
-    raise_pair(gemm_w4a16_tc_pair_kernel<kPlain, true>);
-    raise_pair(gemm_w4a16_tc_pair_kernel<kPlain, false>);
-    raise_pair(gemm_w4a16_tc_pair_kernel<kQkv, true>);
-    raise_pair(gemm_w4a16_tc_pair_kernel<kQkv, false>);
-    raise_pair(gemm_w4a16_tc_pair_kernel<kSwiglu, true>);
+    raise_pair(gemm_w4a16_tc_pair_kernel<kPlain, kStoreValues>);
+    raise_pair(gemm_w4a16_tc_pair_kernel<kPlain, kStoreWords>);
+    raise_pair(gemm_w4a16_tc_pair_kernel<kPlain, kStoreWordsPeers>);
+    raise_pair(gemm_w4a16_tc_pair_kernel<kQkv, kStoreValues>);
+    raise_pair(gemm_w4a16_tc_pair_kernel<kQkv, kStoreWords>);
+    raise_pair(gemm_w4a16_tc_pair_kernel<kSwiglu, kStoreWords>);
     return static_cast<int>(e);
 }
 
@@ -349,9 +350,10 @@ int pair_launch(const GemmArgs& g, int sm_count, cudaStream_t stream) {
     const int T = pair_token_tile(g.M, n_pairs, g.K / kGroup, pairs, nullptr);
     a.halves = T > kPairAccCols ? 2 : 1;
     a.n_half = T / a.halves;
-    // Two rows of an output as one word: even strides and rows, 4-byte aligned; peers get value by value stores.
+    // Two rows of an output as one word: even strides and rows, 4-byte aligned.
     auto word = [](const void* p) { return reinterpret_cast<uintptr_t>(p) % 4 == 0; };
-    bool words = a.num_peers == 0 && word(a.residual);
+    bool words = word(a.residual);
+    for (int p = 0; p < a.num_peers; ++p) words = words && word(a.peer_out[p]);
     for (int t = 0; t < (g.mode == kQkv ? 3 : 1); ++t) words = words && a.out_ld[t] % 2 == 0 && a.rows[t] % 2 == 0 && word(a.out[t]);
     // weight matrices that do not stay in L2 next to the tokens and outputs: panels of 4 token tiles (measured on
     // 28672 x 8192 at 4096 tokens: 1.62 -> 1.56 ms, DRAM reads 1.77 -> under 1 GB); smaller ones: row tiles fastest
@@ -366,9 +368,11 @@ int pair_launch(const GemmArgs& g, int sm_count, cudaStream_t stream) {
         return static_cast<int>(launch_kernel_cluster(kernel, dim3(grid), dim3(kPairThreads), smem, stream, pdl_enabled(), dim3(2, 1, 1), a));
     };
     switch (g.mode) {
-        case kPlain: return words ? launch(gemm_w4a16_tc_pair_kernel<kPlain, true>) : launch(gemm_w4a16_tc_pair_kernel<kPlain, false>);
-        case kQkv: return words ? launch(gemm_w4a16_tc_pair_kernel<kQkv, true>) : launch(gemm_w4a16_tc_pair_kernel<kQkv, false>);
-        default: return launch(gemm_w4a16_tc_pair_kernel<kSwiglu, true>);
+        case kPlain:
+            if (!words) return launch(gemm_w4a16_tc_pair_kernel<kPlain, kStoreValues>);
+            return a.num_peers > 0 ? launch(gemm_w4a16_tc_pair_kernel<kPlain, kStoreWordsPeers>) : launch(gemm_w4a16_tc_pair_kernel<kPlain, kStoreWords>);
+        case kQkv: return words ? launch(gemm_w4a16_tc_pair_kernel<kQkv, kStoreWords>) : launch(gemm_w4a16_tc_pair_kernel<kQkv, kStoreValues>);
+        default: return launch(gemm_w4a16_tc_pair_kernel<kSwiglu, kStoreWords>);
     }
 }
 }  // namespace

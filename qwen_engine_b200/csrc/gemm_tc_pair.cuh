@@ -140,10 +140,12 @@ __device__ __forceinline__ void pair_exchange8(int odd, const uint32_t (&v)[8], 
     }
 }
 
-// WORDS: both rows of an output lie in one aligned word and nothing goes to peers (the host checks); the other form stores
-// value by value.
-template <int MODE, bool WORDS>
+// STORE (the host picks): kStoreWords where both rows of an output lie in one aligned word, kStoreWordsPeers the same with
+// copies to peer GPUs (a warp's store is two runs of 64 bytes, which travel as such), kStoreValues value by value.
+enum PairStore { kStoreValues = 0, kStoreWords = 1, kStoreWordsPeers = 2 };
+template <int MODE, int STORE>
 __global__ void __launch_bounds__(kPairThreads, 1) gemm_w4a16_tc_pair_kernel(const __grid_constant__ PairArgs a) {
+    constexpr bool WORDS = STORE != kStoreValues;
     constexpr int kEpi0 = kPairDqWarps, kMmaWarp = kEpi0 + kPairEpiWarps, kRawWarp = kMmaWarp + 1;
     extern __shared__ uint8_t smem_raw_base[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw_base) + 1023) & ~uintptr_t(1023));
@@ -346,7 +348,12 @@ __global__ void __launch_bounds__(kPairThreads, 1) gemm_w4a16_tc_pair_kernel(con
                             } else if constexpr (WORDS) {
                                 __half2 y = __floats2half2_rn(even_row, odd_row);
                                 if (add) y = __hadd2(y, res[q]);
-                                if (on) *reinterpret_cast<__half2*>(out) = y;
+                                if (on) {
+                                    *reinterpret_cast<__half2*>(out) = y;
+                                    if constexpr (STORE == kStoreWordsPeers) {
+                                        for (int p = 0; p < a.num_peers; ++p) *reinterpret_cast<__half2*>(a.peer_out[p] + (out - a.out[pt.t])) = y;
+                                    }
+                                }
                             } else if (on) {
                                 const size_t o = static_cast<size_t>(out - a.out[pt.t]);
                                 for (int k = 0; k < (ne + 1 < rows ? 2 : 1); ++k) {
@@ -498,12 +505,12 @@ size_t tc_pair_smem_bytes(int T) {
     return 1024 + static_cast<size_t>(kPairSlots) * T * 128 + static_cast<size_t>(kPairRawSlots) * kPairRawBytes +
            (2 * kPairRawSlots + 2 * kPairSlots + 4) * 8 + 16;
 }
-// Estimated cycles of a launch with token tiles of T, from measurements on B200: a step takes 4 T of MMA or 950 of
+// Estimated cycles of a launch with token tiles of T, from measurements on B200: a step takes 4 T of MMA or 1100 of
 // dequantisation, whichever is more; a tile of two accumulators waits 2500 for the second one to be drained; the first fill,
 // the exchange at the start and the last tile's epilogue are not overlapped.
 double pair_cost(int M, int n_pairs, int steps, int pairs, int T) {
     const int tiles = n_pairs * ((M + T - 1) / T), rounds = (tiles + pairs - 1) / pairs;
-    return rounds * (steps * std::max(4.0 * T, 950.0) + (T > kPairAccCols ? 2500.0 : 0.0)) + 6000.0 + 25.0 * T;
+    return rounds * (steps * std::max(4.0 * T, 1100.0) + (T > kPairAccCols ? 2500.0 : 0.0)) + 9000.0 + 25.0 * T;
 }
 // The token tile for `n_pairs` pairs of row tiles on `pairs` pairs of SMs: one accumulator of 16..128 or two of 80..128.
 int pair_token_tile(int M, int n_pairs, int steps, int pairs, double* estimate) {

@@ -46,10 +46,11 @@ def test_pair_kernel_matches_oracle(pairs, M, N, K, scale_max, res):
     util.assert_fp16_close(got[:M * N].reshape(M, N)[np.ix_(m_idx, n_idx)], ref64, what=f"{M}x{N}x{K}", magnitude=acc)
 
 
-def test_pair_kernel_block_with_peer_copies(pairs):
+@pytest.mark.parametrize("col", [130, 131])      # word-aligned and not
+def test_pair_kernel_block_with_peer_copies(pairs, col):
     """A column block of a wider matrix, also stored into matrices standing in for peer GPUs' memory."""
     from qwen_engine_b200 import synth
-    M, N, K, ldc, col = 290, 384, 512, 1024, 130
+    M, N, K, ldc = 290, 384, 512, 1024
     qw, sc, x = synth.packed_weights(5, "b", N, K), synth.scales(5, "b", N, K), synth.activations(5, "b", M, K)
     d = [util.to_dev(v) for v in (qw, sc, x)]
     want = torch.empty((M, N), dtype=torch.float16, device="cuda")

@@ -85,7 +85,8 @@ enum {
                                         sweep on another CTA's counter or tagged word, before giving up and reporting
                                         it (*d_status, w4a16_sweep_status); default 1 << 22, about a second */
     W4A16_OPT_GEMV_FORM = 3,         /* how the batch-1 GEMV brings its weights on chip: 0 (default) the measured
-                                        best, which is 1; 1 register-held 16-byte streaming loads issued before the
+                                        best for the size: 1, or a persistent grid that streams tall matrices;
+                                        1 register-held 16-byte streaming loads issued before the
                                         wait for the previous kernel, 2 bulk copies (cp.async.bulk) into shared
                                         memory (K slices of long plain projections on the CTAs of a cluster).
                                         Same output bits in every form. */

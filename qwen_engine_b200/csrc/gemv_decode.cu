@@ -594,7 +594,7 @@ __device__ __forceinline__ float product_of_step(const float (&p)[2], int i, int
     return __shfl_sync(0xFFFFFFFFu, p[i >> 2], (l & 4) | (i & 3), kSubwarp);
 }
 
-// Streaming form for very tall matrices (lm_head): a persistent grid, each CTA walks row blocks of 32 with
+// Streaming form for tall matrices (lm_head, see gemv_launch for the sizes): a persistent grid, each CTA walks row blocks of 32 with
 // the weights of the NEXT block already in flight while the current one is reduced, and the lane's share
 // of the quantised activation lives in registers for the whole launch (a lane always meets the same
 // 16-byte chunks l, l+8, ... of every row).  PLAIN mode, 16-byte aligned weights, K <= 256 * STEPS.
@@ -1002,6 +1002,9 @@ Plan make_plan(GemvMode mode, int units, int K, int sm_count) {
     };
     int upc = upc_for((sm_count * 5) / 4);
     if (depth_for(upc) > 8) upc = upc_for((sm_count * 13 + 9) / 10);
+    // Long K and rows for more than one full CTA per SM: no K split.  (A split makes twice as many CTAs, which no longer fit
+    // the chip at once: 6144 x 4096 took 5.4 us, 7168 x 4096, which was never split, 5.0.)
+    if (mode == kPlain && steps > 8 && units > kMaxSubwarps * sm_count) upc = kMaxSubwarps;
     int cap = std::max(1, kMaxSubwarps / upc);   // most K slices the CTA can hold
     cap = std::min(cap, steps);
     int per = (steps + cap - 1) / cap;           // steps per slice if all slices were used
@@ -1195,12 +1198,26 @@ int gemv_launch(GemvMode mode, GemvArgs a, cudaStream_t stream) {
     const int block = (threads + 31) / 32 * 32;
 
     cudaError_t e;
-    // very tall PLAIN matrices: persistent streaming kernel (two CTAs per SM, >= 8 row blocks each)
     const int steps = a.K / kStepElems;
     const int weight_rows = mode == kSwiglu ? 2 * a.units : a.units;
     const int num_blocks = (weight_rows + kMaxSubwarps - 1) / kMaxSubwarps;
-    constexpr int kStreamMinBlocksPerSm = 16;   // row blocks per SM from which the persistent streaming form pays
-    const bool tall = num_blocks >= kStreamMinBlocksPerSm * dev->sm_count;
+    // Which sizes the persistent streaming kernels take (two CTAs per SM, blocks of 32 rows; times chained in a graph with
+    // Q8_1 input and weights not in L2, register form -> streaming form).  Only where the register form would not split K
+    // either: the two then add in the same order and every entry point and form gives the same bits.
+    // - K > 2048, plain: from more than one block per SM on.  5120 x 4096 5.1 -> 3.8 us, 8192 x 4096 5.2 -> 4.1,
+    //   16384 x 4096 9.3 -> 7.0, 28672 x 4096 15.4 -> 11.3; 4096 x 4096 would go from 3.1 to 3.4.
+    // - K <= 2048: where the register form would need a second wave (16384 x 2048 5.2 -> 4.7, 28672 x 1536 7.8 -> 5.2), for
+    //   a gate_up with K > 1024 only from a quarter of a second wave on.
+    // - few steps and at most one block per CTA: one round trip for everything (8192 x 1024 2.15 -> 2.0, from an fp16
+    //   activation 2.6 -> 2.2).  An fp16 activation costs more to quantise with fewer threads resident, so its line lies at
+    //   K = 1024 (8192 x 1536 2.85 -> 3.05); an input whose maximum was handed on saves that pass in the register form only.
+    // Between one and two blocks per CTA a single wave of the register form wins (12288 x 1024 would go from 2.4 to 2.8).
+    const int form = option(W4A16_OPT_GEMV_FORM);
+    const int resident = resident_warps_per_sm(mode, p.U) / ((threads + 31) / 32) * dev->sm_count;
+    const bool handed_in = a.amax_in != nullptr || a.sumsq_in != nullptr;
+    const bool second_wave = mode == kSwiglu && steps > 4 ? 4 * grid > 5 * resident : grid > resident;
+    const bool one_block = num_blocks <= 2 * dev->sm_count && !handed_in && (a.x_fp16 != nullptr ? steps <= 4 : steps >= 3 && steps <= 6);
+    const bool by_size = form == 0 && a.ksplit == 1 && (steps > 8 ? num_blocks > dev->sm_count : one_block || second_wave);
     const bool sampling = a.sample_val != nullptr || a.sample_idx != nullptr;
     // signalled row-split output (no sampling): step word + flags given, the streaming kernel whatever the height
     const bool signalled = !sampling && a.sample_step_word != nullptr;
@@ -1210,8 +1227,7 @@ int gemv_launch(GemvMode mode, GemvArgs a, cudaStream_t stream) {
     if (sampling && (mode != kPlain || !a.sample_val || !a.sample_idx || !aligned16 || steps > 8)) return W4A16_ERR_SHAPE;
     // tall plain matrices with a long K: the streaming form that takes K in slices of 2048
     if (mode == kPlain && !q8_epilogue && !sampling && !handoff && aligned16 && steps > 8 && a.x_f32 == nullptr &&
-        static_cast<long long>(num_blocks) * ((steps + 7) / 8) >= 8LL * 2 * dev->sm_count &&
-        staged_x_bytes(a.K) <= 160 * 1024 && option(W4A16_OPT_GEMV_FORM) != 2) {
+        by_size && staged_x_bytes(a.K) <= 160 * 1024) {
         const dim3 sgrid(std::min(num_blocks, 2 * dev->sm_count)), sblock(kMaxThreads);
         const size_t ssmem = staged_x_bytes(a.K);
         const bool pdl = pdl_enabled();
@@ -1223,7 +1239,7 @@ int gemv_launch(GemvMode mode, GemvArgs a, cudaStream_t stream) {
         return static_cast<int>(e);
     }
     if (!q8_epilogue && !handoff && aligned16 && steps <= 8 && a.x_f32 == nullptr &&
-        ((mode == kPlain && (tall || sampling || signalled)) || (mode == kSwiglu && tall))) {
+        ((mode == kPlain && (by_size || sampling || signalled)) || (mode == kSwiglu && by_size))) {
         const dim3 sgrid(std::min(num_blocks, 2 * dev->sm_count)), sblock(kMaxThreads);
         const size_t ssmem = staged_x_bytes(a.K);
         const bool pdl = pdl_enabled();
@@ -1246,7 +1262,6 @@ int gemv_launch(GemvMode mode, GemvArgs a, cudaStream_t stream) {
     // down projection over a cluster costs more in cluster scheduling than the smaller activation staging saves.
     // The bulk-copy form therefore runs only on request (W4A16_OPT_GEMV_FORM = 2); it splits K over a cluster
     // where one CTA would otherwise stage or quantise more than 16 groups.
-    const int form = option(W4A16_OPT_GEMV_FORM);
     if (form == 2 && aligned16 && !q8_epilogue && !handoff) {
         const bool cluster_k = mode == kPlain && a.gamma == nullptr && a.x_f32 == nullptr && a.ksplit >= 2 &&
                                a.ksplit <= 8 && a.K / kGroup > 16;

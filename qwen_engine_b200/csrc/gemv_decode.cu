@@ -44,6 +44,9 @@ __host__ __device__ inline size_t amax_stage_offset(int K, int part_floats) {
 }
 __host__ __device__ inline size_t amax_stage_bytes(int K) { return (static_cast<size_t>(K / kGroup) * 4 + 15) / 16 * 16 + static_cast<size_t>(K) * 2; }
 
+// 200 KB for the staged activation and the partial sums, and always room for some raw groups behind them
+constexpr size_t kMaxStagedSmem = 200 * 1024, kMaxDynamicSmem = 220 * 1024;
+
 // Register caps.  What matters in a chain of dependent launches is that the CTAs of the NEXT launch become
 // resident, and issue their weight loads, while this one still runs: 88 registers for the single-row forms with
 // 8 loads per lane (down: three 192-thread CTAs per SM leave room for CTAs of the next QKV launch; measured
@@ -143,7 +146,7 @@ __global__ void __maxnreg__(gemv_reg_cap(MODE, U)) gemv_w4_kernel(const GemvArgs
         for (int i = tid; i < a.clear_count; i += blockDim.x) a.clear_words[i] = 0u;
     if constexpr (XIN == kXFp16Norm) {
         if (regs_form) stage_x_fp16_regs<true>(a.x_fp16, gam, K, kRmsEps, s_q8, s_seed, s_scale, a.sumsq_in);
-        else stage_x_from_fp16_rmsnorm(a.x_fp16, a.gamma, K, kRmsEps, s_q8, s_seed, s_scale);
+        else stage_x_fp16_raw<true>(a.x_fp16, a.gamma, K, kRmsEps, s_q8, s_seed, s_scale, smem + a.raw_at, a.raw_groups);
     } else if constexpr (XIN == kXFp16Amax) {
         uint8_t* extra = smem + amax_stage_offset(K, a.ksplit * a.units_per_cta * R);
         float* s_inv = reinterpret_cast<float*>(extra);
@@ -151,7 +154,7 @@ __global__ void __maxnreg__(gemv_reg_cap(MODE, U)) gemv_w4_kernel(const GemvArgs
         stage_x_fp16_amax(a.x_fp16, a.amax_in, K, s_q8, s_seed, s_scale, s_raw, s_inv);
     } else if constexpr (XIN == kXFp16) {
         if (regs_form) stage_x_fp16_regs<false>(a.x_fp16, gam, K, kRmsEps, s_q8, s_seed, s_scale);
-        else stage_x_from_fp16(a.x_fp16, K, s_q8, s_seed, s_scale);
+        else stage_x_fp16_raw<false>(a.x_fp16, nullptr, K, kRmsEps, s_q8, s_seed, s_scale, smem + a.raw_at, a.raw_groups);
     } else if constexpr (XIN == kXF32Heads) {
         stage_x_from_f32_heads(a.x_f32, K, s_q8, s_seed, s_scale);
     } else {
@@ -661,9 +664,11 @@ __global__ void __launch_bounds__(kMaxThreads, 2) gemv_w4_stream_kernel(const Ge
         }
     }
     if constexpr (XIN == kXFp16Norm) {
-        stage_x_from_fp16_rmsnorm(a.x_fp16, a.gamma, K, kRmsEps, s_q8, s_seed, s_scale);
+        if constexpr (STEPS <= 4) stage_x_from_fp16_rmsnorm(a.x_fp16, a.gamma, K, kRmsEps, s_q8, s_seed, s_scale);
+        else stage_x_fp16_raw<true>(a.x_fp16, a.gamma, K, kRmsEps, s_q8, s_seed, s_scale, smem + a.raw_at, a.raw_groups);
     } else if constexpr (XIN == kXFp16) {
-        stage_x_from_fp16(a.x_fp16, K, s_q8, s_seed, s_scale);
+        if constexpr (STEPS <= 4) stage_x_from_fp16(a.x_fp16, K, s_q8, s_seed, s_scale);
+        else stage_x_fp16_raw<false>(a.x_fp16, nullptr, K, kRmsEps, s_q8, s_seed, s_scale, smem + a.raw_at, a.raw_groups);
     } else if (!stage_x_from_q8_1_regs<STEPS == 8>(a.q8, a.xscale, a.sum8, K, a.vec_ok != 0, s_q8, s_seed, s_scale)) {
         stage_x_from_q8_1(a.q8, a.xscale, a.sum8, K, a.vec_ok != 0, s_q8, s_seed, s_scale);
     }
@@ -898,9 +903,9 @@ __global__ void __launch_bounds__(kMaxThreads, 2) gemv_w4_stream_longk_kernel(co
     pdl_release_dependents();
     pdl_wait_prior_grids();
     if constexpr (XIN == kXFp16Norm) {
-        stage_x_from_fp16_rmsnorm(a.x_fp16, a.gamma, K, kRmsEps, s_q8, s_seed, s_scale);
+        stage_x_fp16_raw<true>(a.x_fp16, a.gamma, K, kRmsEps, s_q8, s_seed, s_scale, smem + a.raw_at, a.raw_groups);
     } else if constexpr (XIN == kXFp16) {
-        stage_x_from_fp16(a.x_fp16, K, s_q8, s_seed, s_scale);
+        stage_x_fp16_raw<false>(a.x_fp16, nullptr, K, kRmsEps, s_q8, s_seed, s_scale, smem + a.raw_at, a.raw_groups);
     } else if (!stage_x_from_q8_1_regs<true>(a.q8, a.xscale, a.sum8, K, a.vec_ok != 0, s_q8, s_seed, s_scale)) {
         stage_x_from_q8_1(a.q8, a.xscale, a.sum8, K, a.vec_ok != 0, s_q8, s_seed, s_scale);
     }
@@ -1103,7 +1108,7 @@ cudaError_t launch_bulk(const GemvArgs& a, bool cluster_k, dim3 grid, dim3 block
 
 template <typename F>
 cudaError_t raise_smem(F* f) {
-    return cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+    return cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxDynamicSmem);
 }
 template <int MODE, int U>
 cudaError_t raise_smem_mode() {
@@ -1192,10 +1197,17 @@ int gemv_launch(GemvMode mode, GemvArgs a, cudaStream_t stream) {
     const int R = (mode == kSwiglu) ? 2 : 1;
     const int threads = a.units_per_cta * a.ksplit * kSubwarp;
     const int grid = (a.units + a.units_per_cta - 1) / a.units_per_cta;
-    const size_t smem = staged_x_bytes(a.K) + static_cast<size_t>(a.ksplit) * a.units_per_cta * R * sizeof(float);
-    if (smem > 200 * 1024) return W4A16_ERR_TOO_LARGE;
+    size_t smem = staged_x_bytes(a.K) + static_cast<size_t>(a.ksplit) * a.units_per_cta * R * sizeof(float);
+    if (smem > kMaxStagedSmem) return W4A16_ERR_TOO_LARGE;
     // fp16 staging quantises with whole warps
     const int block = (threads + 31) / 32 * 32;
+    // room for the raw groups behind `used` bytes: the whole vector up to 128 groups, which leaves two CTAs on an SM
+    auto add_raw = [&a](size_t used) {
+        const size_t per_group = kGroup * sizeof(__half) * (a.gamma != nullptr ? 2 : 1);
+        a.raw_at = static_cast<int>((used + 15) / 16 * 16);
+        a.raw_groups = static_cast<int>(std::min<size_t>({static_cast<size_t>(a.K / kGroup), 128, (kMaxDynamicSmem - a.raw_at) / per_group}));
+        return a.raw_at + a.raw_groups * per_group;
+    };
 
     cudaError_t e;
     const int steps = a.K / kStepElems;
@@ -1229,7 +1241,7 @@ int gemv_launch(GemvMode mode, GemvArgs a, cudaStream_t stream) {
     if (mode == kPlain && !q8_epilogue && !sampling && !handoff && aligned16 && steps > 8 && a.x_f32 == nullptr &&
         by_size && staged_x_bytes(a.K) <= 160 * 1024) {
         const dim3 sgrid(std::min(num_blocks, 2 * dev->sm_count)), sblock(kMaxThreads);
-        const size_t ssmem = staged_x_bytes(a.K);
+        const size_t ssmem = a.x_fp16 != nullptr ? add_raw(staged_x_bytes(a.K)) : staged_x_bytes(a.K);
         const bool pdl = pdl_enabled();
 #define W4_LONGK(XINV) (steps % 8 == 0 ? launch_kernel(gemv_w4_stream_longk_kernel<XINV, true>, sgrid, sblock, ssmem, stream, pdl, a, num_blocks) \
                                        : launch_kernel(gemv_w4_stream_longk_kernel<XINV, false>, sgrid, sblock, ssmem, stream, pdl, a, num_blocks))
@@ -1241,7 +1253,7 @@ int gemv_launch(GemvMode mode, GemvArgs a, cudaStream_t stream) {
     if (!q8_epilogue && !handoff && aligned16 && steps <= 8 && a.x_f32 == nullptr &&
         ((mode == kPlain && (by_size || sampling || signalled)) || (mode == kSwiglu && by_size))) {
         const dim3 sgrid(std::min(num_blocks, 2 * dev->sm_count)), sblock(kMaxThreads);
-        const size_t ssmem = staged_x_bytes(a.K);
+        const size_t ssmem = a.x_fp16 != nullptr && steps > 4 ? add_raw(staged_x_bytes(a.K)) : staged_x_bytes(a.K);
         const bool pdl = pdl_enabled();
 #define W4_STREAM3(XINV, SW, SA)                                                                                                \
     (steps <= 4 ? launch_kernel(gemv_w4_stream_kernel<XINV, 4, SW, SA>, sgrid, sblock, ssmem, stream, pdl, a, num_blocks)     \
@@ -1290,6 +1302,9 @@ int gemv_launch(GemvMode mode, GemvArgs a, cudaStream_t stream) {
             return static_cast<int>(e);
         }
     }
+    const bool one_round = a.K / kGroup <= kStageRounds * (block / 16);   // a group per half-warp: straight into registers
+    const bool unaligned = ((reinterpret_cast<uintptr_t>(a.x_fp16) | reinterpret_cast<uintptr_t>(a.gamma)) & 15u) != 0;
+    if (a.x_fp16 != nullptr && (!one_round || unaligned)) smem = add_raw(smem);
     switch (mode) {
         case kPlain: e = launch_mode<kPlain>(a, p.U, aligned16, dim3(grid), dim3(block), smem, stream); break;
         case kQkv: e = launch_mode<kQkv>(a, p.U, aligned16, dim3(grid), dim3(block), smem, stream); break;

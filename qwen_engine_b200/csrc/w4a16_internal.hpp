@@ -161,6 +161,9 @@ struct GemvArgs {
     const uint32_t* amax_in;
     double* sumsq_out;
     const double* sumsq_in;
+    // set by the launch: where in shared memory the staging of an fp16 activation keeps the raw groups it fetches, and
+    // how many of them it holds at once
+    int raw_at, raw_groups;
     uint32_t* clear_words;
     int clear_count;
     int K;

@@ -74,3 +74,29 @@ def test_gate_up_bits_do_not_depend_on_the_form(inter, K):
         ops.set_option(ops.OPT_GEMV_FORM, ops.GEMV_FORM_AUTO)
     assert torch.equal(outs[0].view(torch.int16), outs[1].view(torch.int16))
     assert torch.isfinite(outs[1][:inter]).all() and torch.isnan(outs[1][inter:]).all()
+
+
+@pytest.mark.parametrize("K", [256, 1024, 1280, 2048, 2304, 4352, 16384, 16640, 33024])
+@pytest.mark.parametrize("offset", [0, 4])
+def test_fp16_staging_equals_the_stand_alone_quantisers(K, offset):
+    """One and several rounds of groups, one and several turns of the raw buffer, x on an 8-byte boundary only."""
+    import qwen_engine_b200 as ops
+    from qwen_engine_b200 import synth
+    ops.init()
+    N = 40
+    qw, sc = util.to_dev(synth.packed_weights(7, "t", N, K)), util.to_dev(synth.scales(7, "t", N, K))
+    rng = np.random.Generator(np.random.Philox(key=K + offset))
+    x = util.to_dev(rng.standard_normal(K + offset).astype(np.float16))[offset:]
+    gamma = util.to_dev((rng.random(K) * 0.02 + 0.04).astype(np.float16))
+    act = (torch.empty(K, dtype=torch.int8, device="cuda"), torch.empty(K // 128, dtype=torch.float32, device="cuda"),
+           torch.empty(K // 8, dtype=torch.int32, device="cuda"))
+    y = torch.empty((4, N), dtype=torch.float16, device="cuda")
+    ops.launch_gemv_w4a16(qw, sc, x, None, y[0], N, K)
+    ops.launch_quantize_fp16_to_q8_1(x, *act, K)
+    ops.launch_gemv_w4a8(qw, sc, *act, None, y[1], N, K)
+    ops.launch_gemv_rmsnorm_w4a16(qw, sc, x, gamma, None, y[2], N, K)
+    ops.launch_rmsnorm_q8_1(x, gamma, None, *act, hidden_size=K)
+    ops.launch_gemv_w4a8(qw, sc, *act, None, y[3], N, K)
+    torch.cuda.synchronize()
+    assert torch.equal(y[0].view(torch.int16), y[1].view(torch.int16))
+    assert torch.equal(y[2].view(torch.int16), y[3].view(torch.int16))

@@ -669,6 +669,8 @@ __global__ void __launch_bounds__(kMaxThreads, 2) gemv_w4_stream_kernel(const Ge
     } else if constexpr (XIN == kXFp16) {
         if constexpr (STEPS <= 4) stage_x_from_fp16(a.x_fp16, K, s_q8, s_seed, s_scale);
         else stage_x_fp16_raw<false>(a.x_fp16, nullptr, K, kRmsEps, s_q8, s_seed, s_scale, smem + a.raw_at, a.raw_groups);
+    } else if constexpr (XIN == kXF32Heads) {
+        stage_x_from_f32_heads(a.x_f32, K, s_q8, s_seed, s_scale);
     } else if (!stage_x_from_q8_1_regs<STEPS == 8>(a.q8, a.xscale, a.sum8, K, a.vec_ok != 0, s_q8, s_seed, s_scale)) {
         stage_x_from_q8_1(a.q8, a.xscale, a.sum8, K, a.vec_ok != 0, s_q8, s_seed, s_scale);
     }
@@ -906,6 +908,8 @@ __global__ void __launch_bounds__(kMaxThreads, 2) gemv_w4_stream_longk_kernel(co
         stage_x_fp16_raw<true>(a.x_fp16, a.gamma, K, kRmsEps, s_q8, s_seed, s_scale, smem + a.raw_at, a.raw_groups);
     } else if constexpr (XIN == kXFp16) {
         stage_x_fp16_raw<false>(a.x_fp16, nullptr, K, kRmsEps, s_q8, s_seed, s_scale, smem + a.raw_at, a.raw_groups);
+    } else if constexpr (XIN == kXF32Heads) {
+        stage_x_from_f32_heads(a.x_f32, K, s_q8, s_seed, s_scale);
     } else if (!stage_x_from_q8_1_regs<true>(a.q8, a.xscale, a.sum8, K, a.vec_ok != 0, s_q8, s_seed, s_scale)) {
         stage_x_from_q8_1(a.q8, a.xscale, a.sum8, K, a.vec_ok != 0, s_q8, s_seed, s_scale);
     }
@@ -1143,6 +1147,8 @@ int gemv_set_attributes() {
     if (e == cudaSuccess) e = raise_smem(gemv_w4_stream_longk_kernel<kXFp16, false>);
     if (e == cudaSuccess) e = raise_smem(gemv_w4_stream_longk_kernel<kXFp16Norm, true>);
     if (e == cudaSuccess) e = raise_smem(gemv_w4_stream_longk_kernel<kXFp16Norm, false>);
+    if (e == cudaSuccess) e = raise_smem(gemv_w4_stream_longk_kernel<kXF32Heads, true>);
+    if (e == cudaSuccess) e = raise_smem(gemv_w4_stream_longk_kernel<kXF32Heads, false>);
     if (e == cudaSuccess) e = prepare_bulk_mode<kPlain>();
     if (e == cudaSuccess) e = prepare_bulk_mode<kQkv>();
     if (e == cudaSuccess) e = prepare_bulk_mode<kSwiglu>();
@@ -1223,12 +1229,15 @@ int gemv_launch(GemvMode mode, GemvArgs a, cudaStream_t stream) {
     // - few steps and at most one block per CTA: one round trip for everything (8192 x 1024 2.15 -> 2.0, from an fp16
     //   activation 2.6 -> 2.2).  An fp16 activation costs more to quantise with fewer threads resident, so its line lies at
     //   K = 1024 (8192 x 1536 2.85 -> 3.05); an input whose maximum was handed on saves that pass in the register form only.
+    // fp32 heads: 28672 x 2304 19.1 -> 10.8, 28672 x 1536 12.9 -> 6.5, 6144 x 8960 13.1 -> 11.1; a division per value makes
+    // their staging too dear for the one-block line.
     // Between one and two blocks per CTA a single wave of the register form wins (12288 x 1024 would go from 2.4 to 2.8).
     const int form = option(W4A16_OPT_GEMV_FORM);
     const int resident = resident_warps_per_sm(mode, p.U) / ((threads + 31) / 32) * dev->sm_count;
     const bool handed_in = a.amax_in != nullptr || a.sumsq_in != nullptr;
     const bool second_wave = mode == kSwiglu && steps > 4 ? 4 * grid > 5 * resident : grid > resident;
-    const bool one_block = num_blocks <= 2 * dev->sm_count && !handed_in && (a.x_fp16 != nullptr ? steps <= 4 : steps >= 3 && steps <= 6);
+    const bool one_block = num_blocks <= 2 * dev->sm_count && !handed_in && a.x_f32 == nullptr &&
+                           (a.x_fp16 != nullptr ? steps <= 4 : steps >= 3 && steps <= 6);
     const bool by_size = form == 0 && a.ksplit == 1 && (steps > 8 ? num_blocks > dev->sm_count : one_block || second_wave);
     const bool sampling = a.sample_val != nullptr || a.sample_idx != nullptr;
     // signalled row-split output (no sampling): step word + flags given, the streaming kernel whatever the height
@@ -1238,7 +1247,7 @@ int gemv_launch(GemvMode mode, GemvArgs a, cudaStream_t stream) {
         return W4A16_ERR_SHAPE;
     if (sampling && (mode != kPlain || !a.sample_val || !a.sample_idx || !aligned16 || steps > 8)) return W4A16_ERR_SHAPE;
     // tall plain matrices with a long K: the streaming form that takes K in slices of 2048
-    if (mode == kPlain && !q8_epilogue && !sampling && !handoff && aligned16 && steps > 8 && a.x_f32 == nullptr &&
+    if (mode == kPlain && !q8_epilogue && !sampling && !handoff && aligned16 && steps > 8 &&
         by_size && staged_x_bytes(a.K) <= 160 * 1024) {
         const dim3 sgrid(std::min(num_blocks, 2 * dev->sm_count)), sblock(kMaxThreads);
         const size_t ssmem = a.x_fp16 != nullptr ? add_raw(staged_x_bytes(a.K)) : staged_x_bytes(a.K);
@@ -1246,11 +1255,12 @@ int gemv_launch(GemvMode mode, GemvArgs a, cudaStream_t stream) {
 #define W4_LONGK(XINV) (steps % 8 == 0 ? launch_kernel(gemv_w4_stream_longk_kernel<XINV, true>, sgrid, sblock, ssmem, stream, pdl, a, num_blocks) \
                                        : launch_kernel(gemv_w4_stream_longk_kernel<XINV, false>, sgrid, sblock, ssmem, stream, pdl, a, num_blocks))
         if (a.x_fp16 != nullptr) e = a.gamma != nullptr ? W4_LONGK(kXFp16Norm) : W4_LONGK(kXFp16);
+        else if (a.x_f32 != nullptr) e = W4_LONGK(kXF32Heads);
         else e = W4_LONGK(kXQ8);
 #undef W4_LONGK
         return static_cast<int>(e);
     }
-    if (!q8_epilogue && !handoff && aligned16 && steps <= 8 && a.x_f32 == nullptr &&
+    if (!q8_epilogue && !handoff && aligned16 && steps <= 8 &&
         ((mode == kPlain && (by_size || sampling || signalled)) || (mode == kSwiglu && by_size))) {
         const dim3 sgrid(std::min(num_blocks, 2 * dev->sm_count)), sblock(kMaxThreads);
         const size_t ssmem = a.x_fp16 != nullptr && steps > 4 ? add_raw(staged_x_bytes(a.K)) : staged_x_bytes(a.K);
@@ -1260,7 +1270,8 @@ int gemv_launch(GemvMode mode, GemvArgs a, cudaStream_t stream) {
      : steps <= 6 ? launch_kernel(gemv_w4_stream_kernel<XINV, 6, SW, SA>, sgrid, sblock, ssmem, stream, pdl, a, num_blocks)  \
                   : launch_kernel(gemv_w4_stream_kernel<XINV, 8, SW, SA>, sgrid, sblock, ssmem, stream, pdl, a, num_blocks))
 #define W4_STREAM(XINV) (mode == kSwiglu ? W4_STREAM3(XINV, true, 0) : sampling ? W4_STREAM3(XINV, false, 1) : signalled ? W4_STREAM3(XINV, false, 2) : W4_STREAM3(XINV, false, 0))
-        if (a.x_fp16 != nullptr) e = a.gamma != nullptr ? W4_STREAM(kXFp16Norm) : W4_STREAM(kXFp16);
+        if (a.x_f32 != nullptr) e = W4_STREAM3(kXF32Heads, false, 0);   // plain rows only
+        else if (a.x_fp16 != nullptr) e = a.gamma != nullptr ? W4_STREAM(kXFp16Norm) : W4_STREAM(kXFp16);
         else e = W4_STREAM(kXQ8);
 #undef W4_STREAM
 #undef W4_STREAM3

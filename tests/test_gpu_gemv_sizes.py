@@ -33,11 +33,14 @@ def test_plain_projection_bits_do_not_depend_on_the_form(N, K):
            torch.empty(K // 8, dtype=torch.int32, device="cuda"))
     ops.launch_quantize_fp16_to_q8_1(x, *act, K)
 
+    heads = x.float() * 1.1
+
     def outputs():
-        y = torch.full((3, N + 16), float("nan"), dtype=torch.float16, device="cuda")
+        y = torch.full((4, N + 16), float("nan"), dtype=torch.float16, device="cuda")
         ops.launch_gemv_w4a8(qw, sc, *act, None, y[0], N, K)
         ops.launch_gemv_w4a16(qw, sc, x, res, y[1], N, K)
         ops.launch_gemv_rmsnorm_w4a16(qw, sc, x, gamma, None, y[2], N, K)
+        ops.gemv_attn_heads_f32_w4a16(qw, sc, heads, res, y[3], N, K)
         torch.cuda.synchronize()
         return y
 

@@ -156,7 +156,7 @@ __global__ void __maxnreg__(gemv_reg_cap(MODE, U)) gemv_w4_kernel(const GemvArgs
         if (regs_form) stage_x_fp16_regs<false>(a.x_fp16, gam, K, kRmsEps, s_q8, s_seed, s_scale);
         else stage_x_fp16_raw<false>(a.x_fp16, nullptr, K, kRmsEps, s_q8, s_seed, s_scale, smem + a.raw_at, a.raw_groups);
     } else if constexpr (XIN == kXF32Heads) {
-        stage_x_from_f32_heads(a.x_f32, K, s_q8, s_seed, s_scale);
+        stage_x_from_f32_heads<false>(a.x_f32, K, s_q8, s_seed, s_scale);
     } else {
         if (!stage_x_from_q8_1_regs<(R * U >= 16)>(a.q8, a.xscale, a.sum8, K, a.vec_ok != 0, s_q8, s_seed, s_scale))
             stage_x_from_q8_1(a.q8, a.xscale, a.sum8, K, a.vec_ok != 0, s_q8, s_seed, s_scale);
@@ -460,7 +460,7 @@ __global__ void __maxnreg__(64) gemv_w4_bulk_kernel(const GemvArgs a) {
         if (regs_form) stage_x_fp16_regs<false>(x16, gam, klen, kRmsEps, s_q8, s_seed, s_scale);
         else stage_x_from_fp16(x16, klen, s_q8, s_seed, s_scale);
     } else if constexpr (XIN == kXF32Heads) {
-        stage_x_from_f32_heads(a.x_f32, klen, s_q8, s_seed, s_scale);
+        stage_x_from_f32_heads<false>(a.x_f32, klen, s_q8, s_seed, s_scale);
     } else {
         const int8_t* q8 = a.q8 + static_cast<size_t>(k_step0) * kStepElems;
         const float* xsc = a.xscale + k_step0 * (kStepElems / kGroup);
@@ -670,7 +670,7 @@ __global__ void __launch_bounds__(kMaxThreads, 2) gemv_w4_stream_kernel(const Ge
         if constexpr (STEPS <= 4) stage_x_from_fp16(a.x_fp16, K, s_q8, s_seed, s_scale);
         else stage_x_fp16_raw<false>(a.x_fp16, nullptr, K, kRmsEps, s_q8, s_seed, s_scale, smem + a.raw_at, a.raw_groups);
     } else if constexpr (XIN == kXF32Heads) {
-        stage_x_from_f32_heads(a.x_f32, K, s_q8, s_seed, s_scale);
+        stage_x_from_f32_heads<(STEPS > 6)>(a.x_f32, K, s_q8, s_seed, s_scale);
     } else if (!stage_x_from_q8_1_regs<STEPS == 8>(a.q8, a.xscale, a.sum8, K, a.vec_ok != 0, s_q8, s_seed, s_scale)) {
         stage_x_from_q8_1(a.q8, a.xscale, a.sum8, K, a.vec_ok != 0, s_q8, s_seed, s_scale);
     }
@@ -909,7 +909,7 @@ __global__ void __launch_bounds__(kMaxThreads, 2) gemv_w4_stream_longk_kernel(co
     } else if constexpr (XIN == kXFp16) {
         stage_x_fp16_raw<false>(a.x_fp16, nullptr, K, kRmsEps, s_q8, s_seed, s_scale, smem + a.raw_at, a.raw_groups);
     } else if constexpr (XIN == kXF32Heads) {
-        stage_x_from_f32_heads(a.x_f32, K, s_q8, s_seed, s_scale);
+        stage_x_from_f32_heads<true>(a.x_f32, K, s_q8, s_seed, s_scale);
     } else if (!stage_x_from_q8_1_regs<true>(a.q8, a.xscale, a.sum8, K, a.vec_ok != 0, s_q8, s_seed, s_scale)) {
         stage_x_from_q8_1(a.q8, a.xscale, a.sum8, K, a.vec_ok != 0, s_q8, s_seed, s_scale);
     }

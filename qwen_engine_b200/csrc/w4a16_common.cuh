@@ -312,22 +312,29 @@ __device__ __forceinline__ uint2 quantize_group_f32_div_halfwarp(const float v[8
 
 // fp32 vector of whole groups (attention heads of 128) -> staged Q8_1 in shared memory, every CTA for itself.
 // x must be 16-byte aligned; blockDim.x a multiple of 32.
+// AHEAD: the next group is fetched behind this one's divisions; for the kernels that have the registers (the 4-load register form
+// would lose a CTA per SM) and K with more than one round.  6144 x 4096 5.7 -> 4.8 us, 28672 x 2048 7.6 -> 6.8.
+template <bool AHEAD>
 __device__ __forceinline__ void stage_x_from_f32_heads(const float* __restrict__ g_x, int K, int8_t* s_q8,
                                                        int32_t* s_seed, float* s_scale) {
     const int hw = threadIdx.x >> 4, hl = threadIdx.x & 15, nhw = blockDim.x >> 4;
     const int groups = K / kGroup;
+    const float4 zero = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    auto load = [&](int g, float4& a, float4& b) {
+        a = b = zero;
+        if (g < groups) {
+            a = reinterpret_cast<const float4*>(g_x + g * kGroup + hl * 8)[0];
+            b = reinterpret_cast<const float4*>(g_x + g * kGroup + hl * 8)[1];
+        }
+    };
+    float4 a, b;
+    if constexpr (AHEAD) load(hw, a, b);
     for (int g0 = 0; g0 < groups; g0 += nhw) {   // uniform trip count: both halves of a warp shuffle together
         const int g = g0 + hw;
         const bool on = g < groups;
-        float v[8];
-        if (on) {
-            const float4 a = reinterpret_cast<const float4*>(g_x + g * kGroup + hl * 8)[0];
-            const float4 b = reinterpret_cast<const float4*>(g_x + g * kGroup + hl * 8)[1];
-            v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w; v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
-        } else {
-#pragma unroll
-            for (int j = 0; j < 8; ++j) v[j] = 0.0f;
-        }
+        if constexpr (!AHEAD) load(g, a, b);
+        const float v[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+        if constexpr (AHEAD) load(g + nhw, a, b);
         int32_t sum;
         float d;
         const uint2 packed = quantize_group_f32_div_halfwarp(v, &sum, &d);

@@ -15,6 +15,7 @@
 
 #include <array>
 #include <cstring>
+#include <exception>
 #include <tuple>
 #include <type_traits>
 
@@ -43,6 +44,20 @@ PyObject* g_str_cuda_stream = nullptr;
 PyObject* g_check = nullptr;                                  // qwen_engine_b200._lib.check
 PyObject* g_view_names[9] = {};                               // attributes of QKVProjectionView, in the C struct's order
 
+// A torch call that may throw (a tensor without storage, as under vmap; the current stream where CUDA cannot start): a C++
+// exception must not leave through the interpreter's C frames, which ends the process.
+template <typename F>
+bool torch_call(F&& f) {
+    try {
+        f();
+        return true;
+    } catch (const c10::Error& e) {
+        PyErr_SetString(PyExc_RuntimeError, e.what_without_backtrace());
+    } catch (const std::exception& e) {
+        PyErr_SetString(PyExc_RuntimeError, e.what());
+    }
+    return false;
+}
 bool not_on_device() {
     PyErr_SetString(PyExc_ValueError, "device pointer expected: tensor is not on a CUDA device");
     return false;
@@ -66,8 +81,7 @@ bool to_pointer(PyObject* o, void** out) {
     if (!THPVariable_Check(o)) return duck_pointer(o, out);
     const at::Tensor& t = THPVariable_Unpack(o);
     if (!t.is_cuda()) return not_on_device();
-    *out = t.data_ptr();
-    return true;
+    return torch_call([&] { *out = t.data_ptr(); });
 }
 bool to_int(PyObject* o, int* out) {
     long v = PyLong_CheckExact(o) ? PyLong_AsLong(o) : -1;
@@ -84,8 +98,7 @@ bool to_int(PyObject* o, int* out) {
 }
 bool to_stream(PyObject* o, w4a16_stream_t* out) {
     if (o == nullptr || o == Py_None) {
-        *out = reinterpret_cast<w4a16_stream_t>(c10::cuda::getCurrentCUDAStream().stream());
-        return true;
+        return torch_call([&] { *out = reinterpret_cast<w4a16_stream_t>(c10::cuda::getCurrentCUDAStream().stream()); });
     }
     PyObject* handle = nullptr;
     if (PyLong_Check(o)) {

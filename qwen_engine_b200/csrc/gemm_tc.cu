@@ -184,6 +184,19 @@ EncodeTiledFn encode_tiled_fn() {
     return fn;
 }
 
+// A driver call wants a context current in the calling thread; the runtime binds the device's only with the thread's first
+// call that needs it, and for a host thread whose first call is a launch of this file that would be the launch itself.
+// True where there was none and now is; a context that the host made current itself stays.
+bool bind_context() {
+    void* p = nullptr;
+    cudaDriverEntryPointQueryResult q;
+    CUcontext ctx = nullptr;
+    if (cudaGetDriverEntryPoint("cuCtxGetCurrent", &p, cudaEnableDefault, &q) != cudaSuccess || q != cudaDriverEntryPointSuccess) return false;
+    if (reinterpret_cast<CUresult (*)(CUcontext*)>(p)(&ctx) != CUDA_SUCCESS || ctx != nullptr) return false;
+    int dev = 0;
+    return cudaGetDevice(&dev) == cudaSuccess && cudaSetDevice(dev) == cudaSuccess;
+}
+
 // Encoded maps are kept per (pointer, shape, box): a model's weight matrices and an engine's activation buffers
 // come back launch after launch, and an encode costs the host a microsecond or two.  A map holds nothing but the
 // address and the geometry, so an entry stays valid even if the memory behind it was freed and handed out again.
@@ -217,9 +230,11 @@ bool encode_2d(CUtensorMap* map, CUtensorMapDataType dt, const void* base, uint6
     const cuuint64_t strides[1] = {row_bytes};
     const cuuint32_t box[2] = {box_inner, box_outer};
     const cuuint32_t estr[2] = {1, 1};
-    if (fn(map, dt, 2, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-           swizzle, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
-        return false;
+    auto encode = [&] {
+        return fn(map, dt, 2, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle,
+                  CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+    };
+    if (!encode() && !(bind_context() && encode())) return false;
     std::lock_guard<std::mutex> lock(mu);
     if (cache.size() < kMapCacheEntries) cache.emplace_back(key, *map);
     else { cache[next] = {key, *map}; next = (next + 1) % kMapCacheEntries; }

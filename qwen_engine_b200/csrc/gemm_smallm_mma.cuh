@@ -238,6 +238,7 @@ __global__ void __launch_bounds__(512, NT == 1 ? 2 : 1) gemm_smallm_mma_kernel(c
                              : "=r"(have) : "r"(bar) : "memory");
             if (!have) atomicAdd(&g_mma_wait_timeouts, 1u);
         }
+        __syncwarp();            // the peers' stores before the reads of all lanes: a shuffle orders no memory
         have = __shfl_sync(0xFFFFFFFFu, have, 0);
         if (!have) break;
         float y[4] = {0.0f, 0.0f, 0.0f, 0.0f};

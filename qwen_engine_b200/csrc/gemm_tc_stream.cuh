@@ -362,8 +362,10 @@ __global__ void __launch_bounds__(kStThreads, 1) gemm_w4a16_tc_stream_kernel(con
                                 __float_as_uint(v[q + 2]), __float_as_uint(v[q + 3]));
                 }
             }
-            bool have = true;
-            if (lane == 0) have = wait_regardless(part_full, 0, 4 * kWaitLimit);
+            bool have = false;
+            if (lane == 0)
+                for (unsigned it = 0; it < 4 * kWaitLimit && !have; ++it) have = mbar_try_wait_cluster(part_full, 0);
+            __syncwarp();                        // the peers' stores before the reads of all lanes: a shuffle orders no memory
             have = __shfl_sync(0xFFFFFFFFu, have ? 1 : 0, 0) != 0;
             if (!have && lane == 0) { *s_abort = 1; atomicAdd(&g_tc_wait_timeouts, 1u); }
             if (have) {

@@ -194,6 +194,7 @@ __device__ void producer_loop(const PSweepArgs& a, uint8_t* ring, uint32_t full0
             const int rows = min(p.chunk_rows, p.num_rows - r);
             int ok = 1;
             if (lane == 0) ok = bar_wait(empty0 + 8u * slot, phase ^ 1, s_abort) ? 1 : 0;
+            __syncwarp();            // the consumers' reads of the slot before the copies of all lanes into it
             ok = __shfl_sync(0xFFFFFFFFu, ok, 0);
             if (!ok) {
                 // Leaving early: a CTA must not exit while bulk copies into its shared memory are in flight.  The
@@ -526,6 +527,7 @@ __device__ void consumer_loop(const PSweepArgs& a, uint8_t* ring, uint32_t full0
             const int rows = min(p.chunk_rows, p.num_rows - r);
             int wait_ok = 1;
             if (lane == 0) wait_ok = bar_wait(full0 + 8u * slot, phase, s_abort) ? 1 : 0;
+            __syncwarp();            // the copies into the slot before the reads of all lanes: a shuffle orders no memory
             wait_ok = __shfl_sync(0xFFFFFFFFu, wait_ok, 0);
             if (!wait_ok) {
                 if (tid == 0) atomicExch(a.status, 1);

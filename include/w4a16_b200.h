@@ -78,8 +78,12 @@ W4A16_API int w4a16_init(void);
  * option or a value outside its range.
  */
 enum {
-    W4A16_OPT_PDL = 1,               /* 1 (default): programmatic dependent launch, so that the next kernel's weight
-                                        prefetch overlaps this kernel's tail; 0: plain stream-ordered launches */
+    W4A16_OPT_PDL = 1,               /* 1 (default): programmatic dependent launch: the next kernel starts in this kernel's
+                                        tail and reads its weights, its group scales and the RMSNorm gain of a projection
+                                        with the norm in it (*_rmsnorm_*) there, so none of these may be written by launches
+                                        of this library in front of it on the stream, unless a full dependency lies in
+                                        between (an event, a copy, a kernel launched without the attribute); all other
+                                        inputs are read behind the launches in front.  0: plain stream-ordered launches */
     W4A16_OPT_SIGNAL_WAIT_SPINS = 2, /* polls (about 0.2 us apart) that w4a16_sample_finish_after_signals and
                                         w4a16_gather_after_signals spend on a peer's flag, and a CTA of the persistent
                                         sweep on another CTA's counter or tagged word, before giving up and reporting

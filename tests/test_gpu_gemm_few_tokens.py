@@ -56,3 +56,31 @@ def test_rmsnorm_q8_1_sizes(hidden, offset):
     assert np.array_equal(util.to_np(y).view(np.uint16), want.view(np.uint16))
     w8, ws, wsum = oracle.quantize_q8_1(want)
     assert np.array_equal(util.to_np(q8), w8) and np.array_equal(util.to_np(xs), ws) and np.array_equal(util.to_np(s8), wsum)
+
+
+def test_rmsnorm_q8_1_gain_written_by_the_launch_in_front():
+    """The gain is read as the launch in front left it: here a row of an embedding table, another one each time."""
+    import qwen_engine_b200 as ops
+    from qwen_engine_b200 import synth
+    H, V = 1536, 64
+    table, sc = util.to_dev(synth.packed_weights(9, "e", V, H)), util.to_dev(synth.scales(9, "e", V, H))
+    x, tokens = util.to_dev(synth.activations(9, "e", H)), torch.arange(V, dtype=torch.int32, device="cuda")
+    gain = torch.zeros(H, dtype=torch.float16, device="cuda")
+
+    def launch(t, y, gain):
+        q8 = (torch.empty(H, dtype=torch.int8, device="cuda"), torch.empty(H // 128, dtype=torch.float32, device="cuda"),
+              torch.empty(H // 8, dtype=torch.int32, device="cuda"))
+        torch.cuda.synchronize()
+        ops.launch_embed_lookup_w4a16(table, sc, tokens[t:], gain, None, 1, None, H, V)
+        return q8, lambda: ops.launch_rmsnorm_q8_1(x, gain, y, *q8, None, H)
+
+    y = torch.empty((2, V, H), dtype=torch.float16, device="cuda")
+    for t in range(V):
+        q8, norm = launch(t, y[0, t], gain)
+        norm()
+        want8, norm = launch(t, y[1, t], torch.zeros_like(gain))
+        torch.cuda.synchronize()      # the gain is there before the launch
+        norm()
+        torch.cuda.synchronize()
+        assert all(torch.equal(a, b) for a, b in zip(q8, want8))
+    assert torch.equal(y[0].view(torch.int16), y[1].view(torch.int16))

@@ -49,6 +49,15 @@ __device__ __forceinline__ void mma_m16n8k16(float (&d)[4], uint32_t a0, uint32_
 
 __device__ unsigned int g_mma_wait_timeouts = 0;
 
+// Bounded wait for the stores of the cluster's CTAs that are counted on `bar`.
+__device__ __forceinline__ bool wait_for_peers(uint32_t bar) {
+    uint32_t ok = 0;
+    for (unsigned it = 0; it < (1u << 22) && ok == 0; ++it)
+        asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], 0;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+                     : "=r"(ok) : "r"(bar) : "memory");
+    return ok != 0;
+}
+
 template <int MODE, int NT>
 __global__ void __launch_bounds__(512, NT == 1 ? 2 : 1) gemm_smallm_mma_kernel(const SmallMArgs a, const SmallMmaPlan p) {
     constexpr int UW = (MODE == kSwiglu) ? 8 : 16;   // outputs per warp
@@ -233,10 +242,11 @@ __global__ void __launch_bounds__(512, NT == 1 ? 2 : 1) gemm_smallm_mma_kernel(c
         }
         int have = S == 1;
         if (S > 1 && lane == 0) {
-            for (unsigned it = 0; it < (1u << 22) && !have; ++it)
-                asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], 0;\n\tselp.u32 %0, 1, 0, p;\n\t}"
-                             : "=r"(have) : "r"(bar) : "memory");
-            if (!have) atomicAdd(&g_mma_wait_timeouts, 1u);
+            have = wait_for_peers(bar) ? 1 : 0;
+            if (!have) {
+                atomicAdd(&g_mma_wait_timeouts, 1u);
+                wait_for_peers(bar);     // what is still on its way into this CTA's memory has to land before it goes (bounded too)
+            }
         }
         __syncwarp();            // the peers' stores before the reads of all lanes: a shuffle orders no memory
         have = __shfl_sync(0xFFFFFFFFu, have, 0);

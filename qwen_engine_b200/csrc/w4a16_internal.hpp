@@ -59,12 +59,29 @@ inline cudaError_t launch_kernel(void (*kernel)(KArgs...), dim3 grid, dim3 block
 // Clusters of `cluster` CTAs of a kernel that can be resident at once on the current device (0 where the runtime cannot say).
 int max_active_clusters(const void* kernel, int block, size_t smem, int cluster);
 
+// What a plan depends on beside the kernel: the launch's numbers whole, so that no two shapes share one.
+struct PlanKey {
+    int device, mode, tokens, K, rows;
+    bool operator==(const PlanKey&) const = default;
+};
+struct PlanKeyHash {
+    size_t operator()(const PlanKey& k) const {
+        uint64_t h = 0;
+        for (int v : {k.device, k.mode, k.tokens, k.K, k.rows}) h = (h ^ static_cast<uint32_t>(v)) * 0x9E3779B97F4A7C15ull, h ^= h >> 32;
+        return h;
+    }
+};
+inline PlanKey plan_key(int mode, int tokens, int K, int rows) {
+    int dev = 0;
+    cudaGetDevice(&dev);
+    return {dev, mode, tokens, K, rows};
+}
 // How a launch of a shape is cut, worked out once per shape (bounded: a host that goes through many shapes starts over).
 template <typename V>
 class PlanCache {
 public:
     template <typename F>
-    V get(uint64_t key, F&& make) {
+    V get(const PlanKey& key, F&& make) {
         std::lock_guard<std::mutex> lock(mu_);
         auto it = map_.find(key);
         if (it != map_.end()) return it->second;
@@ -74,15 +91,8 @@ public:
 
 private:
     std::mutex mu_;
-    std::unordered_map<uint64_t, V> map_;
+    std::unordered_map<PlanKey, V, PlanKeyHash> map_;
 };
-// device | mode | tokens | K / 128 | rows
-inline uint64_t plan_key(int mode, int tokens, int K, int rows) {
-    int dev = 0;
-    cudaGetDevice(&dev);
-    return (static_cast<uint64_t>(dev) << 58) | (static_cast<uint64_t>(mode & 3) << 56) | (static_cast<uint64_t>(tokens & 0xFFFF) << 40) |
-           (static_cast<uint64_t>((K / 128) & 0xFFFF) << 24) | static_cast<uint64_t>(rows & 0xFFFFFF);
-}
 
 // ---- Q8_1 quantisers (q8_1_quantize.cu) ----
 int quantize_fp16_to_q8_1(const __half* x, int8_t* q8, float* scale, int32_t* sum8, int n, cudaStream_t stream);

@@ -79,3 +79,27 @@ def test_compat_header_compiles(tmp_path):
         '&qwen::launch_sample_and_advance; (void)a; return 0; }\n')
     subprocess.run(["nvcc", "-std=c++17", "-gencode", "arch=compute_100a,code=sm_100a", "-c", "-I", str(ROOT / "include"), "-o", str(tmp_path / "t2.o"), str(src2)],
                    check=True)
+
+
+def test_no_two_shapes_share_a_plan(tmp_path):
+    """Numbers that differ by a power of two only: 65553 tokens are not 17, 16781312 rows not 4096."""
+    import shutil
+    import subprocess
+    if shutil.which("nvcc") is None:
+        pytest.skip("nvcc not on PATH")
+    src = tmp_path / "plan.cu"
+    src.write_text(
+        '#include "w4a16_internal.hpp"\n'
+        'int main() {\n'
+        '    w4::PlanCache<int> plans;\n'
+        '    const int shapes[][4] = {{0, 17, 2048, 4096}, {0, 17 + (1 << 16), 2048, 4096}, {0, 17, 2048 + 128 * (1 << 16), 4096},\n'
+        '                             {0, 17, 2048, 4096 + (1 << 24)}, {2, 17, 2048, 4096}, {0, 17, 4096, 2048}};\n'
+        '    int n = 0;\n'
+        '    for (auto& s : shapes) { plans.get(w4::plan_key(s[0], s[1], s[2], s[3]), [&] { return n; }); ++n; }\n'
+        '    n = 0;\n'
+        '    for (auto& s : shapes) if (plans.get(w4::plan_key(s[0], s[1], s[2], s[3]), [] { return -1; }) != n++) return n;\n'
+        '    return 0;\n'
+        '}\n')
+    exe = tmp_path / "plan"
+    subprocess.run(["nvcc", "-std=c++20", "-I", str(ROOT / "qwen_engine_b200" / "csrc"), "-o", str(exe), str(src)], check=True)
+    assert subprocess.run([str(exe)]).returncode == 0

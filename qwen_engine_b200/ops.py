@@ -59,19 +59,29 @@ _NATIVE = (
     "launch_gemv_dual_gate_up_swiglu_rmsnorm_w4a16_q8_1", "launch_gemm_prefill_w4a16",
     "launch_gemm_prefill_qkv_w4a16", "launch_gemm_prefill_dual_gate_up_swiglu_w4a16", "gemv_group_dots",
 )
-try:
-    from . import _launch
-except ImportError as _e:      # not built (yet): the functions exist and say so, so that the build script can import this
-    _launch_error = str(_e)
 
-    class _launch:  # noqa: N801
-        @staticmethod
+
+def _native(name: str):
+    """The builtin `name`.  Its module, and with it the CUDA library, is loaded by the first function asked for: a process that
+    wants shapes or synthetic tensors only stays free of both.  Where it is not built the function exists and says so when
+    called, so that the build script can import this package."""
+    try:
+        from . import _launch
+    except ImportError as e:
+        why = str(e)
+
         def missing(*_args, **_kwargs):
-            raise ImportError(f"qwen_engine_b200/_launch.so cannot be loaded ({_launch_error}): build it with "
+            raise ImportError(f"qwen_engine_b200/_launch.so cannot be loaded ({why}): build it with "
                               "`python -m qwen_engine_b200.build` (there is no non-CUDA fallback)")
+        return missing
+    globals().update({n: getattr(_launch, n) for n in _NATIVE})      # from now on plain module attributes
+    return getattr(_launch, name)
 
-globals().update({_n: getattr(_launch, _n, None) or _launch.missing for _n in _NATIVE})
-_sweep_run_device = getattr(_launch, "sweep_run_device", None) or _launch.missing
+
+def __getattr__(name: str):
+    if name in _NATIVE:
+        return _native(name)
+    raise AttributeError(f"module {__name__!r} has no attribute {name!r}")
 
 
 @dataclass
@@ -261,10 +271,11 @@ class DecodeSweep:
         check("w4a16_sweep_create", lib.w4a16_sweep_create(ctypes.byref(desc), _stream(stream), ctypes.byref(handle)))
         self._h = handle
         self._handle = handle.value
+        self._run_device = _native("sweep_run_device")
         self.launches = lib.w4a16_sweep_launches(handle)
 
     def run_device(self, h_in: torch.Tensor, h_out: torch.Tensor, stream=None):
-        _sweep_run_device(self._handle, h_in, h_out, stream)
+        self._run_device(self._handle, h_in, h_out, stream)
 
     def run_host(self, h_in: torch.Tensor, h_out: torch.Tensor, stream=None):
         """h_in / h_out: pinned host fp16 tensors; asynchronous on the stream."""

@@ -35,3 +35,48 @@ except RuntimeError as e:
 def test_errors_of_torch_are_python_errors(script):
     r = subprocess.run([sys.executable, "-W", "ignore", "-c", script], cwd=ROOT, capture_output=True, text=True)
     assert r.returncode == 0 and "raised " in r.stdout, r.stderr[-2000:]
+
+
+# Which of the package's two libraries a process has mapped.
+MAPPED = """
+import sys
+def mapped():
+    return sorted({n for l in open("/proc/self/maps") for n in ("_launch.so", "libw4a16_b200.so") if l.rstrip().endswith("/" + n)})
+"""
+
+
+def _python(script):
+    r = subprocess.run([sys.executable, "-W", "ignore", "-c", MAPPED + script], cwd=ROOT, capture_output=True, text=True)
+    assert r.returncode == 0, r.stderr[-2000:]
+    return r.stdout.split()
+
+
+def test_the_cuda_library_is_loaded_by_the_first_launch_function():
+    """The CPU arm of the benchmark and whoever wants shapes and synthetic tensors only stay free of it."""
+    out = _python("""
+from qwen_engine_b200 import nsplit, ops, qwenbin, synth
+import qwen_engine_b200 as q
+assert mapped() == [], mapped()
+assert hasattr(q, "launch_gemv_w4a8") and q.launch_gemv_w4a8 is ops.launch_gemv_w4a8
+assert mapped() == ["_launch.so", "libw4a16_b200.so"], mapped()
+assert "launch_gemv_w4a8" in vars(ops) and "launch_gemm_prefill_w4a16" in vars(q)
+names = {}
+exec("from qwen_engine_b200 import *", names)
+assert set(ops.__all__) <= set(names) and "ops" in names
+assert not hasattr(ops, "launch_nothing") and not hasattr(q, "launch_nothing")
+print("ok")
+""")
+    assert out == ["ok"]
+
+
+def test_a_missing_build_says_so_when_a_function_is_called():
+    out = _python("""
+sys.modules["qwen_engine_b200._launch"] = None
+import qwen_engine_b200 as q
+f = q.launch_gemv_w4a16
+try:
+    f()
+except ImportError as e:
+    print("build" in str(e))
+""")
+    assert out == ["True"]

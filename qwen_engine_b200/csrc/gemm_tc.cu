@@ -15,7 +15,6 @@
 #include <algorithm>
 #include <mutex>
 #include <utility>
-#include <vector>
 
 #include "gemm_smallm.cuh"
 #include "w4a16_common.cuh"
@@ -228,13 +227,13 @@ bool encode_2d(CUtensorMap* map, CUtensorMapDataType dt, const void* base, uint6
                uint64_t row_bytes, uint32_t box_inner, uint32_t box_outer,
                CUtensorMapSwizzle swizzle = CU_TENSOR_MAP_SWIZZLE_128B) {
     static std::mutex mu;
-    static std::vector<std::pair<MapKey, CUtensorMap>> cache;
-    static size_t next = 0;
+    static std::pair<MapKey, CUtensorMap> cache[kMapCacheEntries];
+    static size_t used = 0, next = 0;
     const MapKey key{base, inner, outer, row_bytes, box_inner, box_outer, static_cast<int>(dt), static_cast<int>(swizzle)};
     {
         std::lock_guard<std::mutex> lock(mu);
-        for (const auto& kv : cache)
-            if (kv.first == key) { *map = kv.second; return true; }
+        for (size_t i = 0; i < used; ++i)
+            if (cache[i].first == key) { *map = cache[i].second; return true; }
     }
     EncodeTiledFn fn = encode_tiled_fn();
     if (!fn) return false;
@@ -248,8 +247,9 @@ bool encode_2d(CUtensorMap* map, CUtensorMapDataType dt, const void* base, uint6
     };
     if (!encode() && !(bind_context() && encode())) return false;
     std::lock_guard<std::mutex> lock(mu);
-    if (cache.size() < kMapCacheEntries) cache.emplace_back(key, *map);
-    else { cache[next] = {key, *map}; next = (next + 1) % kMapCacheEntries; }
+    cache[next] = {key, *map};
+    next = (next + 1) % kMapCacheEntries;
+    used = std::min(used + 1, kMapCacheEntries);
     return true;
 }
 

@@ -4,6 +4,7 @@
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
 #include <mutex>
+#include <new>
 #include <unordered_map>
 #include <utility>
 
@@ -85,8 +86,13 @@ public:
         std::lock_guard<std::mutex> lock(mu_);
         auto it = map_.find(key);
         if (it != map_.end()) return it->second;
-        if (map_.size() >= 4096) map_.clear();
-        return map_.emplace(key, make()).first->second;
+        const V plan = make();
+        try {
+            if (map_.size() >= 4096) map_.clear();
+            map_.emplace(key, plan);
+        } catch (const std::bad_alloc&) {        // not kept: the C entry points let no exception out
+        }
+        return plan;
     }
 
 private:

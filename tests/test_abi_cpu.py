@@ -81,25 +81,50 @@ def test_compat_header_compiles(tmp_path):
                    check=True)
 
 
-def test_no_two_shapes_share_a_plan(tmp_path):
-    """Numbers that differ by a power of two only: 65553 tokens are not 17, 16781312 rows not 4096."""
+def _run_cpp(tmp_path, text):
+    """Compiles and runs a host program against the library's internal header; its exit status."""
     import shutil
     import subprocess
     if shutil.which("nvcc") is None:
         pytest.skip("nvcc not on PATH")
-    src = tmp_path / "plan.cu"
-    src.write_text(
-        '#include "w4a16_internal.hpp"\n'
-        'int main() {\n'
-        '    w4::PlanCache<int> plans;\n'
-        '    const int shapes[][4] = {{0, 17, 2048, 4096}, {0, 17 + (1 << 16), 2048, 4096}, {0, 17, 2048 + 128 * (1 << 16), 4096},\n'
-        '                             {0, 17, 2048, 4096 + (1 << 24)}, {2, 17, 2048, 4096}, {0, 17, 4096, 2048}};\n'
-        '    int n = 0;\n'
-        '    for (auto& s : shapes) { plans.get(w4::plan_key(s[0], s[1], s[2], s[3]), [&] { return n; }); ++n; }\n'
-        '    n = 0;\n'
-        '    for (auto& s : shapes) if (plans.get(w4::plan_key(s[0], s[1], s[2], s[3]), [] { return -1; }) != n++) return n;\n'
-        '    return 0;\n'
-        '}\n')
-    exe = tmp_path / "plan"
+    src, exe = tmp_path / "t.cpp", tmp_path / "t"
+    src.write_text(text)
     subprocess.run(["nvcc", "-std=c++20", "-I", str(ROOT / "qwen_engine_b200" / "csrc"), "-o", str(exe), str(src)], check=True)
-    assert subprocess.run([str(exe)]).returncode == 0
+    return subprocess.run([str(exe)]).returncode
+
+
+def test_no_two_shapes_share_a_plan(tmp_path):
+    """Numbers that differ by a power of two only: 65553 tokens are not 17, 16781312 rows not 4096."""
+    assert _run_cpp(tmp_path, '''#include "w4a16_internal.hpp"
+int main() {
+    w4::PlanCache<int> plans;
+    const int shapes[][4] = {{0, 17, 2048, 4096}, {0, 17 + (1 << 16), 2048, 4096}, {0, 17, 2048 + 128 * (1 << 16), 4096},
+                             {0, 17, 2048, 4096 + (1 << 24)}, {2, 17, 2048, 4096}, {0, 17, 4096, 2048}};
+    int n = 0;
+    for (auto& s : shapes) { plans.get(w4::plan_key(s[0], s[1], s[2], s[3]), [&] { return n; }); ++n; }
+    n = 0;
+    for (auto& s : shapes) if (plans.get(w4::plan_key(s[0], s[1], s[2], s[3]), [] { return -1; }) != n++) return n;
+    return 0;
+}
+''') == 0
+
+
+def test_a_plan_that_cannot_be_kept_is_returned(tmp_path):
+    """Out of host memory: no exception leaves the C entry points for that."""
+    assert _run_cpp(tmp_path, '''#include "w4a16_internal.hpp"
+#include <cstdlib>
+#include <new>
+static bool g_full = false;
+void* operator new(size_t n) { void* p = g_full ? nullptr : std::malloc(n); if (!p) throw std::bad_alloc(); return p; }
+void operator delete(void* p) noexcept { std::free(p); }
+void operator delete(void* p, size_t) noexcept { std::free(p); }
+int main() {
+    w4::PlanCache<int> plans;
+    for (int i = 0; i < 40; ++i) {
+        g_full = i % 2;
+        if (plans.get(w4::PlanKey{0, 0, i, 256, 16}, [&] { return i; }) != i) return 1;
+    }
+    g_full = false;
+    return plans.get(w4::PlanKey{0, 0, 2, 256, 16}, [] { return -1; }) == 2 && plans.get(w4::PlanKey{0, 0, 3, 256, 16}, [] { return 7; }) == 7 ? 0 : 2;
+}
+''') == 0

@@ -51,8 +51,15 @@ def up_to_date() -> bool:
     return _newer(LIB, _inputs()) and _launch_up_to_date()
 
 
+def _built_for() -> str:
+    """What the Python module depends on beside its sources: torch's C++ ABI and the interpreter's."""
+    from importlib.metadata import version
+    return f"torch {version('torch')}, {sys.implementation.cache_tag}"
+
+
 def _launch_up_to_date() -> bool:
-    return _newer(LAUNCH, [LAUNCH_SOURCE, PKG.parent / "include" / "w4a16_b200.h"])
+    # (the module carries the text in itself)
+    return _newer(LAUNCH, [LAUNCH_SOURCE, PKG.parent / "include" / "w4a16_b200.h"]) and f"[{_built_for()}]".encode() in LAUNCH.read_bytes()
 
 
 def build_launch(force: bool = False) -> Path:
@@ -67,7 +74,7 @@ def build_launch(force: bool = False) -> Path:
     torch_lib = Path(torch.__file__).resolve().parent / "lib"
     includes = [*cpp_extension.include_paths(device_type="cuda"), sysconfig.get_paths()["include"]]
     cmd = [shutil.which("g++") or "g++", "-O2", "-std=c++20", "-shared", "-fPIC", "-fvisibility=hidden",
-           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch.compiled_with_cxx11_abi())}", *[f"-isystem{p}" for p in includes],
+           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch.compiled_with_cxx11_abi())}", f'-DW4_BUILT_FOR="{_built_for()}"', *[f"-isystem{p}" for p in includes],
            str(LAUNCH_SOURCE), "-o", str(LAUNCH), f"-L{PKG}", "-l:libw4a16_b200.so", f"-L{torch_lib}", "-ltorch_python",
            "-ltorch", "-ltorch_cpu", "-lc10", "-lc10_cuda", "-Wl,-rpath,$ORIGIN"]
     res = subprocess.run(cmd, capture_output=True, text=True)

@@ -363,7 +363,7 @@ PyMethodDef g_methods[] = {
     {nullptr, nullptr, 0, nullptr}};
 
 PyModuleDef g_module = {PyModuleDef_HEAD_INIT, "qwen_engine_b200._launch",
-                        "Launch functions of libw4a16_b200.so on torch CUDA tensors.", -1, g_methods,
+                        "Launch functions of libw4a16_b200.so on torch CUDA tensors [" W4_BUILT_FOR "].", -1, g_methods,
                         nullptr, nullptr, nullptr, nullptr};
 
 }  // namespace

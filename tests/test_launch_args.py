@@ -80,3 +80,12 @@ except ImportError as e:
     print("build" in str(e))
 """)
     assert out == ["True"]
+
+
+def test_the_module_is_built_anew_for_another_torch_or_python(monkeypatch):
+    from qwen_engine_b200 import build
+    build.build()
+    assert build.up_to_date()
+    for text in ("torch 2.11", "torch 0.0.1, cpython-312"):
+        monkeypatch.setattr(build, "_built_for", lambda text=text: text)
+        assert not build.up_to_date()

@@ -98,6 +98,7 @@ class QKVProjectionView:
     d_v: torch.Tensor
 
     def pod(self) -> QKVView:
+        """The C struct, for hosts that call the C functions through load()."""
         return QKVView(*[_ptr(getattr(self, n)) for n, _ in QKVView._fields_])
 
 

@@ -39,7 +39,7 @@ def test_first_cuda_call_of_a_thread(M, N, K):
 
 # (tokens, rows, K): few tokens with K over a cluster, streaming with a K split (partials in memory of their own and on top
 # of the rings), CTA pairs
-SIZES = [(4, 1536, 8960), (16, 1536, 8960), (47, 1536, 8960), (115, 1536, 1536), (128, 640, 8960), (600, 4096, 1024)]
+SIZES = [(4, 1536, 8960), (16, 1536, 8960), (47, 1536, 8960), (115, 1536, 1536), (128, 7680, 8960), (600, 4096, 1024)]
 
 
 def test_two_threads_on_two_streams_give_the_bits_of_one():

@@ -15,6 +15,8 @@ torch = pytest.importorskip("torch")
     (17, 128, 256, 0.02, False), (47, 1536, 8960, 0.02, True), (48, 520, 512, 0.5, True), (64, 2048, 1536, 0.02, False),
     (65, 20000, 256, 0.02, True), (112, 384, 2304, 0.07, True), (115, 1536, 1536, 0.02, True), (128, 17920, 768, 0.02, False),
     (129, 1536, 1536, 0.5, True), (203, 17920, 1536, 0.02, False), (255, 132, 8960, 0.02, True), (256, 300, 1024, 0.02, False),
+    # 128-token tiles with a K split leave no room beside the rings: the partial sums go on top of them
+    (120, 7680, 8960, 0.02, True), (256, 4600, 8960, 0.5, False),
 ])
 def test_stream_kernel_matches_oracle(M, N, K, scale_max, res):
     import qwen_engine_b200 as ops

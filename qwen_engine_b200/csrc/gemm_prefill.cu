@@ -168,10 +168,12 @@ int gemm_launch(GemmArgs g, cudaStream_t stream) {
     if (int st = ensure_device_ready(&dev)) return st;
 
     // The tcgen05 kernel pads the token count to its smallest tile (16), so below a handful of tokens the CUDA-core
-    // few-token form (the decode GEMV's memory behaviour with fp16 arithmetic) is the faster one.  Measured
-    // crossovers on B200: 3 tokens where K > 4096 (down: the few-token form stages only two tokens per pass there),
-    // 4 on matrices tall enough to give every SM a CTA of their own (gate_up), 7 on the narrow K <= 4096 shapes
-    // (QKV, O).  The CUDA-core forms also take what TMA cannot address.
+    // few-token form (the decode GEMV's memory behaviour with fp16 arithmetic) is the faster one: 3 tokens where K > 4096
+    // (down: the few-token form stages only two tokens per pass there), 4 on matrices tall enough to give every SM a CTA of
+    // their own (gate_up), 7 on the narrow K <= 4096 shapes (QKV, O).  These lines were measured against the tcgen05 kernel
+    // in front of the streaming one; against that the two forms meet earlier (CUDA cores / tcgen05, us: down 10.6 / 7.3 and
+    // gate_up 8.2 / 8.1 at 2 tokens, O 5.4 / 4.0 and QKV 4.4 / 4.8 at 4).  Only shapes that the mma form below refuses come
+    // here with 2 tokens or more.  The CUDA-core forms also take what TMA cannot address.
     const int tc_min_m_opt = option(W4A16_OPT_GEMM_MIN_TOKENS_TENSOR_CORE);
     const int rows_all = g.rows[0] + (g.mode == kQkv ? g.rows[1] + g.rows[2] : 0);
     const int tc_min_m = tc_min_m_opt > 0 ? tc_min_m_opt : (g.K > 4096 ? 3 : (rows_all >= 64 * dev->sm_count ? 4 : 7));

@@ -382,8 +382,8 @@ int pair_launch(const GemmArgs& g, int sm_count, cudaStream_t stream) {
     bool words = word(a.residual);
     for (int p = 0; p < a.num_peers; ++p) words = words && word(a.peer_out[p]);
     for (int t = 0; t < (g.mode == kQkv ? 3 : 1); ++t) words = words && a.out_ld[t] % 2 == 0 && a.rows[t] % 2 == 0 && word(a.out[t]);
-    // weight matrices that do not stay in L2 next to the tokens and outputs: panels of 4 token tiles (measured on
-    // 28672 x 8192 at 4096 tokens: 1.62 -> 1.56 ms, DRAM reads 1.77 -> under 1 GB); smaller ones: row tiles fastest
+    // weight matrices that do not stay in L2 next to the tokens and outputs: panels of 4 token tiles (28672 x 8192 at 4096
+    // tokens, passes back to back: 1543 us in panels of 1, 1460 in panels of 4); smaller ones: row tiles fastest
     a.panel = static_cast<size_t>(tiles) * kTileRows * (g.K / 2) > (48u << 20) ? 4 : 1;
     if (!encode_2d(&a.tmap_x, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, g.x, static_cast<uint64_t>(g.K), static_cast<uint64_t>(g.M),
                    static_cast<uint64_t>(g.K) * 2, kBK, static_cast<uint32_t>(a.n_half / 2)))

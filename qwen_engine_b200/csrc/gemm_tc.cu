@@ -307,7 +307,7 @@ StreamPlan stream_plan(int M, int K, int tiles, int sm_count) {
                 const double work = per * std::max(400.0, 4.0 * T) + ends;
                 if (best.smem != 0 && work >= best_work) continue;
                 StreamPlan p;
-                if (!plan_stream(T, split, per, &p)) continue;
+                if (!plan_stream(T, split, steps, &p)) continue;
                 if (split > 1 && max_active_clusters(reinterpret_cast<const void*>(gemm_w4a16_tc_stream_kernel<MODE>), kStThreads, p.smem, split) < tiles * ts) continue;
                 best = p;
                 best.cost = waves * (5500.0 + per * std::max(450.0, 8.6 * T) + ends);

@@ -452,7 +452,7 @@ __global__ void __launch_bounds__(kPairThreads, 1) gemm_w4a16_tc_pair_kernel(con
         __syncwarp();
     } else if (warp == kRawWarp) {
         // ================= TMA: raw packed weights of this CTA's 128 rows (private ring) =================
-        if (lane == 0) {
+        if (elect_one()) {
             int rs = 0;
             uint32_t rph = 1;
             bool ok = true;
@@ -469,7 +469,7 @@ __global__ void __launch_bounds__(kPairThreads, 1) gemm_w4a16_tc_pair_kernel(con
         __syncwarp();
     } else if (warp == kRawWarp + 1) {
         // ================= TMA: this CTA's half of the token tile; bytes counted on the LEADER's barrier =================
-        if (lane == 0) {
+        if (elect_one()) {
             int slot = 0;
             uint32_t dph = 1;
             bool ok = true;

@@ -14,9 +14,16 @@
 // `lane == 0` branch every operand is moved to a uniform register first and each MMA costs 67.
 //
 //   warps 0..15 : dequantise, four warps a step (steps s % 4), then the epilogue
-//   warp 16     : allocates tensor memory; one thread issues the MMAs (8 per step) behind ONE barrier per slot that counts
-//                 the dequantising warps and the token tile's bytes
-//   warp 17     : one thread loads by TMA: packed weights, 128 rows x 128 k (8 KB) per ring slot, and tokens, T x 128 k per slot
+//   warp 16     : allocates tensor memory; one thread issues the MMAs of the even steps (8 per step) behind ONE barrier per slot
+//                 that counts the dequantising warps and the token tile's bytes; warp 19 the same for the odd steps, which have an
+//                 accumulator of their own
+//   warp 17     : one thread loads packed weights by TMA, 128 rows x 128 k (8 KB) per ring slot
+//   warp 18     : one thread loads tokens by TMA, T x 128 k per slot
+//
+// The loading threads are chosen by elect.sync too, and each ring has one of its own: as one `lane == 0` thread that looked
+// after both rings a step took them 430 cycles, and with every other part of the kernel taken out a launch was hardly faster
+// (gate_up at 47 tokens 8.6 us, 5.7 without data, dequantisation, MMAs or epilogue).  Every token slot that fits is asked for at
+// once.  One layer of 1536 / 8960 at 47 tokens: QKV 6.0 -> 4.7, O 5.6 -> 4.3, gate_up 8.5 -> 6.7, down 8.4 -> 6.4 us a launch.
 //
 // Tensor memory: even and odd steps go into accumulators of their own: half as many additions per fp32 sum, which at
 // K = 8192 is the difference between 2.7 and 2 fp16 steps of error.  A slots of 64 columns follow: six up to 64 tokens,
@@ -26,12 +33,13 @@
 // into the owner's shared memory which count themselves on the owner's mbarrier, so the exchange needs no cluster barrier
 // behind it; the one that makes sure that the peers have started is passed before the main loop.  A CTA sends T x 512 bytes
 // at about 18 bytes a cycle, which is why the planner prefers a smaller token tile to a deeper K split.
-constexpr int kStDqWarps = 16;
-constexpr int kStGroups = kStDqWarps / 4;        // groups of four warps = 128 rows
-constexpr int kStDqThreads = kStDqWarps * 32;
-constexpr int kStThreads = kStDqThreads + 2 * 32;
+constexpr int kStGroups = 4;                     // groups of four dequantising warps = 128 rows
+constexpr int kStDqWarps = 4 * kStGroups, kStDqThreads = kStDqWarps * 32;
+constexpr int kStWeightWarp = kStDqWarps + 1, kStTokenWarp = kStDqWarps + 2;      // the others behind the dequantising ones issue MMAs
+constexpr int kStIssuers = 2;
+constexpr int kStThreads = kStDqThreads + (2 + kStIssuers) * 32;
 constexpr int kStRawBytes = kTileRows * 64;      // 128 rows x 128 k of packed nibbles
-constexpr int kStMaxRaw = 24, kStMaxSlots = 6;   // ring slots at most
+constexpr int kStMaxRaw = 24, kStMaxSlots = 12;  // ring slots at most
 constexpr int kStACols = kGroup / 2;             // 128 k of fp16 = 64 columns
 constexpr int kStMaxSplit = 8;                   // portable cluster size
 
@@ -39,9 +47,11 @@ constexpr int kStMaxSplit = 8;                   // portable cluster size
 struct StreamPlan {
     int T;                // tokens of a CTA's tile
     int ksplit;           // cluster size along grid z
+    int steps_each;       // steps of every slice; the first K / 128 - ksplit * steps_each have one more
     int tpr;              // tokens a CTA of the cluster finishes (multiple of 4)
     int raw_slots;        // multiple of 4: a slot always belongs to the same group of dequantising warps (parity waits)
-    int slots;            // A / token slots, at least 4 (the MMAs complete in order, so a group is never two uses ahead)
+    int a_slots;          // A slots in tensor memory, at least `groups` (the MMAs complete in order, so a group is never two uses ahead)
+    int slots;            // token slots, and barriers of a step; at least a_slots.  Both even: an issuing thread has its own slots
     int x_mem;            // token slots that have memory: `slots`, or the steps of a short K range
     int part_offset;      // K split: byte offset of the partials in shared memory; 0 = on top of the rings
     int acc2_col, a_col;  // second accumulator; first column of the A slots
@@ -167,7 +177,7 @@ template <int MODE>
 __global__ void __launch_bounds__(kStThreads, 1) gemm_w4a16_tc_stream_kernel(const __grid_constant__ StreamArgs a) {
     extern __shared__ uint8_t smem_raw_base[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw_base) + 1023) & ~uintptr_t(1023));
-    const int T = a.p.T, NS = a.p.slots, SR = a.p.raw_slots, K = a.K;
+    const int T = a.p.T, NS = a.p.slots, NA = a.p.a_slots, SR = a.p.raw_slots, K = a.K;
     const int x_box = T * 128, x_bytes = 2 * x_box;      // a step's tokens: two boxes of 64 k
     uint8_t* s_x = smem;
     uint8_t* s_raw = s_x + a.p.x_mem * x_bytes;
@@ -181,8 +191,7 @@ __global__ void __launch_bounds__(kStThreads, 1) gemm_w4a16_tc_stream_kernel(con
     const uint32_t accum_full = bar0 + 8u * (kBars - 2), part_full = bar0 + 8u * (kBars - 1);
     uint32_t* s_tmem = reinterpret_cast<uint32_t*>(s_bar + kBars);
     volatile int* s_abort = reinterpret_cast<volatile int*>(s_tmem + 1);
-    int* s_issued = reinterpret_cast<int*>(s_tmem + 2);           // steps whose copies were issued: weights, tokens
-    __half* s_scale = reinterpret_cast<__half*>(s_tmem + 4);      // [step][128 rows]
+    int* s_issued = reinterpret_cast<int*>(s_tmem + 2);          // steps whose weights were asked for
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     int t = 0, tile = blockIdx.x;
@@ -193,33 +202,31 @@ __global__ void __launch_bounds__(kStThreads, 1) gemm_w4a16_tc_stream_kernel(con
     const int n0 = tile * kTileRows, rows_t = a.rows[t], m0 = blockIdx.y * T;
     // K range: whole steps, spread over the cluster as evenly as they go
     const int ksplit = a.p.ksplit, krank = static_cast<int>(blockIdx.z);
-    const int G = K / kGroup, per = G / ksplit, rest = G - per * ksplit;
+    const int G = K / kGroup, per = a.p.steps_each, rest = G - per * ksplit;
     const int st0 = krank * per + min(krank, rest), nst = per + (krank < rest ? 1 : 0);
 
-    // The group scales of the 128 rows are the first loads: behind the weight stream they would arrive last.
-    constexpr int kScaleRegs = 4;
-    const __half* sc = a.scales[t];
-    auto load_scale = [&](int idx) -> __half {
-        const int rr = idx / nst, g = idx - rr * nst, row = n0 + rr;
-        return row < rows_t ? __ldg(sc + static_cast<size_t>(row) * G + st0 + g) : __half(0.0f);
+    const int r = (warp & 3) * 32 + lane, group = warp >> 2;      // dequantising warps: weight row = TMEM lane, first step
+    // Scales of this thread's next two steps, straight into registers: the first loads, since behind the weight stream they would arrive
+    // last.  (Through shared memory they cost a division per value, a block barrier and 0.4 us of a launch's start.)
+    const bool row_ok = n0 + r < rows_t;
+    const unsigned short* scale_row = reinterpret_cast<const unsigned short*>(a.scales[t]) + (row_ok ? static_cast<size_t>(n0 + r) * G + st0 : 0);
+    auto load_scale = [&](int s) -> unsigned short {
+        unsigned short v = 0;
+        if (row_ok && s < nst) v = __ldg(scale_row + s);
+        return v;
     };
-    auto store_scale = [&](int idx, __half v) {
-        const int rr = idx / nst, g = idx - rr * nst;
-        s_scale[g * kTileRows + rr] = v;
-    };
-    __half sreg[kScaleRegs];
+    unsigned short sc_a = 0, sc_b = 0;
     if (warp < kStDqWarps) {
-#pragma unroll
-        for (int q = 0; q < kScaleRegs; ++q)
-            if (tid + q * kStDqThreads < kTileRows * nst) sreg[q] = load_scale(tid + q * kStDqThreads);
-    } else if (warp == kStDqWarps + 1) {
+        sc_a = load_scale(group);
+        sc_b = load_scale(group + kStGroups);
+    } else if (warp == kStWeightWarp) {
         // barriers (a lane each), then the ring of packed weights
-        if (lane == 0) { tma_prefetch_desc(&a.tmap_w[t]); *s_abort = 0; s_issued[0] = min(SR, nst); s_issued[1] = 0; }
-        if (lane == 1) tma_prefetch_desc(&a.tmap_x);
+        if (lane == 30) { tma_prefetch_desc(&a.tmap_w[t]); *s_abort = 0; *s_issued = min(SR, nst); }
+        if (lane == 29) tma_prefetch_desc(&a.tmap_x);
         if (lane < SR) { mbar_init(raw_full(lane), 1); mbar_init(raw_empty(lane), 4); }
         if (lane < NS) { mbar_init(full(lane), 4 + 1); mbar_init(empty(lane), 1); }
         if (lane == 31) {
-            mbar_init(accum_full, 1);
+            mbar_init(accum_full, kStIssuers);
             mbar_init(part_full, 1);
             const int mine = max(0, min(a.p.tpr, T - krank * a.p.tpr));
             if (ksplit > 1) mbar_arrive_expect_tx(part_full, static_cast<uint32_t>(ksplit * mine * kTileRows * 4));
@@ -227,8 +234,11 @@ __global__ void __launch_bounds__(kStThreads, 1) gemm_w4a16_tc_stream_kernel(con
         fence_barrier_init();
         fence_proxy_async_smem();
         __syncwarp();
-        if (lane == 0) {
+        // (only announced: this warp goes on to the weights)
+        asm volatile("bar.arrive 2, %0;" ::"n"(kStThreads) : "memory");
+        if (elect_one()) {
             const int first = min(SR, nst);
+#pragma unroll 1
             for (int i = 0; i < first; ++i) {
                 mbar_arrive_expect_tx(raw_full(i), kStRawBytes);
                 tma_load_2d(smem_u32(s_raw + i * kStRawBytes), &a.tmap_w[t], (st0 + i) * 64, n0, raw_full(i));
@@ -243,33 +253,31 @@ __global__ void __launch_bounds__(kStThreads, 1) gemm_w4a16_tc_stream_kernel(con
         pdl_release_dependents();
     }
     tc_fence_before();
-    // (the loader only announces its barriers: it goes on to wait for the previous kernel, the others do not)
-    if (warp == kStDqWarps + 1) asm volatile("bar.arrive 2, %0;" ::"n"(kStThreads) : "memory");
-    else asm volatile("bar.sync 2, %0;" ::"n"(kStThreads) : "memory");
+    if (warp != kStWeightWarp) asm volatile("bar.sync 2, %0;" ::"n"(kStThreads) : "memory");
     tc_fence_after();
     const bool own_part = a.p.part_offset != 0;      // partials in memory of their own: they may come while the rings are in use
-    if (ksplit > 1 && own_part) cluster_arrive();
+    // (one warp has something to publish, the barriers; a release here would make the others wait for their scales: 0.7 us)
+    if (ksplit > 1 && own_part) {
+        if (warp == kStWeightWarp) cluster_arrive();
+        else asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
+    }
 
     if (warp < kStDqWarps) {
         const uint32_t tmem_base = *s_tmem;
-#pragma unroll
-        for (int q = 0; q < kScaleRegs; ++q)
-            if (tid + q * kStDqThreads < kTileRows * nst) store_scale(tid + q * kStDqThreads, sreg[q]);
-        for (int idx = tid + kScaleRegs * kStDqThreads; idx < kTileRows * nst; idx += kStDqThreads) store_scale(idx, load_scale(idx));
-        asm volatile("bar.sync 1, %0;" ::"n"(kStDqThreads) : "memory");
-
-        const int r = (warp & 3) * 32 + lane, part = warp >> 2;
         const uint32_t lane_base = tmem_base + (static_cast<uint32_t>((warp & 3) * 32) << 16);
         const int swz = (r >> 1) & 3;            // 64-byte swizzle: 16-byte chunk index xor row pair
         const uint8_t* raw_lane = s_raw + r * 64;
         bool ok = true;
-        int rs = part;                           // ring slot of this group's next step
+        int rs = group;                          // ring slot of this group's next step
         uint32_t rph = 0;
-        int slot = part;                         // A slot of the step, and the parity its previous use completes
+        int slot = group, aslot = group;         // the step's barrier and its A slot
+        int wslot = group + NS - NA;             // barrier of the step that had the A slot before, and the parity it completes
         uint32_t eph = 1;
         if (rs >= SR) { rs -= SR; rph ^= 1; }    // (SR is a multiple of 4: never for the first step)
-        for (int s = part; s < nst; s += kStGroups) {
-            const __half sc1 = s_scale[s * kTileRows + r];
+        for (int s = group; s < nst; s += kStGroups) {
+            const __half sc1 = __ushort_as_half(sc_a);
+            sc_a = sc_b;
+            sc_b = load_scale(s + 2 * kStGroups);
             ok = group_wait(raw_full(rs), rph, s_abort, lane);
             if (!ok) break;
             const uint8_t* raw_row = raw_lane + rs * kStRawBytes;
@@ -304,10 +312,10 @@ __global__ void __launch_bounds__(kStThreads, 1) gemm_w4a16_tc_stream_kernel(con
             }
             __syncwarp();
             if (lane == 0) mbar_arrive(raw_empty(rs));
-            ok = group_wait(empty(slot), eph, s_abort, lane);
+            ok = group_wait(empty(wslot), eph, s_abort, lane);
             if (!ok) break;
             tc_fence_after();
-            const uint32_t a_lane = lane_base + static_cast<uint32_t>(a.p.a_col + slot * kStACols);
+            const uint32_t a_lane = lane_base + static_cast<uint32_t>(a.p.a_col + aslot * kStACols);
             tmem_st32(a_lane, cols[0]);
             tmem_st32(a_lane + 32u, cols[1]);
             tmem_st_wait();
@@ -317,25 +325,28 @@ __global__ void __launch_bounds__(kStThreads, 1) gemm_w4a16_tc_stream_kernel(con
             rs += kStGroups;
             if (rs >= SR) { rs -= SR; rph ^= 1; }
             slot += kStGroups;
-            if (slot >= NS) { slot -= NS; eph ^= 1; }
+            if (slot >= NS) slot -= NS;
+            aslot += kStGroups;
+            if (aslot >= NA) aslot -= NA;
+            wslot += kStGroups;
+            if (wslot >= NS) { wslot -= NS; eph ^= 1; }
         }
         // ---------------- epilogue: thread = weight row, registers = tokens ----------------
         pdl_wait_prior_grids();                  // the previous kernels' reads of the outputs and writes of the residual
         const int n = n0 + r;
-        const bool row_ok = n < rows_t;
         if (ksplit == 1) {
             // eight tokens a round (a loop, not unrolled: this code runs once and its instructions have to be fetched)
             __half res[8];
-            stream_load_residual<MODE>(a, t, n, row_ok, m0 + part * 8, res);
+            stream_load_residual<MODE>(a, t, n, row_ok, m0 + group * 8, res);
             if (ok) ok = warp_wait(accum_full, 0, s_abort, lane);
             tc_fence_after();
             if (ok) {
 #pragma unroll 1
-                for (int c0 = part * 8; c0 < T; c0 += 32) {
+                for (int c0 = group * 8; c0 < T; c0 += 8 * kStGroups) {
                     float acc[8];
                     stream_load_acc(lane_base + static_cast<uint32_t>(c0), a.p.acc2_col, acc);
                     stream_store<MODE>(a, t, n, row_ok, m0 + c0, acc, res);
-                    if (c0 + 32 < T) stream_load_residual<MODE>(a, t, n, row_ok, m0 + c0 + 32, res);
+                    if (c0 + 8 * kStGroups < T) stream_load_residual<MODE>(a, t, n, row_ok, m0 + c0 + 8 * kStGroups, res);
                 }
             }
         } else {
@@ -344,14 +355,14 @@ __global__ void __launch_bounds__(kStThreads, 1) gemm_w4a16_tc_stream_kernel(con
             const int tpr = a.p.tpr;
             uint8_t* s_part = smem + a.p.part_offset;
             __half res[4];
-            stream_load_residual<MODE>(a, t, n, row_ok && part * 4 < tpr, m0 + krank * tpr + part * 4, res);
+            stream_load_residual<MODE>(a, t, n, row_ok && group * 4 < tpr, m0 + krank * tpr + group * 4, res);
             if (ok) ok = warp_wait(accum_full, 0, s_abort, lane);
             tc_fence_after();
             if (!own_part) cluster_arrive();     // this CTA's rings are free
             cluster_wait();
             const uint32_t part0 = smem_u32(s_part) + static_cast<uint32_t>(krank * (tpr / 4) * kTileRows + r) * 16u;
 #pragma unroll 1
-            for (int c0 = part * 8; c0 < T; c0 += 32) {
+            for (int c0 = group * 8; c0 < T; c0 += 8 * kStGroups) {
                 float v[8];
                 stream_load_acc(lane_base + static_cast<uint32_t>(c0), a.p.acc2_col, v);
 #pragma unroll
@@ -370,7 +381,7 @@ __global__ void __launch_bounds__(kStThreads, 1) gemm_w4a16_tc_stream_kernel(con
             if (!have && lane == 0) { *s_abort = 1; atomicAdd(&g_tc_wait_timeouts, 1u); }
             if (have) {
 #pragma unroll 1
-                for (int k = part * 4; k < tpr; k += 16) {
+                for (int k = group * 4; k < tpr; k += 4 * kStGroups) {
                     const int m = krank * tpr + k;
                     if (m >= T) break;
                     float acc[4] = {0.0f, 0.0f, 0.0f, 0.0f};
@@ -382,69 +393,70 @@ __global__ void __launch_bounds__(kStThreads, 1) gemm_w4a16_tc_stream_kernel(con
                         }
                     }
                     stream_store<MODE>(a, t, n, row_ok, m0 + m, acc, res);
-                    if (k + 16 < tpr) stream_load_residual<MODE>(a, t, n, row_ok, m0 + m + 16, res);
+                    if (k + 4 * kStGroups < tpr) stream_load_residual<MODE>(a, t, n, row_ok, m0 + m + 4 * kStGroups, res);
                 }
             }
         }
     } else {
-        if (warp == kStDqWarps) {
-            // ---------------- MMA issue: one thread ----------------
+        if (warp != kStWeightWarp && warp != kStTokenWarp) {
+            // ---------------- MMA issue: one thread, or one each for the even and the odd steps ----------------
             const uint32_t tmem_base = *s_tmem;
             if (elect_one()) {
+                const int first = warp == kStDqWarps ? 0 : 1;
                 const uint32_t idesc = make_idesc(T);
                 const uint64_t b_desc0 = make_smem_desc(smem_u32(s_x));
                 const uint32_t b_step = static_cast<uint32_t>(x_bytes) >> 4, b_half = static_cast<uint32_t>(x_box) >> 4;
-                int slot = 0;
+                int slot = first, aslot = first;
                 uint32_t ph = 0;
-                uint64_t b_desc = b_desc0;
-                uint32_t a_tmem = tmem_base + static_cast<uint32_t>(a.p.a_col);
-                bool ready = mbar_test_wait(full(0), 0);
-                for (int s = 0; s < nst; ++s) {
+                bool ready = mbar_test_wait(full(slot), 0);
+                for (int s = first; s < nst; s += kStIssuers) {
                     if (!ready && !mbar_wait(full(slot), ph, s_abort)) break;
                     tc_fence_after();
                     const uint32_t bar_empty = empty(slot);
+                    const uint64_t b0 = b_desc0 + static_cast<uint32_t>(slot) * b_step;
+                    const uint32_t a0 = tmem_base + static_cast<uint32_t>(a.p.a_col + aslot * kStACols);
+                    aslot += kStIssuers;
+                    if (aslot >= NA) aslot -= NA;
+                    slot += kStIssuers;
+                    if (slot >= NS) { slot -= NS; ph ^= 1; }
+                    ready = mbar_test_wait(full(slot), ph);      // the answer arrives while the MMAs below are issued
                     const uint32_t tmem_d = tmem_base + ((s & 1) != 0 ? static_cast<uint32_t>(a.p.acc2_col) : 0u);
 #pragma unroll
                     for (int ks = 0; ks < kGroup / 16; ++ks)
-                        tc_mma_f16_ts(tmem_d, a_tmem + 8u * ks, b_desc + (ks >= 4 ? b_half : 0u) + static_cast<uint32_t>(2 * (ks & 3)), idesc,
+                        tc_mma_f16_ts(tmem_d, a0 + 8u * ks, b0 + (ks >= 4 ? b_half : 0u) + static_cast<uint32_t>(2 * (ks & 3)), idesc,
                                       (ks != 0 || s >= 2) ? 1u : 0u);
                     tc_commit(bar_empty);
-                    a_tmem += kStACols;
-                    b_desc += b_step;
-                    if (++slot == NS) { slot = 0; ph ^= 1; b_desc = b_desc0; a_tmem = tmem_base + static_cast<uint32_t>(a.p.a_col); }
-                    ready = mbar_test_wait(full(slot), ph);
                 }
                 tc_commit(accum_full);   // also after a wait that ran out: nothing may be in flight at the end
             }
-        } else if (lane == 0) {
-            // ---------------- loader: tokens as soon as the previous kernel is through, then both rings as they empty ----------------
-            int iw = min(SR, nst), ix = 0, ws = 0, xs = 0;
-            uint32_t wph = 0, xph = 0;
-            pdl_wait_prior_grids();
-            for (unsigned spins = 0; iw < nst || ix < nst;) {
-                bool moved = false;
-                if (ix < nst && (ix < NS || mbar_test_wait(empty(xs), xph))) {
-                    mbar_arrive_expect_tx(full(xs), static_cast<uint32_t>(x_bytes));
-                    tma_load_2d(smem_u32(s_x + xs * x_bytes), &a.tmap_x, (st0 + ix) * kGroup, m0, full(xs));
-                    tma_load_2d(smem_u32(s_x + xs * x_bytes + x_box), &a.tmap_x, (st0 + ix) * kGroup + kBK, m0, full(xs));
-                    if (++xs == NS) { xs = 0; if (ix >= NS) xph ^= 1; }
-                    ++ix;
-                    moved = true;
+        } else if (warp == kStWeightWarp) {
+            // ---------------- packed weights, as the ring empties ----------------
+            if (elect_one()) {
+                int i = min(SR, nst), slot = 0;
+                uint32_t ph = 0;
+#pragma unroll 1
+                for (; i < nst; ++i) {
+                    if (!mbar_wait(raw_empty(slot), ph, s_abort)) break;
+                    mbar_arrive_expect_tx(raw_full(slot), kStRawBytes);
+                    tma_load_2d(smem_u32(s_raw + slot * kStRawBytes), &a.tmap_w[t], (st0 + i) * 64, n0, raw_full(slot));
+                    if (++slot == SR) { slot = 0; ph ^= 1; }
                 }
-                if (iw < nst && mbar_test_wait(raw_empty(ws), wph)) {
-                    mbar_arrive_expect_tx(raw_full(ws), kStRawBytes);
-                    tma_load_2d(smem_u32(s_raw + ws * kStRawBytes), &a.tmap_w[t], (st0 + iw) * 64, n0, raw_full(ws));
-                    if (++ws == SR) { ws = 0; wph ^= 1; }
-                    ++iw;
-                    moved = true;
-                }
-                if (moved) { spins = 0; continue; }
-                if (*s_abort) break;
-                if (++spins > 2048) __nanosleep(64);
-                if (spins > kWaitLimit) { *s_abort = 1; atomicAdd(&g_tc_wait_timeouts, 1u); break; }
+                *s_issued = i;
             }
-            s_issued[0] = iw;
-            s_issued[1] = ix;
+        } else if (elect_one()) {
+            // ---------------- tokens, as soon as the previous kernel is through ----------------
+            int i = 0, slot = 0;
+            uint32_t ph = 1;
+            pdl_wait_prior_grids();
+#pragma unroll 1
+            for (; i < nst; ++i) {
+                if (i >= NS && !mbar_wait(empty(slot), ph, s_abort)) break;
+                const uint32_t dst = smem_u32(s_x + slot * x_bytes), bar = full(slot);
+                mbar_arrive_expect_tx(bar, static_cast<uint32_t>(x_bytes));
+                tma_load_2d(dst, &a.tmap_x, (st0 + i) * kGroup, m0, bar);
+                tma_load_2d(dst + x_box, &a.tmap_x, (st0 + i) * kGroup + kBK, m0, bar);
+                if (++slot == NS) { slot = 0; ph ^= 1; }
+            }
         }
         __syncwarp();
         if (ksplit > 1) {
@@ -456,7 +468,7 @@ __global__ void __launch_bounds__(kStThreads, 1) gemm_w4a16_tc_stream_kernel(con
     __syncthreads();
     if (*s_abort) {          // a bounded wait ran out: what is in flight has to land before the memory goes (bounded too)
         if (tid == 0) {
-            for (int i = 0; i < min(SR, s_issued[0]); ++i) wait_regardless(raw_full(i), static_cast<uint32_t>((s_issued[0] - 1 - i) / SR) & 1u, kWaitLimit);
+            for (int i = 0; i < min(SR, *s_issued); ++i) wait_regardless(raw_full(i), static_cast<uint32_t>((*s_issued - 1 - i) / SR) & 1u, kWaitLimit);
             wait_regardless(accum_full, 0, kWaitLimit);
             __nanosleep(100000);     // token copies whose slot never filled up have no barrier phase of their own to wait for
         }
@@ -466,24 +478,31 @@ __global__ void __launch_bounds__(kStThreads, 1) gemm_w4a16_tc_stream_kernel(con
 }
 
 // ---- host side of the streaming form ----
-// Ring sizes for token tiles of T and K split `ksplit` ways, `steps` steps each at most.  False where it does not fit.
-bool plan_stream(int T, int ksplit, int steps, StreamPlan* a) {
+// Ring sizes for token tiles of T and the `all_steps` steps of K split `ksplit` ways.  False where it does not fit.
+bool plan_stream(int T, int ksplit, int all_steps, StreamPlan* a) {
+    const int steps = (all_steps + ksplit - 1) / ksplit;
     a->T = T;
     a->ksplit = ksplit;
-    a->slots = T <= 64 ? 6 : 4;
+    a->steps_each = all_steps / ksplit;
     a->acc2_col = T <= 64 ? 64 : 128;
     a->a_col = 2 * a->acc2_col;
+    a->a_slots = T <= 64 ? 6 : 4;
     a->tpr = ((T + a->ksplit - 1) / a->ksplit + 3) & ~3;
     const size_t part_bytes = a->ksplit > 1 ? static_cast<size_t>(a->ksplit) * a->tpr * kTileRows * 4 : 0;
     const size_t budget = 226 * 1024;
-    const size_t fixed = 1024 + (2 * kStMaxRaw + 2 * kStMaxSlots + 2) * 8 + 16 + static_cast<size_t>(steps) * kTileRows * 2;
-    for (; a->slots >= 4; a->slots -= 2) {
+    const size_t fixed = 1024 + (2 * kStMaxRaw + 2 * kStMaxSlots + 2) * 8 + 16;
+    // As many token slots as fit beside a whole ring of weights: every slot that does not have to be waited for is asked for at once.
+    const int all_raw = std::min(kStMaxRaw, (steps + kStGroups - 1) / kStGroups * kStGroups);
+    a->slots = std::max(a->a_slots, std::min(kStMaxSlots, (steps + 1) & ~1));
+    while (a->slots > a->a_slots && fixed + part_bytes + 128 + static_cast<size_t>(a->slots) * T * 256 + static_cast<size_t>(all_raw) * kStRawBytes > budget) a->slots -= 2;
+    for (; a->slots >= kStGroups; a->slots -= 2) {
+        a->a_slots = std::min(a->a_slots, a->slots);
         a->x_mem = std::min(a->slots, steps);
         const size_t x_bytes = static_cast<size_t>(a->x_mem) * T * 256;
         for (int own = part_bytes ? 1 : 0; own >= 0; --own) {
             const size_t extra = own ? part_bytes + 128 : 0;
-            int raw = std::min(kStMaxRaw, (steps + 3) & ~3);
-            while (raw > 4 && fixed + extra + x_bytes + static_cast<size_t>(raw) * kStRawBytes > budget) raw -= 4;
+            int raw = all_raw;
+            while (raw > kStGroups && fixed + extra + x_bytes + static_cast<size_t>(raw) * kStRawBytes > budget) raw -= kStGroups;
             const size_t ring = x_bytes + static_cast<size_t>(raw) * kStRawBytes;
             if (fixed + extra + ring > budget) continue;
             if (!own && ring < part_bytes) continue;     // the partials go on top of the rings
@@ -491,8 +510,7 @@ bool plan_stream(int T, int ksplit, int steps, StreamPlan* a) {
             const size_t used = (fixed - 1024 + ring + 127) / 128 * 128;
             a->part_offset = own ? static_cast<int>(used) : 0;
             // At least half an SM, so that no SM ever holds two of these CTAs: each takes all columns of tensor memory, and the
-            // second would sit in its allocation.  Today the registers (576 threads x 96) rule that out already and the floor
-            // costs nothing (one layer at 47 / 115 tokens: 30.0 / 37.2 us with and without it).
+            // second would sit in its allocation.  (Today the registers rule that out already.)
             a->smem = std::max<size_t>(1024 + used + (own ? part_bytes : 0), 116 * 1024);
             return true;
         }

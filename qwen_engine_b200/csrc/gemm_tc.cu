@@ -285,33 +285,38 @@ bool gemm_tc_supported(const GemmArgs& g) {
 
 namespace {
 // The streaming kernel's cut of a shape: token tiles and K slices, two steps each at least, within one CTA per SM where that is
-// possible.  The cut is chosen by what a CTA has to do, in cycles: 400 a step of dequantisation or 4 T of MMA, whichever is
-// longer; the exchange of partials at 18 bytes a cycle after its latency; 25 a token for the epilogue.  What a launch takes (the
-// plan's cost) is more than that: 8.6 T a step, the token tile's way from L2 (measured at 128 tokens, 96 CTAs: 0.58 us a
-// step), and 5500 of start and end, for every wave of CTAs.
+// possible, by the time it is estimated to take, in cycles of 1.9 GHz.  The constants are fitted to 2200 timed cuts of 14
+// shapes (512 x 512 to 17920 x 1536 and 1536 x 8960) at 4 to 1024 tokens, launches one behind another (the cut they choose is on
+// average 1.4 % slower than the best one; the former rule's 3.2 %).  The first steps hide behind the launch; a step is 400 of
+// dequantisation, 650 beyond what the token slots hold, or 6 a token of its tile's way from L2; 35 a token of the tile for the
+// epilogue; the exchange of a K split 1100 and 66 a token sent; CTAs on more than half of the SMs keep the next launch's from
+// starting early; a further wave costs its launch again.
+double stream_cost(int T, int split, int steps, int ctas, int sm_count) {
+    const int per = (steps + split - 1) / split, waves = (ctas + sm_count - 1) / sm_count;
+    const double work = std::max(0, std::min(per, 12) - 2) * std::max(400.0, 6.0 * T) + std::max(0, per - 12) * std::max(650.0, 6.0 * T) + 35.0 * T / split;
+    const double exchange = split > 1 ? 1100.0 + 66.0 * T * (split - 1) / split : 0.0;
+    const double crowd = 3100.0 * std::min(1.0, std::max(0.0, 2.0 * ctas / sm_count - 1.0));
+    return 4700.0 + waves * work + exchange + crowd + 3200.0 * (waves - 1);
+}
 template <int MODE>
 StreamPlan stream_plan(int M, int K, int tiles, int sm_count) {
     static PlanCache<StreamPlan> plans;
     return plans.get(plan_key(MODE, M, K, tiles), [&] {
         const int steps = K / kGroup;
         StreamPlan best;
-        double best_work = 0;
         const int ts_min = (M + 127) / 128, ts_max = (M + 15) / 16;
         for (int ts = ts_min; ts <= ts_max; ++ts) {
             const int T = ((M + ts - 1) / ts + 15) & ~15;
             if (ts > ts_min && static_cast<long long>(tiles) * ts > sm_count) break;
             if (ts > ts_min && (M + T - 1) / T != ts) continue;
             for (int split = std::max(1, std::min({kStMaxSplit, sm_count / (tiles * ts), steps / 2})); split >= 1; --split) {
-                const int per = (steps + split - 1) / split, waves = (tiles * ts * split + sm_count - 1) / sm_count;
-                const double ends = split > 1 ? 1500.0 + T * 512.0 * (split - 1) / split / 18.0 + 25.0 * T / split : 25.0 * T;
-                const double work = per * std::max(400.0, 4.0 * T) + ends;
-                if (best.smem != 0 && work >= best_work) continue;
+                const double cost = stream_cost(T, split, steps, tiles * ts * split, sm_count);
+                if (best.smem != 0 && cost >= best.cost) continue;
                 StreamPlan p;
                 if (!plan_stream(T, split, steps, &p)) continue;
                 if (split > 1 && max_active_clusters(reinterpret_cast<const void*>(gemm_w4a16_tc_stream_kernel<MODE>), kStThreads, p.smem, split) < tiles * ts) continue;
                 best = p;
-                best.cost = waves * (5500.0 + per * std::max(450.0, 8.6 * T) + ends);
-                best_work = work;
+                best.cost = cost;
             }
         }
         return best;

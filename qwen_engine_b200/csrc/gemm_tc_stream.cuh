@@ -220,16 +220,17 @@ __global__ void __launch_bounds__(kStThreads, 1) gemm_w4a16_tc_stream_kernel(con
         sc_a = load_scale(group);
         sc_b = load_scale(group + kStGroups);
     } else if (warp == kStWeightWarp) {
-        // barriers (a lane each), then the ring of packed weights
-        if (lane == 30) { tma_prefetch_desc(&a.tmap_w[t]); *s_abort = 0; *s_issued = min(SR, nst); }
-        if (lane == 29) tma_prefetch_desc(&a.tmap_x);
-        if (lane < SR) { mbar_init(raw_full(lane), 1); mbar_init(raw_empty(lane), 4); }
-        if (lane < NS) { mbar_init(full(lane), 4 + 1); mbar_init(empty(lane), 1); }
-        if (lane == 31) {
-            mbar_init(accum_full, kStIssuers);
-            mbar_init(part_full, 1);
+        // barriers (three a lane, without a branch), then the ring of packed weights
+#pragma unroll
+        for (int i = lane; i < (kBars + 31) / 32 * 32; i += 32) {
+            const int count = i < kStMaxRaw ? 1 : i < 2 * kStMaxRaw ? 4 : i < 2 * kStMaxRaw + kStMaxSlots ? 4 + 1 : i == kBars - 2 ? kStIssuers : 1;
+            if (i < kBars) mbar_init(bar0 + 8u * i, count);
+        }
+        if (lane == (kBars - 1) % 32) {
             const int mine = max(0, min(a.p.tpr, T - krank * a.p.tpr));
             if (ksplit > 1) mbar_arrive_expect_tx(part_full, static_cast<uint32_t>(ksplit * mine * kTileRows * 4));
+            *s_abort = 0;
+            *s_issued = min(SR, nst);
         }
         fence_barrier_init();
         fence_proxy_async_smem();
@@ -245,7 +246,11 @@ __global__ void __launch_bounds__(kStThreads, 1) gemm_w4a16_tc_stream_kernel(con
             }
         }
         __syncwarp();
-    } else if (warp == kStDqWarps) {
+    } else if (warp == kStTokenWarp) {
+        if (elect_one()) tma_prefetch_desc(&a.tmap_x);
+    } else if (warp == kStTokenWarp + 1) {
+        if (elect_one()) tma_prefetch_desc(&a.tmap_w[t]);
+    } else {
         // Blocks while a CTA of the previous launch on this SM holds it; the next launch may only follow once every CTA of
         // this one has its share, or a CTA of the next could take it first and wait for this launch with it.
         tmem_alloc(smem_u32(s_tmem), 512);

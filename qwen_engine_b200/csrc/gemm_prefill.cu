@@ -167,16 +167,14 @@ int gemm_launch(GemmArgs g, cudaStream_t stream) {
     const DeviceInfo* dev = nullptr;
     if (int st = ensure_device_ready(&dev)) return st;
 
-    // The tcgen05 kernel pads the token count to its smallest tile (16), so below a handful of tokens the CUDA-core
-    // few-token form (the decode GEMV's memory behaviour with fp16 arithmetic) is the faster one: 3 tokens where K > 4096
-    // (down: the few-token form stages only two tokens per pass there), 4 on matrices tall enough to give every SM a CTA of
-    // their own (gate_up), 7 on the narrow K <= 4096 shapes (QKV, O).  These lines were measured against the tcgen05 kernel
-    // in front of the streaming one; against that the two forms meet earlier (CUDA cores / tcgen05, us: down 10.6 / 7.3 and
-    // gate_up 8.2 / 8.1 at 2 tokens, O 5.4 / 4.0 and QKV 4.4 / 4.8 at 4).  Only shapes that the mma form below refuses come
-    // here with 2 tokens or more.  The CUDA-core forms also take what TMA cannot address.
+    // The tcgen05 kernel pads the token count to its smallest tile (16), so for shapes that the mma form below refuses the CUDA-core
+    // form (the decode GEMV's memory behaviour with fp16 arithmetic) is the faster one at the fewest tokens: up to 3 on the narrow
+    // K <= 4096 shapes (QKV, O), one where K > 4096 (the few-token form stages only two tokens per pass there) or where the matrix
+    // gives every SM a CTA of its own.  CUDA cores / tcgen05, us: down 10.6 / 5.6 and gate_up 8.2 / 6.3 at 2 tokens, 8192 x 8192
+    // 80 / 13 at 2, O 5.4 / 3.7 and QKV 4.4 / 3.8 at 4 (3.6 / 3.8 at 2).  The CUDA-core forms also take what TMA cannot address.
     const int tc_min_m_opt = option(W4A16_OPT_GEMM_MIN_TOKENS_TENSOR_CORE);
     const int rows_all = g.rows[0] + (g.mode == kQkv ? g.rows[1] + g.rows[2] : 0);
-    const int tc_min_m = tc_min_m_opt > 0 ? tc_min_m_opt : (g.K > 4096 ? 3 : (rows_all >= 64 * dev->sm_count ? 4 : 7));
+    const int tc_min_m = tc_min_m_opt > 0 ? tc_min_m_opt : (g.K > 4096 || rows_all >= 64 * dev->sm_count ? 2 : 4);
     SmallMArgs a;
     a.g = g;
     const int total_rows = g.rows[0] + (g.mode == kQkv ? g.rows[1] + g.rows[2] : 0);
@@ -189,10 +187,15 @@ int gemm_launch(GemmArgs g, cudaStream_t stream) {
     bool aligned = reinterpret_cast<uintptr_t>(g.x) % 16 == 0;
     for (int t = 0; t < (g.mode == kQkv ? 3 : 1); ++t) aligned = aligned && reinterpret_cast<uintptr_t>(g.qweight[t]) % 16 == 0;
 
-    // Two to sixteen tokens: the weight-streaming kernel with the warp-level MMA (no fixed tcgen05 costs).  Rows in whole groups
-    // of 16 (a group of QKV rows from one tensor).
+    // A few tokens: the weight-streaming kernel with the warp-level MMA (no fixed tcgen05 costs).  Rows in whole groups of 16 (a
+    // group of QKV rows from one tensor).  One token tile of 8 on all but the largest matrices, two on the smallest ones only.  mma /
+    // tcgen05, us, each behind itself: at 4 tokens QKV 2.9 / 3.8, down 5.5 / 5.6, gate_up 6.5 / 6.3 (but a layer of all four
+    // 17.8 / 19.8, since CTAs of two launches share an SM in the mma form), 17920 x 2048 7.8 / 7.5, 8192 x 8192 13.0 / 13.0; at 9
+    // 2048 x 512 2.9 / 3.5, QKV 4.4 / 3.8, gate_up 7.6 / 6.4; at 16 QKV 4.5 / 3.4, O 4.1 / 3.7, gate_up 8.2 / 5.9, down 8.0 / 5.7, the
+    // layer 23.6 / 19.1.
+    const size_t weights = static_cast<size_t>(rows_all) * g.K;
     const int mma_max_opt = option(W4A16_OPT_GEMM_MMA_MAX_TOKENS);
-    const int mma_max_m = mma_max_opt > 0 ? mma_max_opt : 16;
+    const int mma_max_m = mma_max_opt > 0 ? mma_max_opt : (weights <= 2u << 20 ? 16 : weights <= 32u << 20 ? 8 : 1);
     const bool whole_groups = a.units % (g.mode == kSwiglu ? 8 : 16) == 0 && (g.mode != kQkv || (g.rows[0] % 16 == 0 && g.rows[1] % 16 == 0 && g.rows[2] % 16 == 0));
     bool scale_pairs = true;
     for (int t = 0; t < (g.mode == kQkv ? 3 : 1); ++t) scale_pairs = scale_pairs && reinterpret_cast<uintptr_t>(g.scales[t]) % 4 == 0;

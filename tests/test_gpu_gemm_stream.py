@@ -59,3 +59,14 @@ def test_stream_kernel_swiglu_and_qkv_routing(M):
     ref64, _ = oracle.gemm_prefill(qw, sc, x, m_idx, n_idx)
     got = np.concatenate([util.to_np(p[2]) for p in qkv], axis=1)
     util.assert_fp16_close(got[np.ix_(m_idx, n_idx)], ref64, what="qkv")
+
+
+@pytest.mark.parametrize("M,N,K,scale_max,res", [
+    # token counts that come to it from the few-token forms: 9 to 16, 2 on long K, 4 on rows that are no whole groups of 16
+    (9, 1536, 1536, 0.02, True), (16, 17920, 1536, 0.5, False), (13, 2048, 8960, 0.02, True), (2, 264, 8192, 0.02, False),
+    (4, 130, 512, 0.07, True), (3, 8200, 8192, 0.02, False),
+    # one more step than token slots, steps beyond both rings, an odd number of steps in a CTA (two issuing threads)
+    (40, 20000, 1792, 0.02, False), (33, 19000, 3328, 0.5, True), (64, 19100, 1792, 0.02, False), (47, 384, 8960, 0.02, True),
+])
+def test_stream_kernel_few_tokens_and_ring_lengths(M, N, K, scale_max, res):
+    test_stream_kernel_matches_oracle(M, N, K, scale_max, res)

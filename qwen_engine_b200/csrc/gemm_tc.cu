@@ -395,7 +395,7 @@ int pair_launch(const GemmArgs& g, int sm_count, cudaStream_t stream) {
         return W4A16_ERR_INVALID_ARG;
     // persistent: one pair per two SMs, each walking the pair tiles p, p + P, ...
     const int grid = 2 * std::min(pairs, n_pairs * ((g.M + T - 1) / T));
-    const size_t smem = tc_pair_smem_bytes(T);
+    const size_t smem = tc_pair_smem_bytes(g.mode, T);
     auto launch = [&](auto* kernel) {
         return static_cast<int>(launch_kernel_cluster(kernel, dim3(grid), dim3(kPairThreads), smem, stream, pdl_enabled(), dim3(2, 1, 1), a));
     };

@@ -9,33 +9,36 @@
 // What bounds it: the tensor pipe on long K (28672 x 8192), the work around a tile on short K (K = 1536 gives 12 steps per
 // tile).  So the epilogue has warps of its own, and tensor memory holds two accumulators of up to 128 token columns: a tile
 // of up to 128 tokens uses one of them in turn with the next tile's, a larger one both as its two halves.  The epilogue
-// takes a half into registers and gives it back at once, and the MMAs of the next tile's first half run ahead meanwhile.
+// takes a half into registers (SWIGLU: the second one into shared memory) and gives it back at once, and the MMAs of the next
+// tile's first half run ahead meanwhile.
 // The rest of tensor memory are four A slots of one step.  Arrivals on the leader's barriers carry no cluster-scope release:
 // with one the peer's dequantising warps waited for their own prefetched loads at every step (1400 cycles a step, 930 of
 // them for nothing).
 //
-//   warps 0..7  : dequantise; group g = warp / 4 takes the steps g, g + 2, ...  A step is in registers as fp16 before its
-//                 slot is free, so a slot is refilled one store after the MMA that read it.
+//   warps 0..7  : dequantise; group g = warp / 4 takes the steps g, g + 2, ...  A quarter of a step is in registers as fp16
+//                 before its slot is free, the rest is stored as it comes.  (The whole step in registers took 88 of them, by
+//                 setmaxnreg, and spilled; with 72 for every warp and no spills gate_up at 300 / 1024 / 4096 tokens
+//                 23.8 -> 22.4, 48.2 -> 47.1, 184 -> 179 us, 8192 x 8192 at 1024 104 -> 102.)
 //   warps 8..23 : epilogue, 128 rows of a finished accumulator (four warps per 32 rows, a quarter of the tokens each)
 //   warp 24     : tensor memory; in the leading CTA one thread issues the MMAs
 //   warp 25     : TMA of the packed weights, 128 rows x 128 k per slot (private ring, before the wait for the previous kernel)
 //   warp 26     : TMA of this CTA's half of the token tile, T / 2 x 128 k per slot
-//   warp 27     : none (whole warpgroups, for the register split)
 //
 // Synchronisation: one "full" barrier per slot in the leader counts the dequantising warps of both CTAs and the bytes
 // of both token halves; one "done" barrier per slot in both CTAs (tcgen05.commit with a CTA mask) frees the A slot and
 // the token slot.  Two "accumulator full" barriers in both CTAs, two "accumulator empty" ones in the leader.
 constexpr int kPairGroups = 2;
 constexpr int kPairDqWarps = 4 * kPairGroups, kPairEpiWarps = 16;
-constexpr int kPairThreads = (kPairDqWarps + kPairEpiWarps + 4) * 32;
+constexpr int kPairThreads = (kPairDqWarps + kPairEpiWarps + 3) * 32;
 constexpr int kPairAccCols = 128;            // one accumulator
 constexpr int kPairACol = 2 * kPairAccCols, kPairACols = kGroup / 2;   // A slots behind the two accumulators
 constexpr int kPairSlots = 4;                // A and token slots; a multiple of the groups (parity waits)
-constexpr int kPairRawSlots = 8;             // packed weights; likewise
+constexpr int kPairMaxRaw = 8;               // packed weights; likewise
 constexpr int kPairRawBytes = kTileRows * 64;
-// Registers a thread: 72 at launch (28 warps), then by role; the sum over the warps stays what was launched with.
-constexpr int kPairRegsLaunch = 72, kPairRegsDq = 88, kPairRegsEpi = 64, kPairRegsRest = 72;
-static_assert(kPairDqWarps * kPairRegsDq + kPairEpiWarps * kPairRegsEpi + 4 * kPairRegsRest <= (kPairThreads / 32) * kPairRegsLaunch, "register split");
+constexpr int kPairParkBytes = kPairEpiWarps * 32 * (kPairAccCols / 4) * 4;    // an accumulator in shared memory
+// SWIGLU parks the second accumulator of a tile (see the epilogue); its 64 KB are taken from the ring of packed weights.
+constexpr bool pair_parks(int mode) { return mode == kSwiglu; }
+constexpr int pair_raw_slots(int mode) { return pair_parks(mode) ? 4 : kPairMaxRaw; }
 
 struct PairArgs {
     CUtensorMap tmap_w[3];
@@ -145,7 +148,8 @@ __device__ __forceinline__ void pair_exchange8(int odd, const uint32_t (&v)[8], 
 enum PairStore { kStoreValues = 0, kStoreWords = 1, kStoreWordsPeers = 2 };
 template <int MODE, int STORE>
 __global__ void __launch_bounds__(kPairThreads, 1) gemm_w4a16_tc_pair_kernel(const __grid_constant__ PairArgs a) {
-    constexpr bool WORDS = STORE != kStoreValues;
+    constexpr bool WORDS = STORE != kStoreValues, PARK = pair_parks(MODE);
+    constexpr int kRawSlots = pair_raw_slots(MODE);
     constexpr int kEpi0 = kPairDqWarps, kMmaWarp = kEpi0 + kPairEpiWarps, kRawWarp = kMmaWarp + 1;
     extern __shared__ uint8_t smem_raw_base[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw_base) + 1023) & ~uintptr_t(1023));
@@ -153,15 +157,16 @@ __global__ void __launch_bounds__(kPairThreads, 1) gemm_w4a16_tc_pair_kernel(con
     const int b_box = (NH / 2) * 128, b_bytes = 2 * H * b_box;      // [accumulator][64 k]: half of each accumulator's tokens
     uint8_t* s_b = smem;
     uint8_t* s_raw = s_b + kPairSlots * b_bytes;
-    uint64_t* s_bar = reinterpret_cast<uint64_t*>(s_raw + kPairRawSlots * kPairRawBytes);
+    uint8_t* s_park = s_raw + kRawSlots * kPairRawBytes;
+    uint64_t* s_bar = reinterpret_cast<uint64_t*>(s_park + (PARK && H == 2 ? kPairParkBytes : 0));
     const uint32_t bar0 = smem_u32(s_bar);
     auto raw_full = [&](int i) { return bar0 + 8u * i; };
-    auto raw_empty = [&](int i) { return bar0 + 8u * (kPairRawSlots + i); };
-    auto full = [&](int i) { return bar0 + 8u * (2 * kPairRawSlots + i); };
-    auto done = [&](int i) { return bar0 + 8u * (2 * kPairRawSlots + kPairSlots + i); };
-    auto acc_full = [&](int i) { return bar0 + 8u * (2 * kPairRawSlots + 2 * kPairSlots + i); };
-    auto acc_empty = [&](int i) { return bar0 + 8u * (2 * kPairRawSlots + 2 * kPairSlots + 2 + i); };
-    constexpr int kBars = 2 * kPairRawSlots + 2 * kPairSlots + 4;
+    auto raw_empty = [&](int i) { return bar0 + 8u * (kPairMaxRaw + i); };
+    auto full = [&](int i) { return bar0 + 8u * (2 * kPairMaxRaw + i); };
+    auto done = [&](int i) { return bar0 + 8u * (2 * kPairMaxRaw + kPairSlots + i); };
+    auto acc_full = [&](int i) { return bar0 + 8u * (2 * kPairMaxRaw + 2 * kPairSlots + i); };
+    auto acc_empty = [&](int i) { return bar0 + 8u * (2 * kPairMaxRaw + 2 * kPairSlots + 2 + i); };
+    constexpr int kBars = 2 * kPairMaxRaw + 2 * kPairSlots + 4;
     uint32_t* s_tmem = reinterpret_cast<uint32_t*>(s_bar + kBars);
     volatile int* s_abort = reinterpret_cast<volatile int*>(s_tmem + 1);
     volatile int* s_epi_ok = reinterpret_cast<volatile int*>(s_tmem + 2);
@@ -174,7 +179,7 @@ __global__ void __launch_bounds__(kPairThreads, 1) gemm_w4a16_tc_pair_kernel(con
     const int total_pt = n_pairs * ((a.M + T - 1) / T);
 
     if (warp == kRawWarp) {
-        if (lane < kPairRawSlots) { mbar_init(raw_full(lane), 1); mbar_init(raw_empty(lane), 4); }
+        if (lane < kPairMaxRaw) { mbar_init(raw_full(lane), 1); mbar_init(raw_empty(lane), 4); }
         // full: four dequantising warps of each CTA and the leader's expect_tx arrival
         if (lane < kPairSlots) { mbar_init(full(lane), 2 * 4 + 1); mbar_init(done(lane), 1); }
         if (lane < 2) { mbar_init(acc_full(lane), 1); mbar_init(acc_empty(lane), 2 * kPairEpiWarps); }
@@ -193,9 +198,6 @@ __global__ void __launch_bounds__(kPairThreads, 1) gemm_w4a16_tc_pair_kernel(con
     cluster_sync_all();              // the peer's barriers exist before anything arrives on them from here
     tc_fence_after();
     const uint32_t tmem_base = *s_tmem;
-    if (warp < kPairDqWarps) asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kPairRegsDq));
-    else if (warp < kMmaWarp) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kPairRegsEpi));
-    else asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kPairRegsRest));
 
     if (warp < kPairDqWarps) {
         // ================= dequantise: thread = weight row = tensor-memory lane =================
@@ -234,45 +236,39 @@ __global__ void __launch_bounds__(kPairThreads, 1) gemm_w4a16_tc_pair_kernel(con
             ok = group_wait(raw_full(rs), rph, s_abort, lane);
             if (!ok) break;
             const uint8_t* raw_row = s_raw + rs * kPairRawBytes + r * 64;
-            const __half2 sc2 = __half2half2(sc);
+            const __half2 sc2 = __half2half2(sc), k10 = __float2half2_rn(1024.0f);
+            const __half2 s20 = __hmul2(__hmul2(sc2, k10), k10), m8s = __hmul2(sc2, __float2half2_rn(-8.0f));
             const uint32_t a_slot = a_lane + static_cast<uint32_t>(slot * kPairACols);
+            auto slot_free = [&]() -> bool {
+                ok = group_wait(done(slot), dph, s_abort, lane);
+                tc_fence_after();
+                return ok;
+            };
             if (__all_sync(0xFFFFFFFFu, __habs(sc) < __float2half_rn(0.0624f))) {
-                const __half2 k10 = __float2half2_rn(1024.0f);
-                const __half2 s20 = __hmul2(__hmul2(sc2, k10), k10), m8s = __hmul2(sc2, __float2half2_rn(-8.0f));
-                uint32_t cols[2][32];
 #pragma unroll
                 for (int c = 0; c < 4; ++c) {
                     const uint4 w = *reinterpret_cast<const uint4*>(raw_row + ((c ^ swz) << 4));
-                    uint32_t* o = &cols[c >> 1][16 * (c & 1)];
+                    uint32_t o[16];
                     dequant_word_small_scale(w.x, s20, m8s, o);
                     dequant_word_small_scale(w.y, s20, m8s, o + 4);
                     dequant_word_small_scale(w.z, s20, m8s, o + 8);
                     dequant_word_small_scale(w.w, s20, m8s, o + 12);
+                    if (c == 0 && !slot_free()) break;
+                    tmem_st16(a_slot + 16u * c, o);
                 }
-                ok = group_wait(done(slot), dph, s_abort, lane);
-                if (!ok) break;
-                tc_fence_after();
-                tmem_st32(a_slot, cols[0]);
-                tmem_st32(a_slot + 32u, cols[1]);
-            } else {
-                ok = group_wait(done(slot), dph, s_abort, lane);
-                if (!ok) break;
-                tc_fence_after();
+            } else if (slot_free()) {
 #pragma unroll 1
                 for (int c = 0; c < 4; ++c) {
                     const uint4 w = *reinterpret_cast<const uint4*>(raw_row + ((c ^ swz) << 4));
-                    const uint32_t words[4] = {w.x, w.y, w.z, w.w};
-                    uint32_t cols[16];
-#pragma unroll
-                    for (int k = 0; k < 4; ++k) {
-                        __half2 h[4];
-                        dequant_word_fp16(words[k], sc2, h);
-#pragma unroll
-                        for (int q = 0; q < 4; ++q) cols[4 * k + q] = *reinterpret_cast<const uint32_t*>(&h[q]);
-                    }
-                    tmem_st16(a_slot + 16u * c, cols);
+                    uint32_t o[16];
+                    dequant_word_fp16(w.x, sc2, reinterpret_cast<__half2(&)[4]>(o[0]));
+                    dequant_word_fp16(w.y, sc2, reinterpret_cast<__half2(&)[4]>(o[4]));
+                    dequant_word_fp16(w.z, sc2, reinterpret_cast<__half2(&)[4]>(o[8]));
+                    dequant_word_fp16(w.w, sc2, reinterpret_cast<__half2(&)[4]>(o[12]));
+                    tmem_st16(a_slot + 16u * c, o);
                 }
             }
+            if (!ok) break;
             tmem_st_wait();
             tc_fence_before();
             __syncwarp();
@@ -282,7 +278,7 @@ __global__ void __launch_bounds__(kPairThreads, 1) gemm_w4a16_tc_pair_kernel(con
                 else mbar_arrive_remote(leader_full0 + 8u * slot);
             }
             rs += kPairGroups;
-            if (rs >= kPairRawSlots) { rs -= kPairRawSlots; rph ^= 1; }
+            if (rs >= kRawSlots) { rs -= kRawSlots; rph ^= 1; }
             slot += kPairGroups;
             if (slot >= kPairSlots) { slot -= kPairSlots; dph ^= 1; }
         }
@@ -301,11 +297,67 @@ __global__ void __launch_bounds__(kPairThreads, 1) gemm_w4a16_tc_pair_kernel(con
         for (int pt_i = pair_id; pt_i < total_pt && ok; pt_i += num_pairs) {
             const PairTile pt = pair_tile(a, pt_i, n_pairs, rank, MODE == kQkv);
             const int ne = (pt.n0 + r) & ~1, rows = a.rows[pt.t];
+            const size_t ld = static_cast<size_t>(a.out_ld[pt.t]);
+            // One warp polls, the others wait at a block barrier: sixteen polling warps slow the dequantising ones down.
+            // Its answer goes through one word per buffer, rewritten only after everybody has read it.
+            auto wait_full = [&]() -> bool {
+                if (warp == kEpi0) {
+                    ok = group_wait(acc_full(buf), ph, s_abort, lane);
+                    if (lane == 0) s_epi_ok[buf] = ok ? 1 : 0;
+                }
+                asm volatile("bar.sync 1, %0;" ::"n"(kPairEpiWarps * 32) : "memory");
+                ok = s_epi_ok[buf] != 0;
+                if (ok) tc_fence_after();
+                return ok;
+            };
+            auto give_back = [&]() {
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) {
+                    if (leader) mbar_arrive(acc_empty(buf));
+                    else mbar_arrive_remote(leader_empty0 + 8u * buf);
+                }
+                buf ^= 1;
+                if (buf == 0) ph ^= 1;
+            };
+            // This warp's columns of an accumulator into registers, then it goes back: the next tile's MMAs need it.
+            uint32_t v[kMaxGroups][8];
+            auto take = [&]() -> bool {
+                if (!wait_full()) return false;
+#pragma unroll
+                for (int i = 0; i < kMaxGroups; ++i)
+                    if (i < n_groups) tmem_ld8(lane_base + static_cast<uint32_t>(buf * kPairAccCols + 32 * i), v[i]);
+                tmem_ld_wait();
+                give_back();
+                return true;
+            };
+            // SWIGLU: the arithmetic on the first accumulator takes longer than the MMAs can run ahead without the second, so that one is
+            // parked in shared memory and goes back too (each thread has its own words there, nobody waits for anybody).  gate_up at
+            // 1024 / 4096 tokens 47.0 -> 43.5 / 177 -> 160 us; the others, whose epilogue is short, lose by it (O at 4096 tokens 22 -> 26).
+            [[maybe_unused]] uint4* park = reinterpret_cast<uint4*>(s_park) + (tid - kEpi0 * 32);
+            if constexpr (PARK) {
+                if (!take()) break;
+                if (H == 2) {
+                    if (!wait_full()) break;
+#pragma unroll
+                    for (int i = 0; i < kMaxGroups; ++i) {
+                        if (i < n_groups) {
+                            uint32_t u[8];
+                            tmem_ld8(lane_base + static_cast<uint32_t>(buf * kPairAccCols + 32 * i), u);
+                            tmem_ld_wait();
+                            park[(2 * i) * kPairEpiWarps * 32] = make_uint4(u[0], u[1], u[2], u[3]);
+                            park[(2 * i + 1) * kPairEpiWarps * 32] = make_uint4(u[4], u[5], u[6], u[7]);
+                        }
+                    }
+                    give_back();
+                }
+            }
+#pragma unroll 1
             for (int h = 0; h < H; ++h) {
-                const int m0 = pt.m0 + h * NH + 8 * part + odd;        // this lane's first token
-                const size_t ld = static_cast<size_t>(a.out_ld[pt.t]);
+                // this lane's first token, its place in the output, and how many tokens are left from there (it has 0, 2, 4, .. of them)
+                const int m0 = pt.m0 + h * NH + 8 * part + odd;
                 const size_t off = static_cast<size_t>(m0) * ld + (MODE == kSwiglu ? ne >> 1 : ne);
-                const int left = ne < rows ? a.M - m0 : 0;             // this lane's tokens are 0, 2, 4, .. below that
+                const int left = ne < rows ? a.M - m0 : 0;
                 // the residual of the first group while the tensor core is still at it
                 __half2 res[4];
                 auto load_res = [&](int i) {
@@ -314,27 +366,17 @@ __global__ void __launch_bounds__(kPairThreads, 1) gemm_w4a16_tc_pair_kernel(con
                         if (32 * i + 2 * q < left) res[q] = *reinterpret_cast<const __half2*>(a.residual + off + static_cast<size_t>(32 * i + 2 * q) * ld);
                 };
                 if (WORDS && add) load_res(0);
-                // One warp polls, the others wait at a block barrier: sixteen polling warps slow the dequantising ones down.
-                // Its answer goes through one word per buffer, rewritten only after everybody has read it.
-                if (warp == kEpi0) {
-                    ok = group_wait(acc_full(buf), ph, s_abort, lane);
-                    if (lane == 0) s_epi_ok[buf] = ok ? 1 : 0;
-                }
-                asm volatile("bar.sync 1, %0;" ::"n"(kPairEpiWarps * 32) : "memory");
-                ok = s_epi_ok[buf] != 0;
-                if (!ok) break;
-                tc_fence_after();
-                // this warp's columns into registers, then the accumulator goes back
-                uint32_t v[kMaxGroups][8];
+                if constexpr (!PARK) {
+                    if (!take()) break;
+                } else if (h == 1) {
 #pragma unroll
-                for (int i = 0; i < kMaxGroups; ++i)
-                    if (i < n_groups) tmem_ld8(lane_base + static_cast<uint32_t>(buf * kPairAccCols + 32 * i), v[i]);
-                tmem_ld_wait();
-                tc_fence_before();
-                __syncwarp();
-                if (lane == 0) {
-                    if (leader) mbar_arrive(acc_empty(buf));
-                    else mbar_arrive_remote(leader_empty0 + 8u * buf);
+                    for (int i = 0; i < kMaxGroups; ++i) {
+                        if (i < n_groups) {
+                            const uint4 x = park[(2 * i) * kPairEpiWarps * 32], y = park[(2 * i + 1) * kPairEpiWarps * 32];
+                            v[i][0] = x.x; v[i][1] = x.y; v[i][2] = x.z; v[i][3] = x.w;
+                            v[i][4] = y.x; v[i][5] = y.y; v[i][6] = y.z; v[i][7] = y.w;
+                        }
+                    }
                 }
                 __half* out = a.out[pt.t] + off;
 #pragma unroll
@@ -371,8 +413,6 @@ __global__ void __launch_bounds__(kPairThreads, 1) gemm_w4a16_tc_pair_kernel(con
                         if (WORDS && add && i + 1 < n_groups) load_res(i + 1);
                     }
                 }
-                buf ^= 1;
-                if (buf == 0) ph ^= 1;
             }
         }
     } else if (warp == kMmaWarp) {
@@ -462,7 +502,7 @@ __global__ void __launch_bounds__(kPairThreads, 1) gemm_w4a16_tc_pair_kernel(con
                     if (!mbar_wait(raw_empty(rs), rph, s_abort)) { ok = false; break; }
                     mbar_arrive_expect_tx(raw_full(rs), kPairRawBytes);
                     tma_load_2d(smem_u32(s_raw + rs * kPairRawBytes), &a.tmap_w[pt.t], s * 64, pt.n0, raw_full(rs));
-                    if (++rs == kPairRawSlots) { rs = 0; rph ^= 1; }
+                    if (++rs == kRawSlots) { rs = 0; rph ^= 1; }
                 }
             }
         }
@@ -501,9 +541,10 @@ __global__ void __launch_bounds__(kPairThreads, 1) gemm_w4a16_tc_pair_kernel(con
 }
 
 // ---- host side ----
-size_t tc_pair_smem_bytes(int T) {
-    return 1024 + static_cast<size_t>(kPairSlots) * T * 128 + static_cast<size_t>(kPairRawSlots) * kPairRawBytes +
-           (2 * kPairRawSlots + 2 * kPairSlots + 4) * 8 + 16;
+size_t tc_pair_smem_bytes(int mode, int T) {
+    return 1024 + static_cast<size_t>(kPairSlots) * T * 128 + static_cast<size_t>(pair_raw_slots(mode)) * kPairRawBytes +
+           (pair_parks(mode) && T > kPairAccCols ? kPairParkBytes : 0) +
+           (2 * kPairMaxRaw + 2 * kPairSlots + 4) * 8 + 16;
 }
 // Estimated cycles of a launch with token tiles of T, from measurements on B200: a step takes 4 T of MMA or 1100 of
 // dequantisation, whichever is more; a tile of two accumulators waits 2500 for the second one to be drained; the first fill,

@@ -111,7 +111,8 @@ struct MmaLaunch {
 // step of the chain; the staging of a CTA's tokens at 25 bytes a cycle; 900 for an exchange over a cluster, 1200 more where
 // the clusters would fill nearly every SM (the GPCs' sizes are not multiples of theirs, so the last ones wait: down at 4
 // tokens 6.0 us as 24 clusters of 6, 5.0 as 24 of 5); 500 per further CTA on an SM (they stand in the way of the
-// next launch's); the owner's addition of the slices.
+// next launch's); the owner's addition of the slices; and 200 per KB above 98.4 KB of shared memory an SM, where a gate_up CTA of
+// 1536 x 17920 no longer fits beside one of down's: one layer at 5 tokens 19.1 us, at 6 to 8 with 104 to 113 KB 23.0, so 20.3.
 MmaLaunch plan_mma(int mode, int units, int M, int K, int sm_count) {
     MmaLaunch best;
     const int uw = mode == kSwiglu ? 8 : 16, groups = units / uw, G = K / kGroup;
@@ -137,7 +138,8 @@ MmaLaunch plan_mma(int mode, int units, int M, int K, int sm_count) {
                 if (c.smem * per_sm > kMmaMaxSmem) continue;
                 const double cost = static_cast<double>(per_sm) * warps * per * std::max(34.0 + 3 * NT, 16.0 * NT) + 300.0 * per +
                                     static_cast<double>(per_sm) * M * cta_steps * 256 / 25 + 12.0 * slices * ((own * NT + warps - 1) / warps) +
-                                    (S == 1 ? 0.0 : ctas > 0.85 * per_sm * sm_count ? 2100.0 : 900.0) + 500.0 * (per_sm - 1);
+                                    (S == 1 ? 0.0 : ctas > 0.85 * per_sm * sm_count ? 2100.0 : 900.0) + 500.0 * (per_sm - 1) +
+                                    200.0 * std::max(0.0, static_cast<double>(c.smem) * per_sm / 1024 - 98.4);
                 if (best.ok && cost >= best_cost) continue;
                 c.NT = NT; c.grid = ctas; c.block = 32 * warps; c.ok = true;
                 if (S > 1 && max_active_clusters(reinterpret_cast<const void*>(mma_kernel(mode, NT)), c.block, c.smem, S) < blocks) continue;

@@ -61,3 +61,21 @@ def test_pair_kernel_block_with_peer_copies(pairs, col):
     for m in mats:
         assert torch.equal(m[:, col:col + N], want)
         assert (m[:, :col] == 7.0).all() and (m[:, col + N:] == 7.0).all()
+
+
+@pytest.mark.parametrize("M,I,K,scale_max", [(260, 640, 512, 0.5), (700, 8960, 256, 0.02), (513, 4480, 1536, 0.07), (1030, 5000, 768, 0.02)])
+def test_pair_kernel_swiglu_with_both_accumulators(pairs, M, I, K, scale_max):
+    """Tiles of one accumulator and of two (the second one goes through shared memory), several tiles a pair, fewer steps than ring slots."""
+    from qwen_engine_b200 import synth
+    seed = M * 31 + I + K
+    rng = np.random.default_rng(seed)
+    qw, x = synth.packed_weights(seed, "s", 2 * I, K), synth.activations(seed, "s", M, K)
+    sc = rng.uniform(0.002, scale_max, size=(2 * I, K // 128)).astype(np.float16)
+    y = torch.full((M * I + 64,), float("nan"), dtype=torch.float16, device="cuda")
+    pairs.launch_gemm_prefill_dual_gate_up_swiglu_w4a16(util.to_dev(qw), util.to_dev(sc), util.to_dev(x), y, M, None, K, I)
+    torch.cuda.synchronize()
+    got = util.to_np(y)
+    assert np.isnan(got[M * I:]).all(), "wrote past the output"
+    m_idx, n_idx = _pick(rng, M), _pick(rng, I)
+    ref64, _ = oracle.gemm_prefill(qw, sc, x, m_idx, n_idx, swiglu=True)
+    util.assert_fp16_close(got[:M * I].reshape(M, I)[np.ix_(m_idx, n_idx)], ref64, what=f"swiglu {M}x{I}x{K}")

@@ -118,7 +118,17 @@ __device__ __forceinline__ void stream_load_acc(uint32_t taddr, int acc2_col, fl
     for (int j = 0; j < 8; ++j) v[j] = __uint_as_float(x[j]) + __uint_as_float(y[j]);
 }
 
-__device__ __forceinline__ float swiglu_f32(float gate, float up) { return (gate / (1.0f + expf(-gate))) * up; }
+// gate / (1 + e^-gate) * up.  The quotient: by the approximate reciprocal (1 ulp), then one correction by its residual, Newton's
+// step for a quotient, which leaves little but the last rounding.  It has no residual (NaN) where it is infinite or the divisor is;
+// the quotient itself is right there.  430 000 values against 64 bits: the bits of an IEEE division, whose checks and branch cost
+// gate_up at 300 / 512 / 1024 tokens 22.0 / 26.1 / 44.0 us, so 20.4 / 24.9 / 42.7.
+__device__ __forceinline__ float swiglu_f32(float gate, float up) {
+    const float d = 1.0f + expf(-gate);
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(d));
+    const float q = gate * r, rest = fmaf(-q, d, gate);
+    return (rest == rest ? fmaf(rest, r, q) : q) * up;
+}
 
 // NV tokens m0 .. m0 + NV - 1 of weight row n (acc) to the output.  All lanes of a warp call it with consecutive rows and
 // the same tokens.  SWIGLU: rows 2i / 2i + 1 are gate and up of one output; the lane pair exchanges one value per two
@@ -132,7 +142,8 @@ __device__ __forceinline__ void stream_store(const StreamArgs& a, int t, int n, 
 #pragma unroll
         for (int q = 0; q < NV; q += 2) {
             const float other = __shfl_xor_sync(0xFFFFFFFFu, odd ? acc[q] : acc[q + 1], 1);
-            const float y = odd ? swiglu_f32(other, acc[q + 1]) : swiglu_f32(acc[q], other);
+            // (the operands are chosen, not the result: a choice between two calls ran both, gate_up at 47 / 115 tokens 6.8 -> 6.1 / 9.9 -> 8.5 us)
+            const float y = swiglu_f32(odd ? other : acc[q], odd ? acc[q + 1] : other);
             if (row_ok && m0 + q + odd < a.M) *out = __float2half_rn(y);
             out += 2 * ld;
         }

@@ -70,3 +70,37 @@ def test_stream_kernel_swiglu_and_qkv_routing(M):
 ])
 def test_stream_kernel_few_tokens_and_ring_lengths(M, N, K, scale_max, res):
     test_stream_kernel_matches_oracle(M, N, K, scale_max, res)
+
+
+@pytest.mark.parametrize("M", [16, 64, 700])
+def test_swiglu_quotient_over_its_range(M):
+    """Gate and up values planted through tokens with one nonzero element, from 1e-4 to the ends of fp16's range, against 64 bits.
+    exp (2 ulp), the sum, the quotient and the product leave at most 6 * 2^-24 of a value, so an output is the nearest fp16
+    value except within that of a midpoint, two neighbours of which are 2^-11 apart: 0.2 % of them, and by one step."""
+    import qwen_engine_b200 as ops
+    K, I = 256, 512
+    rng = np.random.default_rng(M)
+    q, sc = rng.integers(0, 16, 2 * I), rng.uniform(0.002, 0.05, (2 * I, 2)).astype(np.float16)
+    qw = np.zeros((2 * I, K // 8), dtype=np.uint32)
+    qw[:, 0] = q                                   # element 0 is the word's lowest nibble
+    x = np.zeros((M, K), dtype=np.float16)
+    x[:, 0] = (rng.standard_normal(M) * np.logspace(-2, 3, M)).astype(np.float16)
+    w = ((q - 8) * sc[:, 0].astype(np.float32)).astype(np.float16).astype(np.float64)
+
+    def run(xs):
+        y = torch.empty((M, I), dtype=torch.float16, device="cuda")
+        ops.launch_gemm_prefill_dual_gate_up_swiglu_w4a16(util.to_dev(qw), util.to_dev(sc), util.to_dev(xs), y, M, None, K, I)
+        torch.cuda.synchronize()
+        with np.errstate(all="ignore"):
+            acc = (xs[:, :1].astype(np.float64) * w[None, :]).astype(np.float32).astype(np.float64)
+            return util.to_np(y), acc[:, 0::2] / (1.0 + np.exp(-acc[:, 0::2])) * acc[:, 1::2]
+    got, ref = run(x)
+    ok = (np.abs(ref) > 1e-4) & (np.abs(ref) < 6e4)
+    with np.errstate(over="ignore"):
+        near = ref.astype(np.float16)
+    steps = np.abs(got[ok].view(np.int16).astype(np.int32) - near[ok].view(np.int16).astype(np.int32))
+    assert steps.max() <= 1 and np.mean(steps != 0) <= 2e-3, (steps.max(), np.mean(steps != 0))
+    # infinite accumulators: -inf / (1 + inf) is NaN, inf / 1 is inf, whatever up makes of them
+    x[:, 0] = np.where(np.arange(M) % 2 == 0, np.inf, -np.inf).astype(np.float16)
+    got, ref = run(x)
+    assert np.array_equal(np.isnan(got), np.isnan(ref)) and np.array_equal(np.isposinf(got), np.isposinf(ref)) and np.array_equal(np.isneginf(got), np.isneginf(ref))

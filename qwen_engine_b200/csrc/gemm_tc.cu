@@ -410,8 +410,8 @@ int pair_launch(const GemmArgs& g, int sm_count, cudaStream_t stream) {
 }  // namespace
 
 // Up to 256 tokens the streaming kernel (more CTAs, K split), above that whichever of the two is estimated to be faster: thin
-// matrices stay with the streaming kernel up to about 1024 tokens (QKV at 1024: 9.4 us against 11.7 on pairs), gate_up goes to
-// pairs at once (300 tokens: 29.7 against 23.2 us).  W4A16_OPT_GEMM_FORM = 1 / 2 asks for one of them.
+// matrices stay with the streaming kernel up to about 1024 tokens (streaming / pairs, us, at 1024: QKV 8.4 / 10.7, O 9.3 / 11.1,
+// down 25.0 / 31.8), gate_up goes to pairs at once (23.1 / 20.0 at 300, 32.3 / 24.8 at 450).  W4A16_OPT_GEMM_FORM = 1 / 2 asks for one of them.
 int gemm_tc_launch(const GemmArgs& g, int sm_count, cudaStream_t stream) {
     const int form = option(W4A16_OPT_GEMM_FORM);
     if (form != 2) {

@@ -548,7 +548,8 @@ size_t tc_pair_smem_bytes(int mode, int T) {
 }
 // Estimated cycles of a launch with token tiles of T, from measurements on B200: a step takes 4 T of MMA or 1100 of
 // dequantisation, whichever is more; a tile of two accumulators waits 2500 for the second one to be drained; the first fill,
-// the exchange at the start and the last tile's epilogue are not overlapped.
+// the exchange at the start and the last tile's epilogue are not overlapped.  (Constants of the kernel's first form.  A fit to the
+// present one, 4.4 T, 780 and 1900, is closer to the times but picks worse tiles: gate_up at 4096 tokens 183 -> 199 us, QKV 24 -> 29.)
 double pair_cost(int M, int n_pairs, int steps, int pairs, int T) {
     const int tiles = n_pairs * ((M + T - 1) / T), rounds = (tiles + pairs - 1) / pairs;
     return rounds * (steps * std::max(4.0 * T, 1100.0) + (T > kPairAccCols ? 2500.0 : 0.0)) + 9000.0 + 25.0 * T;

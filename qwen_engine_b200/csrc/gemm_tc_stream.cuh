@@ -1,5 +1,5 @@
-// Batched-decode W4A16 contraction on tcgen05 (17 to 256 tokens) as a weight-streaming kernel: one launch is about as long
-// as its weights take to arrive.  Included by gemm_tc.cu behind the PTX wrappers.
+// Batched-decode W4A16 contraction on tcgen05 (9 to 256 tokens, thin matrices above) as a weight-streaming kernel.  Included by
+// gemm_tc.cu behind the PTX wrappers.
 //
 // What bounds it: at these token counts a launch reads 1-14 MB of packed weights (0.2-2 us of HBM time) and the rest is
 // latency -- the launch boundary, the dequantisation, the token tile's way from L2, the hand-overs between roles, the

@@ -1,4 +1,4 @@
-"""The weight-streaming tcgen05 kernel (17-256 tokens) at the edges of its tiles: token tiles of 16 to 128, one and two of
+"""The weight-streaming tcgen05 kernel (up to 256 tokens) at the edges of its tiles: token tiles of 16 to 128, one and two of
 them, K ranges of two steps and of many, split and not, rows past the last whole tile, scales on both sides of the limit
 of the short dequantisation."""
 import numpy as np

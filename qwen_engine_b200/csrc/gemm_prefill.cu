@@ -111,8 +111,7 @@ struct MmaLaunch {
 // step of the chain; the staging of a CTA's tokens at 25 bytes a cycle; 900 for an exchange over a cluster, 1200 more where
 // the clusters would fill nearly every SM (the GPCs' sizes are not multiples of theirs, so the last ones wait: down at 4
 // tokens 6.0 us as 24 clusters of 6, 5.0 as 24 of 5); 500 per further CTA on an SM (they stand in the way of the
-// next launch's); the owner's addition of the slices; and 200 per KB above 98.4 KB of shared memory an SM, where a gate_up CTA of
-// 1536 x 17920 no longer fits beside one of down's: one layer at 5 tokens 19.1 us, at 6 to 8 with 104 to 113 KB 23.0, so 20.3.
+// next launch's); the owner's addition of the slices.
 MmaLaunch plan_mma(int mode, int units, int M, int K, int sm_count) {
     MmaLaunch best;
     const int uw = mode == kSwiglu ? 8 : 16, groups = units / uw, G = K / kGroup;
@@ -138,8 +137,7 @@ MmaLaunch plan_mma(int mode, int units, int M, int K, int sm_count) {
                 if (c.smem * per_sm > kMmaMaxSmem) continue;
                 const double cost = static_cast<double>(per_sm) * warps * per * std::max(34.0 + 3 * NT, 16.0 * NT) + 300.0 * per +
                                     static_cast<double>(per_sm) * M * cta_steps * 256 / 25 + 12.0 * slices * ((own * NT + warps - 1) / warps) +
-                                    (S == 1 ? 0.0 : ctas > 0.85 * per_sm * sm_count ? 2100.0 : 900.0) + 500.0 * (per_sm - 1) +
-                                    200.0 * std::max(0.0, static_cast<double>(c.smem) * per_sm / 1024 - 98.4);
+                                    (S == 1 ? 0.0 : ctas > 0.85 * per_sm * sm_count ? 2100.0 : 900.0) + 500.0 * (per_sm - 1);
                 if (best.ok && cost >= best_cost) continue;
                 c.NT = NT; c.grid = ctas; c.block = 32 * warps; c.ok = true;
                 if (S > 1 && max_active_clusters(reinterpret_cast<const void*>(mma_kernel(mode, NT)), c.block, c.smem, S) < blocks) continue;
@@ -190,14 +188,16 @@ int gemm_launch(GemmArgs g, cudaStream_t stream) {
     for (int t = 0; t < (g.mode == kQkv ? 3 : 1); ++t) aligned = aligned && reinterpret_cast<uintptr_t>(g.qweight[t]) % 16 == 0;
 
     // A few tokens: the weight-streaming kernel with the warp-level MMA (no fixed tcgen05 costs).  Rows in whole groups of 16 (a
-    // group of QKV rows from one tensor).  One token tile of 8 on all but the largest matrices, two on the smallest ones only.  mma /
+    // group of QKV rows from one tensor).  One token tile of 8 (from 6 tokens on gate_up and down of a 1536 / 8960 layer, 138 and 113 KB
+    // of shared memory, no longer share an SM, and a layer with those two on tcgen05 takes 20.1 us against 23.0; of 2048 / 6144 21.2
+    // against 23.9, of 1024 / 4096 14.9 against 14.4), two on the smallest matrices only, none on the largest.  mma /
     // tcgen05, us, each behind itself: at 4 tokens QKV 2.9 / 3.8, down 5.5 / 5.6, gate_up 6.5 / 6.3 (but a layer of all four
     // 17.8 / 19.8, since CTAs of two launches share an SM in the mma form), 17920 x 2048 7.8 / 7.5, 8192 x 8192 13.0 / 13.0; at 9
     // 2048 x 512 2.9 / 3.5, QKV 4.4 / 3.8, gate_up 7.6 / 6.4; at 16 QKV 4.5 / 3.4, O 4.1 / 3.7, gate_up 8.2 / 5.9, down 8.0 / 5.7, the
     // layer 23.6 / 19.1.
     const size_t weights = static_cast<size_t>(rows_all) * g.K;
     const int mma_max_opt = option(W4A16_OPT_GEMM_MMA_MAX_TOKENS);
-    const int mma_max_m = mma_max_opt > 0 ? mma_max_opt : (weights <= 2u << 20 ? 16 : weights <= 32u << 20 ? 8 : 1);
+    const int mma_max_m = mma_max_opt > 0 ? mma_max_opt : (weights <= 2u << 20 ? 16 : weights <= 10u << 20 ? 8 : weights <= 32u << 20 ? 5 : 1);
     const bool whole_groups = a.units % (g.mode == kSwiglu ? 8 : 16) == 0 && (g.mode != kQkv || (g.rows[0] % 16 == 0 && g.rows[1] % 16 == 0 && g.rows[2] % 16 == 0));
     bool scale_pairs = true;
     for (int t = 0; t < (g.mode == kQkv ? 3 : 1); ++t) scale_pairs = scale_pairs && reinterpret_cast<uintptr_t>(g.scales[t]) % 4 == 0;

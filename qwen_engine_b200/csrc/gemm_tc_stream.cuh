@@ -1,4 +1,4 @@
-// Batched-decode W4A16 contraction on tcgen05 (9 to 256 tokens, thin matrices above) as a weight-streaming kernel.  Included by
+// Batched-decode W4A16 contraction on tcgen05 (6 to 256 tokens, thin matrices above) as a weight-streaming kernel.  Included by
 // gemm_tc.cu behind the PTX wrappers.
 //
 // What bounds it: at these token counts a launch reads 1-14 MB of packed weights (0.2-2 us of HBM time) and the rest is

@@ -86,9 +86,9 @@ def test_rmsnorm_q8_1_gain_written_by_the_launch_in_front():
     assert torch.equal(y[0].view(torch.int16), y[1].view(torch.int16))
 
 
-@pytest.mark.parametrize("M,N,K,scale_max", [(9, 17920, 1536, 0.02), (13, 272, 4096, 0.5), (16, 1536, 8960, 0.02), (16, 30000, 512, 0.07)])
-def test_few_token_kernel_with_two_token_tiles(M, N, K, scale_max):
-    """9 to 16 tokens through this kernel whatever the matrix (by default only the smallest ones)."""
+@pytest.mark.parametrize("M,N,K,scale_max", [(7, 1536, 8960, 0.02), (8, 17920, 1536, 0.5), (9, 17920, 1536, 0.02), (13, 272, 4096, 0.5), (16, 1536, 8960, 0.02), (16, 30000, 512, 0.07)])
+def test_few_token_kernel_asked_for(M, N, K, scale_max):
+    """6 to 16 tokens through this kernel whatever the matrix (by default only the smaller ones)."""
     import qwen_engine_b200 as ops
     ops.set_option(ops.OPT_GEMM_MMA_MAX_TOKENS, 16)
     try:

@@ -62,7 +62,8 @@ def test_stream_kernel_swiglu_and_qkv_routing(M):
 
 
 @pytest.mark.parametrize("M,N,K,scale_max,res", [
-    # token counts that come to it from the few-token forms: 9 to 16, 2 on long K, 4 on rows that are no whole groups of 16
+    # token counts that come to it from the few-token forms: 6 to 16, 2 on long K, 4 on rows that are no whole groups of 16
+    (6, 17920, 1536, 0.02, False), (8, 1536, 8960, 0.02, True),
     (9, 1536, 1536, 0.02, True), (16, 17920, 1536, 0.5, False), (13, 2048, 8960, 0.02, True), (2, 264, 8192, 0.02, False),
     (4, 130, 512, 0.07, True), (3, 8200, 8192, 0.02, False),
     # one more step than token slots, steps beyond both rings, an odd number of steps in a CTA (two issuing threads)

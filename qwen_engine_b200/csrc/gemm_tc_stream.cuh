@@ -119,15 +119,18 @@ __device__ __forceinline__ void stream_load_acc(uint32_t taddr, int acc2_col, fl
 }
 
 // gate / (1 + e^-gate) * up.  The quotient: by the approximate reciprocal (1 ulp), then one correction by its residual, Newton's
-// step for a quotient, which leaves little but the last rounding.  It has no residual (NaN) where it is infinite or the divisor is;
-// the quotient itself is right there.  430 000 values against 64 bits: the bits of an IEEE division, whose checks and branch cost
-// gate_up at 300 / 512 / 1024 tokens 22.0 / 26.1 / 44.0 us, so 20.4 / 24.9 / 42.7.
+// step for a quotient, which leaves little but the last rounding.  The divisor is a sixteenth (and up with it): the reciprocal of
+// one above 2^126, gates of -87.4 to -88.7, would be flushed to zero, and an infinite up then made NaN of it.  No correction where
+// there is nothing to correct or no residual (NaN, with an infinite gate or divisor): the quotient itself is right there, the sign
+// of a zero included.  Compared with an IEEE division for every gate of 2^-48 to 2^124 (sums of fp16 products lie in between), of
+// both signs, zeros and infinities: the same bits.  Its checks and branch cost gate_up at 300 / 512 / 1024 tokens 22.0 / 26.1 / 44.0
+// us, so 20.4 / 24.9 / 42.7, and with the sixteenth 1 % more.
 __device__ __forceinline__ float swiglu_f32(float gate, float up) {
-    const float d = 1.0f + expf(-gate);
+    const float d = fmaf(0.0625f, expf(-gate), 0.0625f);
     float r;
     asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(d));
     const float q = gate * r, rest = fmaf(-q, d, gate);
-    return (rest == rest ? fmaf(rest, r, q) : q) * up;
+    return (fabsf(rest) > 0.0f ? fmaf(rest, r, q) : q) * (0.0625f * up);
 }
 
 // NV tokens m0 .. m0 + NV - 1 of weight row n (acc) to the output.  All lanes of a warp call it with consecutive rows and

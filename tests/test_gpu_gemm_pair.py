@@ -79,3 +79,10 @@ def test_pair_kernel_swiglu_with_both_accumulators(pairs, M, I, K, scale_max):
     m_idx, n_idx = _pick(rng, M), _pick(rng, I)
     ref64, _ = oracle.gemm_prefill(qw, sc, x, m_idx, n_idx, swiglu=True)
     util.assert_fp16_close(got[:M * I].reshape(M, I)[np.ix_(m_idx, n_idx)], ref64, what=f"swiglu {M}x{I}x{K}")
+
+
+@pytest.mark.parametrize("M,K", [(700, 256), (2400, 1024)])      # tiles of one accumulator, of two
+def test_pair_kernel_swiglu_quotient(pairs, M, K):
+    from tests import test_gpu_gemm_stream as stream
+    stream.test_swiglu_quotient_over_its_range(M, K)
+    stream.test_swiglu_with_an_infinite_up(M, K)

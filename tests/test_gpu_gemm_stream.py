@@ -74,14 +74,14 @@ def test_stream_kernel_few_tokens_and_ring_lengths(M, N, K, scale_max, res):
 
 
 @pytest.mark.parametrize("M", [16, 64, 700])
-def test_swiglu_quotient_over_its_range(M):
+def test_swiglu_quotient_over_its_range(M, K=256):
     """Gate and up values planted through tokens with one nonzero element, from 1e-4 to the ends of fp16's range, against 64 bits.
     exp (2 ulp), the sum, the quotient and the product leave at most 6 * 2^-24 of a value, so an output is the nearest fp16
     value except within that of a midpoint, two neighbours of which are 2^-11 apart: 0.2 % of them, and by one step."""
     import qwen_engine_b200 as ops
-    K, I = 256, 512
+    I = 512
     rng = np.random.default_rng(M)
-    q, sc = rng.integers(0, 16, 2 * I), rng.uniform(0.002, 0.05, (2 * I, 2)).astype(np.float16)
+    q, sc = rng.integers(0, 16, 2 * I), rng.uniform(0.002, 0.05, (2 * I, K // 128)).astype(np.float16)
     qw = np.zeros((2 * I, K // 8), dtype=np.uint32)
     qw[:, 0] = q                                   # element 0 is the word's lowest nibble
     x = np.zeros((M, K), dtype=np.float16)
@@ -105,3 +105,22 @@ def test_swiglu_quotient_over_its_range(M):
     x[:, 0] = np.where(np.arange(M) % 2 == 0, np.inf, -np.inf).astype(np.float16)
     got, ref = run(x)
     assert np.array_equal(np.isnan(got), np.isnan(ref)) and np.array_equal(np.isposinf(got), np.isposinf(ref)) and np.array_equal(np.isneginf(got), np.isneginf(ref))
+
+
+@pytest.mark.parametrize("M", [4, 16, 64, 700])
+def test_swiglu_with_an_infinite_up(M, K=256):
+    """Gates around the one from which e^-gate is infinite (-88.7), and of both signs: an infinity where IEEE arithmetic has one."""
+    import qwen_engine_b200 as ops
+    gates = np.concatenate([np.linspace(-91, -86, 448), np.linspace(-80, 80, 64)]).astype(np.float16)
+    I = len(gates)
+    qw, sc = np.full((2 * I, K // 8), 0x88888888, dtype=np.uint32), np.ones((2 * I, K // 128), dtype=np.float16)
+    qw[0::2, 0], sc[0::2, 0] = 0x88888889, gates               # one weight of a gate row is its scale, the others are zero
+    qw[1::2, :16], sc[1::2, 0] = 0x99999999, np.inf            # a group of infinite weights
+    x = np.ones((M, K), dtype=np.float16)
+    y = torch.empty((M, I), dtype=torch.float16, device="cuda")
+    ops.launch_gemm_prefill_dual_gate_up_swiglu_w4a16(util.to_dev(qw), util.to_dev(sc), util.to_dev(x), y, M, None, K, I)
+    torch.cuda.synchronize()
+    g = gates.astype(np.float32)
+    with np.errstate(all="ignore"):
+        ref = (g / (np.float32(1) + np.exp(-g)) * np.float32(np.inf)).astype(np.float16)
+    assert np.array_equal(util.to_np(y), np.broadcast_to(ref, (M, I)), equal_nan=True)

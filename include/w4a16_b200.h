@@ -100,8 +100,8 @@ enum {
     W4A16_OPT_GEMM_FORM = 5,         /* tensor-core form of the M-token contraction: 0 (default) chosen by tokens and
                                         shape, 1 weight streaming (one CTA per tile and K slice), 2 CTA pairs */
     W4A16_OPT_GEMM_MMA_MAX_TOKENS = 6, /* largest token count that takes the weight-streaming mma.sync kernel instead of
-                                        the tcgen05 kernels: 0 (default) the measured crossover (1 to 16 by size), 1 never, n up to
-                                        n (at most 16) */
+                                        the tcgen05 kernels: 0 (default) the measured crossover (1 to 16 by size; 16 where those
+                                        do not take the call), 1 never, n up to n (at most 16) */
     W4A16_OPT_COUNT_ = 7
 };
 W4A16_API int w4a16_set_option(int option, int value);

@@ -1,6 +1,7 @@
 // Host dispatch of the M-token W4A16 contraction (small-M decode batches and prefill).
 #include <algorithm>
 
+#include "gemm_dispatch.hpp"
 #include "gemm_smallm.cuh"
 #include "gemm_smallm_mma.cuh"
 #include "w4a16_internal.hpp"
@@ -167,14 +168,6 @@ int gemm_launch(GemmArgs g, cudaStream_t stream) {
     const DeviceInfo* dev = nullptr;
     if (int st = ensure_device_ready(&dev)) return st;
 
-    // The tcgen05 kernel pads the token count to its smallest tile (16), so for shapes that the mma form below refuses the CUDA-core
-    // form (the decode GEMV's memory behaviour with fp16 arithmetic) is the faster one at the fewest tokens: up to 3 on the narrow
-    // K <= 4096 shapes (QKV, O), one where K > 4096 (the few-token form stages only two tokens per pass there) or where the matrix
-    // gives every SM a CTA of its own.  CUDA cores / tcgen05, us: down 10.6 / 5.6 and gate_up 8.2 / 6.3 at 2 tokens, 8192 x 8192
-    // 80 / 13 at 2, O 5.4 / 3.7 and QKV 4.4 / 3.8 at 4 (3.6 / 3.8 at 2).  The CUDA-core forms also take what TMA cannot address.
-    const int tc_min_m_opt = option(W4A16_OPT_GEMM_MIN_TOKENS_TENSOR_CORE);
-    const int rows_all = g.rows[0] + (g.mode == kQkv ? g.rows[1] + g.rows[2] : 0);
-    const int tc_min_m = tc_min_m_opt > 0 ? tc_min_m_opt : (g.K > 4096 || rows_all >= 64 * dev->sm_count ? 2 : 4);
     SmallMArgs a;
     a.g = g;
     const int total_rows = g.rows[0] + (g.mode == kQkv ? g.rows[1] + g.rows[2] : 0);
@@ -184,37 +177,26 @@ int gemm_launch(GemmArgs g, cudaStream_t stream) {
     } else {
         a.out_ld[0] = (g.mode == kPlain && g.ldc > 0) ? g.ldc : a.units; a.out_ld[1] = a.out_ld[2] = 0;
     }
-    bool aligned = reinterpret_cast<uintptr_t>(g.x) % 16 == 0;
-    for (int t = 0; t < (g.mode == kQkv ? 3 : 1); ++t) aligned = aligned && reinterpret_cast<uintptr_t>(g.qweight[t]) % 16 == 0;
-
-    // A few tokens: the weight-streaming kernel with the warp-level MMA (no fixed tcgen05 costs).  Rows in whole groups of 16 (a
-    // group of QKV rows from one tensor).  One token tile of 8 (from 6 tokens on gate_up and down of a 1536 / 8960 layer, 138 and 113 KB
-    // of shared memory, no longer share an SM, and a layer with those two on tcgen05 takes 20.1 us against 23.0; of 2048 / 6144 21.2
-    // against 23.9, of 1024 / 4096 14.9 against 14.4), two on the smallest matrices only, none on the largest.  mma /
-    // tcgen05, us, each behind itself: at 4 tokens QKV 2.9 / 3.8, down 5.5 / 5.6, gate_up 6.5 / 6.3 (but a layer of all four
-    // 17.8 / 19.8, since CTAs of two launches share an SM in the mma form), 17920 x 2048 7.8 / 7.5, 8192 x 8192 13.0 / 13.0; at 9
-    // 2048 x 512 2.9 / 3.5, QKV 4.4 / 3.8, gate_up 7.6 / 6.4; at 16 QKV 4.5 / 3.4, O 4.1 / 3.7, gate_up 8.2 / 5.9, down 8.0 / 5.7, the
-    // layer 23.6 / 19.1.
-    const size_t weights = static_cast<size_t>(rows_all) * g.K;
-    const int mma_max_opt = option(W4A16_OPT_GEMM_MMA_MAX_TOKENS);
-    const int mma_max_m = mma_max_opt > 0 ? mma_max_opt : (weights <= 2u << 20 ? 16 : weights <= 10u << 20 ? 8 : weights <= 32u << 20 ? 5 : 1);
-    const bool whole_groups = a.units % (g.mode == kSwiglu ? 8 : 16) == 0 && (g.mode != kQkv || (g.rows[0] % 16 == 0 && g.rows[1] % 16 == 0 && g.rows[2] % 16 == 0));
-    bool scale_pairs = true;
-    for (int t = 0; t < (g.mode == kQkv ? 3 : 1); ++t) scale_pairs = scale_pairs && reinterpret_cast<uintptr_t>(g.scales[t]) % 4 == 0;
-    if (aligned && scale_pairs && whole_groups && g.num_peers == 0 && g.M >= std::max(2, tc_min_m_opt) && g.M <= std::min(mma_max_m, 16)) {
+    const bool tc = gemm_tc_supported(g);
+    auto form_of = [&](bool mma) {
+        return gemm_form(g, dev->sm_count, tc, mma, option(W4A16_OPT_GEMM_MIN_TOKENS_TENSOR_CORE), option(W4A16_OPT_GEMM_MMA_MAX_TOKENS));
+    };
+    GemmForm form = form_of(gemm_mma_supported(g));
+    if (form == GemmForm::kMma) {
         static PlanCache<MmaLaunch> plans;
         const MmaLaunch m = plans.get(plan_key(g.mode, g.M, g.K, a.units), [&] { return plan_mma(g.mode, a.units, g.M, g.K, dev->sm_count); });
         if (m.ok)
             return static_cast<int>(launch_kernel_cluster(mma_kernel(g.mode, m.NT), dim3(m.grid), dim3(m.block), m.smem, stream, pdl_enabled(),
                                                           dim3(static_cast<unsigned>(m.plan.cluster), 1, 1), a, m.plan));
+        form = form_of(false);
     }
-    if ((g.M >= tc_min_m || g.num_peers > 0) && gemm_tc_supported(g)) return gemm_tc_launch(g, dev->sm_count, stream);
+    if (form == GemmForm::kTc) return gemm_tc_launch(g, dev->sm_count, stream);
     if (g.num_peers > 0) return W4A16_ERR_SHAPE;   // peer stores exist in the tensor-core form only
 
     // few tokens, 16-byte aligned tensors: the form that streams like the decode GEMV
     SmallMPlan plan;
     int U = 8;
-    if (aligned && plan_v2(g, a.units, dev->sm_count, &plan, &U)) {
+    if (gemm_aligned16(g) && plan_v2(g, a.units, dev->sm_count, &plan, &U)) {
         const int R = g.mode == kSwiglu ? 2 : 1;
         // tokens per pass: as many as the shared-memory budget of a CTA (about a third of an SM) allows
         int mt = g.M >= 4 ? 4 : (g.M >= 2 ? 2 : 1);

@@ -128,3 +128,42 @@ int main() {
     return plans.get(w4::PlanKey{0, 0, 2, 256, 16}, [] { return -1; }) == 2 && plans.get(w4::PlanKey{0, 0, 3, 256, 16}, [] { return 7; }) == 7 ? 0 : 2;
 }
 ''') == 0
+
+
+def test_few_tokens_stay_off_the_cuda_cores(tmp_path):
+    """Rows in whole groups of 16 and aligned tensors: at 2 to 16 tokens, with the options at their defaults, the rule sends no size to
+    the CUDA-core forms, whether tcgen05 can take it (QKV widths in multiples of 128) or not; and asking for a form is heeded."""
+    assert _run_cpp(tmp_path, '''#include "gemm_dispatch.hpp"
+#include <cstdio>
+using namespace w4;
+int main() {
+    int bad = 0;
+    for (int mode : {int(kPlain), int(kQkv), int(kSwiglu)})
+        for (int K = 256; K <= 16384; K += K < 1024 ? 256 : 768)
+            for (int n : {16, 48, 128, 320, 336, 512, 1536, 2048, 4608, 8192, 8208, 9216, 9456, 9472, 9488, 17920, 28672, 151936})
+                for (int heads : {16, 64, 128, 576})
+                    for (int M = 1; M <= 17; ++M) {
+                        if (mode != kQkv && heads != 16) continue;
+                        GemmArgs g = {};
+                        g.mode = mode; g.M = M; g.K = K; g.rows[0] = n;
+                        if (mode == kQkv) g.rows[1] = g.rows[2] = heads;
+                        const bool tc = mode != kQkv || (n % 128 == 0 && heads % 128 == 0);
+                        if (!gemm_mma_supported(g)) return 1;
+                        const GemmForm f = gemm_form(g, 148, tc, true, 0, 0);
+                        if (M == 1 && f == GemmForm::kMma) return 2;
+                        if (M >= 2 && M <= 16 && f == GemmForm::kCuda) { ++bad; std::printf("mode %d: %d + 2 x %d rows, K %d, %d tokens\\n", mode, n, heads, K, M); }
+                        if (M == 17 && f != (tc ? GemmForm::kTc : GemmForm::kCuda)) return 3;
+                        if (M >= 2 && M <= 16 && gemm_form(g, 148, tc, true, 0, 16) != GemmForm::kMma) return 4;
+                        if (tc && M >= 2 && gemm_form(g, 148, tc, true, 2, 1) != GemmForm::kTc) return 5;
+                        if (gemm_form(g, 148, tc, true, 1000, 0) != GemmForm::kCuda) return 6;
+                    }
+    GemmArgs g = {};
+    g.mode = kPlain; g.M = 3; g.K = 512; g.rows[0] = 48; g.num_peers = 1;
+    if (gemm_mma_supported(g) || gemm_form(g, 148, true, false, 0, 0) != GemmForm::kTc || gemm_form(g, 148, false, false, 0, 0) != GemmForm::kCuda) return 7;
+    g.num_peers = 0; g.rows[0] = 40;
+    if (gemm_mma_supported(g)) return 8;
+    g.rows[0] = 48; g.scales[0] = reinterpret_cast<const __half*>(2);
+    if (gemm_mma_supported(g)) return 9;
+    return bad ? 10 : 0;
+}
+''') == 0

@@ -95,3 +95,27 @@ def test_few_token_kernel_asked_for(M, N, K, scale_max):
         test_few_token_kernel_matches_oracle(M, N, K, scale_max)
     finally:
         ops.set_option(ops.OPT_GEMM_MMA_MAX_TOKENS, 0)
+
+
+@pytest.mark.parametrize("M,N,K", [(2, 8208, 4096), (3, 9456, 4096), (3, 9376, 3584)])
+def test_large_matrix_below_the_first_tokens_of_tcgen05(M, N, K):
+    test_few_token_kernel_matches_oracle(M, N, K, 0.02)
+
+
+@pytest.mark.parametrize("M,K,q_heads,kv_heads", [(9, 1536, 24, 5), (16, 1024, 15, 3), (6, 4096, 64, 9)])
+def test_qkv_of_heads_of_64(M, K, q_heads, kv_heads):
+    """Widths that are no multiples of 128, which the tcgen05 kernels refuse."""
+    import qwen_engine_b200 as ops
+    from qwen_engine_b200 import synth
+    rows = [64 * q_heads, 64 * kv_heads, 64 * kv_heads]
+    qw, sc, x = synth.packed_weights(M, "q", sum(rows), K), synth.scales(M, "q", sum(rows), K), synth.activations(M, "q", M, K)
+    cut = np.cumsum([0, *rows])
+    qkv = [(util.to_dev(qw[a:b].copy()), util.to_dev(sc[a:b].copy()), torch.full((M, b - a), float("nan"), dtype=torch.float16, device="cuda"))
+           for a, b in zip(cut, cut[1:])]
+    ops.launch_gemm_prefill_qkv_w4a16(ops.QKVProjectionView(*[t for p in qkv for t in p]), util.to_dev(x), M, None, K, q_heads, kv_heads, 64)
+    m_idx, n_idx = np.arange(M, dtype=np.int32), np.unique(np.concatenate([np.arange(0, sum(rows), 29), cut[1:] - 1, cut[:-1]])).astype(np.int32)
+    ref64, _ = oracle.gemm_prefill(qw, sc, x, m_idx, n_idx)
+    got = np.concatenate([util.to_np(p[2]) for p in qkv], axis=1)
+    assert not np.isnan(got).any()
+    util.assert_fp16_close(got[:, n_idx], ref64, what="qkv")
+    assert ops.debug_counter(0) == 0

@@ -43,13 +43,16 @@ inline GemmForm gemm_form(const GemmArgs& g, int sm_count, bool tc, bool mma, in
     tc = tc && (g.M >= tc_min_m || g.num_peers > 0);     // (stores to peers exist in the tcgen05 kernels only)
 
     // A few tokens: the weight-streaming kernel with the warp-level MMA (no fixed tcgen05 costs).  Where tcgen05 takes the call
-    // too: one token tile of 8 (from 6 tokens on gate_up and down of a 1536 / 8960 layer, 138 and 113 KB
-    // of shared memory, no longer share an SM, and a layer with those two on tcgen05 takes 20.1 us against 23.0; of 2048 / 6144 21.2
-    // against 23.9, of 1024 / 4096 14.9 against 14.4), two on the smallest matrices only, none on the largest.  mma /
-    // tcgen05, us, each behind itself: at 4 tokens QKV 2.9 / 3.8, down 5.5 / 5.6, gate_up 6.5 / 6.3 (but a layer of all four
-    // 17.8 / 19.8, since CTAs of two launches share an SM in the mma form), 17920 x 2048 7.8 / 7.5, 8192 x 8192 13.0 / 13.0; at 9
-    // 2048 x 512 2.9 / 3.5, QKV 4.4 / 3.8, gate_up 7.6 / 6.4; at 16 QKV 4.5 / 3.4, O 4.1 / 3.7, gate_up 8.2 / 5.9, down 8.0 / 5.7, the
-    // layer 23.6 / 19.1.  Where it does not, up to 16 tokens whatever the size: mma / CUDA cores, us, 9216 x 4096 at 2 / 3 tokens
+    // too, by what a layer takes, since CTAs of two launches share an SM in the mma form and one launch chained with itself says
+    // little about that.  28 layers with weights of their own in a graph, us a layer, everything on mma / as the lines have it / mma
+    // never:
+    //   1536 / 8960   at 4 tokens 18.2 / 18.3 / 18.8, at 6 22.1 / 18.5 / 18.8 (from there on gate_up and down, 138 and 113 KB of shared
+    //                 memory, no longer share an SM), at 9 22.5 / 19.0 / 19.0, at 16 24.1 / 19.4 / 19.2
+    //   2048 / 8960   (gate_up 35 Mi weights) at 2 / 3 tokens 24.1 / 23.9, 24.5 / 24.2, at 5 24.6 / 24.5 / 21.4
+    //   2048 / 6144   at 4 tokens 22.1 / 22.2 / 19.8, at 6 22.0 / 19.3 / 19.9, at 9 24.7 / 20.0 / 19.9
+    //   1024 / 4096   at 6 tokens the lines leave it on mma: 12.8 to 13.9 against 14.8; at 9 14.9 / 15.1 / 14.9
+    // (so a layer of 2048 would be better off whole on tcgen05 from 4 tokens, which no line by one matrix's size says.)
+    // The smallest matrices keep mma to 16 tokens: 2048 x 512 at 9 2.9 / 3.5 chained with itself.  Where tcgen05 does not take it, up to 16 tokens whatever the size: mma / CUDA cores, us, 9216 x 4096 at 2 / 3 tokens
     // 8.2 / 37 and 8.3 / 58 (SWIGLU 8.1 / 11.3 and 8.2 / 20.4), QKV of 24 + 2 x 5 heads of 64 on K = 1536 at 9 / 16 4.4 / 10.9 and
     // 4.6 / 14.3, of 64 + 2 x 9 on K = 4096 at 6 / 16 7.5 / 30 and 9.2 / 71.
     const int mma_max_m = mma_opt > 0 ? mma_opt : !tc || weights <= 2u << 20 ? 16 : weights <= 10u << 20 ? 8 : weights <= 32u << 20 ? 5 : 1;

@@ -249,7 +249,7 @@ namespace {
 // The streaming kernel's cut of a shape: token tiles and K slices, two steps each at least, within one CTA per SM where that is
 // possible, by the time it is estimated to take, in cycles of 1.9 GHz.  The constants are fitted to 2200 timed cuts of 14
 // shapes (512 x 512 to 17920 x 1536 and 1536 x 8960) at 4 to 1024 tokens, launches one behind another (the cut they choose is on
-// average 1.4 % slower than the best one; the former rule's 3.2 %).  The first steps hide behind the launch; a step is 400 of
+// average 1.2 % slower than the best one).  The first steps hide behind the launch; a step is 400 of
 // dequantisation, 650 beyond what the token slots hold, or 6 a token of its tile's way from L2; 35 a token of the tile for the
 // epilogue; the exchange of a K split 1100 and 66 a token sent; CTAs on more than half of the SMs keep the next launch's from
 // starting early; a further wave costs its launch again.

@@ -1,5 +1,5 @@
-// Batched-decode W4A16 contraction on tcgen05 (6 to 256 tokens, thin matrices above) as a weight-streaming kernel.  Included by
-// gemm_tc.cu behind the PTX wrappers.
+// Batched-decode W4A16 contraction on tcgen05 (from a few tokens, by size, to 256; thin matrices above) as a weight-streaming
+// kernel.  Included by gemm_tc.cu behind the PTX wrappers.
 //
 // What bounds it: at these token counts a launch reads 1-14 MB of packed weights (0.2-2 us of HBM time) and the rest is
 // latency -- the launch boundary, the dequantisation, the token tile's way from L2, the hand-overs between roles, the
@@ -23,7 +23,8 @@
 // The loading threads are chosen by elect.sync too, and each ring has one of its own: as one `lane == 0` thread that looked
 // after both rings a step took them 430 cycles, and with every other part of the kernel taken out a launch was hardly faster
 // (gate_up at 47 tokens 8.6 us, 5.7 without data, dequantisation, MMAs or epilogue).  Every token slot that fits is asked for at
-// once.  One layer of 1536 / 8960 at 47 tokens: QKV 6.0 -> 4.7, O 5.6 -> 4.3, gate_up 8.5 -> 6.7, down 8.4 -> 6.4 us a launch.
+// once.  One layer of 1536 / 8960 at 47 tokens: QKV 6.0 -> 4.7, O 5.6 -> 4.3, gate_up 8.5 -> 6.7, down 8.4 -> 6.4 us a launch (as
+// the kernel is now 4.3, 4.3, 6.1 and 6.5).
 //
 // Tensor memory: even and odd steps go into accumulators of their own: half as many additions per fp32 sum, which at
 // K = 8192 is the difference between 2.7 and 2 fp16 steps of error.  A slots of 64 columns follow: six up to 64 tokens,

@@ -1,5 +1,6 @@
-// Few-token W4A16 contraction (decode batches of 2 to 5 tokens, to 8 or 16 on small matrices) as a weight-streaming kernel
-// whose inner product runs on the warp-level tensor-core instruction mma.sync.m16n8k16 (fp16 x fp16 -> fp32).
+// Few-token W4A16 contraction (decode batches of 2 to 5 tokens; to 8 or 16 on small matrices and where tcgen05 does not take
+// the call) as a weight-streaming kernel whose inner product runs on the warp-level tensor-core instruction mma.sync.m16n8k16
+// (fp16 x fp16 -> fp32).
 //
 // Why not tcgen05 here: at these token counts a launch is latency, and one on tcgen05 carries tensor-memory allocation,
 // TMA round trips, commits and barrier hand-overs whatever the token count.  Here a launch is: weights into registers
